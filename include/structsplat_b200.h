@@ -348,6 +348,12 @@ int ss_fit_adam_update(const ss_batch* batch, const void* records, int64_t n,
  * ref_dev points to the energy reference (a device double, e.g. stats_dev[0] of
  * ss_structure_tensor). */
 int ss_placement_workspace_bytes(int height, int width, size_t* bytes);
+/* The next `count` doubles of a numpy PCG64 generator's random(), into the device array out:
+ * the sampler's uniforms without a host draw and copy.  state and increment are the generator's
+ * 128-bit words as {high, low} host pairs; state_after (host, may be NULL) receives the state
+ * after the draw, written when the launch has succeeded. */
+int ss_pcg64_uniforms(const uint64_t* state, const uint64_t* increment, int64_t count,
+                      double* out, uint64_t* state_after, ss_stream_t stream);
 int ss_density_from_energy(const float* energy, int height, int width, double base,
                            double power, const double* ref_dev, double* density, void* workspace,
                            size_t workspace_bytes, ss_stream_t stream);

@@ -18,6 +18,7 @@ _int = ctypes.c_int
 _f32 = ctypes.c_float
 _f64 = ctypes.c_double
 _szp = ctypes.POINTER(ctypes.c_size_t)
+_u64p = ctypes.POINTER(ctypes.c_uint64)
 
 
 class SsBatch(ctypes.Structure):
@@ -119,6 +120,7 @@ SIGNATURES = {
     "ss_fit_adam_update": [_bp, _vp, _i64, _vp, _i64, _vp, _int, _vp, _f32, _pp, _pp, _pp, _dp,
                            _f64, _f64, _f64, _f32, _vp, _vp, _vp],
     "ss_placement_workspace_bytes": [_int, _int, _szp],
+    "ss_pcg64_uniforms": [_u64p, _u64p, _i64, _vp, _u64p, _vp],
     "ss_density_from_energy": [_vp, _int, _int, _f64, _f64, _vp, _vp, _vp, ctypes.c_size_t, _vp],
     "ss_sample_candidates": [_vp, _int, _int, _vp, _i64, _vp, _vp, _vp, ctypes.c_size_t, _vp],
     "ss_place_gaussians": [_vp, _i64, _vp, _vp, _vp, _vp, _int, _int, _int, _f64, _f64, _f64,

@@ -77,6 +77,45 @@ __device__ __forceinline__ double reflect(double v, double hi) {
   return __dsub_rn(hi, fabs(__dsub_rn(hi, v)));
 }
 
+// The doubles a numpy PCG64 Generator's random() draws, computed in parallel.  PCG64 (O'Neill,
+// "PCG: A Family of Simple Fast Space-Efficient Statistically Good Algorithms for Random Number
+// Generation", 2014) is a 128-bit linear congruential generator s <- A s + C with the XSL-RR output
+// rotr64(hi ^ lo, s >> 122) of the advanced state; random() is the output's top 53 bits times
+// 2^-53.  k steps at once are again affine, s <- A_k s + C_k, so a thread reaches the state
+// before its first value with one such map per set bit of its index and then strides by the grid
+// size with one multiply-add per value.  Integer-bound: 6 M values take ~20 us where one host core
+// takes 20 ms and the copy of its pageable result another 3 ms.
+typedef unsigned __int128 u128;
+
+struct PcgJumps {
+  u128 state;            // the generator's state before its first value
+  u128 mul[32], add[32];  // the affine map of 2^k steps
+};
+
+constexpr int kPcgLogThreads = 17;  // 131,072 threads, ~7 warps per scheduler
+constexpr int kPcgThreads = 1 << kPcgLogThreads;
+
+__global__ void __launch_bounds__(kThreads)
+    pcg64_uniforms_kernel(__grid_constant__ const PcgJumps j, int64_t count,
+                          double* __restrict__ out) {
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (tid >= count) return;
+  u128 s = j.state;
+  const uint32_t steps = tid + 1;  // the output reads the advanced state
+  for (int k = 0; k <= kPcgLogThreads; ++k)
+    if ((steps >> k) & 1u) s = s * j.mul[k] + j.add[k];
+  const u128 mul = j.mul[kPcgLogThreads], add = j.add[kPcgLogThreads];
+  for (int64_t i = tid; i < count; i += kPcgThreads) {
+    const uint64_t hi = (uint64_t)(s >> 64), v = hi ^ (uint64_t)s;
+    const unsigned r = (unsigned)(hi >> 58);
+    const uint64_t x = (v >> r) | (v << ((64u - r) & 63u));
+    out[i] = __dmul_rn((double)(x >> 11), 0x1p-53);
+    s = s * mul + add;
+  }
+}
+
 __global__ void sample_kernel(const double* __restrict__ cdf, int64_t npx, int W, int H,
                               const double* __restrict__ uniforms, int64_t n,
                               double* __restrict__ pts, int64_t* __restrict__ index_out) {
@@ -240,6 +279,41 @@ int ss_placement_workspace_bytes(int height, int width, size_t* bytes) {
   if (rc) return rc;
   if (!bytes) return fail(SS_ERR_INVALID_ARGUMENT, "null bytes pointer");
   *bytes = place_ws_bytes((int64_t)height * width);
+  return SS_OK;
+}
+
+int ss_pcg64_uniforms(const uint64_t* state, const uint64_t* increment, int64_t count,
+                      double* out, uint64_t* state_after, ss_stream_t stream) {
+  if (count < 0) return fail(SS_ERR_INVALID_ARGUMENT, "negative count");
+  if (!state || !increment || (count > 0 && !out))
+    return fail(SS_ERR_INVALID_ARGUMENT, "null pointer");
+  const u128 c = ((u128)increment[0] << 64) | increment[1];
+  // the multiplier of the PCG paper's 128-bit generator
+  const u128 a = ((u128)0x2360ED051FC65DA4ull << 64) | 0x4385DF649FCCF645ull;
+  PcgJumps j;
+  j.state = ((u128)state[0] << 64) | state[1];
+  u128 mul = a, add = c, after = j.state;
+  for (int k = 0; k < 63; ++k) {  // the map of 2^k steps, applied twice, is that of 2^(k+1)
+    if (k < 32) {
+      j.mul[k] = mul;
+      j.add[k] = add;
+    }
+    if ((count >> k) & 1) after = after * mul + add;
+    add = add * mul + add;
+    mul = mul * mul;
+  }
+  if (count > 0) {
+    const int64_t threads = count < kPcgThreads ? count : kPcgThreads;
+    const int rc = launch("pcg64_uniforms_kernel", pcg64_uniforms_kernel, blocks_for(threads),
+                          kThreads, 0, as_stream(stream), j, count, out);
+    if (rc) return rc;
+    const int lc = check_launch("pcg64_uniforms");
+    if (lc) return lc;
+  }
+  if (state_after) {
+    state_after[0] = (uint64_t)(after >> 64);
+    state_after[1] = (uint64_t)after;
+  }
   return SS_OK;
 }
 
