@@ -342,7 +342,7 @@ int ss_fit_adam_update(const ss_batch* batch, const void* records, int64_t n,
 /* ---------------------------------------------------------------- placement
  * Density-weighted placement of a field from the structure tensor (density.py, init.py).
  * All images are (H,W) row-major; the workspace (ss_placement_workspace_bytes) holds a copy of
- * the cdf and CUB's temporary storage.
+ * the cdf, the search guide of the sampler and CUB's temporary storage.
  *
  * ss_density_from_energy: density.py:16-29.  energy (H,W) f32 -> density (H,W) f64 pmf;
  * ref_dev points to the energy reference (a device double, e.g. stats_dev[0] of
