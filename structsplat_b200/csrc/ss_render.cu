@@ -397,6 +397,33 @@ __device__ __forceinline__ float4 finish_pixel(const float* a, int64_t p, float 
   }
 }
 
+// Adds a tile's loss and squared error to its image's, one atomic each per tile: the rounding of
+// the running sum grows with the number of additions, and one per warp (16 times as many) cost
+// several times the error for no time saved.  Every thread of the CTA calls it.
+template <int NT>
+__device__ __forceinline__ void add_tile_loss(float loss_sum, float sq_sum, float per_value,
+                                              float* loss) {
+  __shared__ float part[2][NT / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    loss_sum += __shfl_xor_sync(0xffffffffu, loss_sum, o);
+    sq_sum += __shfl_xor_sync(0xffffffffu, sq_sum, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    part[0][threadIdx.x >> 5] = loss_sum;
+    part[1][threadIdx.x >> 5] = sq_sum;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {  // one warp: lanes 0-15 the loss, 16-31 the squared error
+    constexpr int kWarps = NT / 32;
+    const int which = threadIdx.x >> 4, k = threadIdx.x & 15;
+    float v = k < kWarps ? part[which][k] : 0.f;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (k == 0) atomicAdd(loss + which, v * per_value);
+  }
+}
+
 // Shared memory of the forward kernel (dynamic): the stage (whole lists up to kStageAll
 // records, or two halves of it for a streamed list) followed by every warp's carry slots and
 // the null record; the staged records' rectangles, packed; and every warp's hit list, which
@@ -587,17 +614,7 @@ __global__ void __launch_bounds__(Tiling<TS>::kFwdThreads, 2)
       }
     }
   }
-  if (LOSS != kNoLoss && loss) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      loss_sum += __shfl_xor_sync(0xffffffffu, loss_sum, o);
-      sq_sum += __shfl_xor_sync(0xffffffffu, sq_sum, o);
-    }
-    if (lane == 0) {
-      atomicAdd(loss + 2 * fr.image, loss_sum * per_value);
-      atomicAdd(loss + 2 * fr.image + 1, sq_sum * per_value);
-    }
-  }
+  if (LOSS != kNoLoss && loss) add_tile_loss<NT>(loss_sum, sq_sum, per_value, loss + 2 * fr.image);
 }
 
 // One level of a reduce-scatter butterfly: lanes whose `bit` is clear keep slots [0, K) of v,
@@ -995,17 +1012,7 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
       stage_range<NT>(stage, rec, L, 0, (int)(L.count < kHalf ? L.count : kHalf), stage_gid);
       cp_async_commit();
     }
-    if (ff.loss) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        loss_sum += __shfl_xor_sync(0xffffffffu, loss_sum, o);
-        sq_sum += __shfl_xor_sync(0xffffffffu, sq_sum, o);
-      }
-      if (lane == 0) {
-        atomicAdd(ff.loss + 2 * fr.image, loss_sum * per_value);
-        atomicAdd(ff.loss + 2 * fr.image + 1, sq_sum * per_value);
-      }
-    }
+    if (ff.loss) add_tile_loss<NT>(loss_sum, sq_sum, per_value, ff.loss + 2 * fr.image);
     // the barrier before the first group (below) orders these pix writes before their reads
   }
   tile_finite = __syncthreads_and(pix_ok) != 0;
