@@ -140,6 +140,11 @@ int ss_batch_project_rs_index_count(const ss_batch* batch, const float* means,
  * (render_ext.cu:101-133,178-191); callers enable it only together with the support fade. */
 int ss_tile_index_workspace_bytes(int64_t n, int height, int width, int tile_size,
                                   size_t* bytes);
+/* The larger workspace of the binned index: with at least this many bytes the count also keeps
+ * every pair's id in a bin of its tile, and the fill only orders the bins (one launch instead of
+ * three).  The same lists either way.  Both stages must get the same workspace and size. */
+int ss_tile_index_binned_workspace_bytes(int64_t n, int height, int width, int tile_size,
+                                         size_t* bytes);
 /* Stage 1: per-tile counts and offsets.  tile_offsets (T+1) int32 receives the offsets;
  * tile_offsets[T] is the entry total.  workspace must be kept for stage 2. */
 int ss_tile_index_count(const void* records, int64_t n, int height, int width, int tile_size,
@@ -178,6 +183,8 @@ int ss_batch_project_rs(const ss_batch* batch, const float* means, const float* 
                         const float* opacity_logits, int64_t n, float dilation,
                         float sigma_cutoff, void* records, ss_stream_t stream);
 int ss_batch_tile_index_workspace_bytes(const ss_batch* batch, int64_t n, size_t* bytes);
+/* depends on n too */
+int ss_batch_tile_index_binned_workspace_bytes(const ss_batch* batch, int64_t n, size_t* bytes);
 int ss_batch_tile_index_count(const ss_batch* batch, const void* records, int64_t n,
                               int ellipse_cull, float sigma_cutoff, int32_t* tile_offsets,
                               void* workspace, size_t workspace_bytes, uint32_t* status,

@@ -54,6 +54,7 @@ SIGNATURES = {
     "ss_project_rs": [_vp, _vp, _vp, _vp, _vp, _i64, _f32, _f32, _int, _int, _vp, _vp, _vp, _vp],
     "ss_project_rs_backward": [_vp, _vp, _vp, _i64, _f32, _vp, _vp, _vp, _vp, _vp, _vp],
     "ss_tile_index_workspace_bytes": [_i64, _int, _int, _int, _szp],
+    "ss_tile_index_binned_workspace_bytes": [_i64, _int, _int, _int, _szp],
     "ss_tile_index_count": [_vp, _i64, _int, _int, _int, _int, _f32, _vp, _vp, ctypes.c_size_t,
                             _vp, _vp],
     "ss_tile_index_fill": [_vp, _i64, _int, _int, _int, _int, _f32, _vp, _vp, _i64, _vp,
@@ -92,6 +93,7 @@ SIGNATURES = {
                           ctypes.c_size_t, _vp, _vp],
     "ss_batch_project_rs": [_bp, _vp, _vp, _vp, _vp, _vp, _i64, _f32, _f32, _vp, _vp],
     "ss_batch_tile_index_workspace_bytes": [_bp, _i64, _szp],
+    "ss_batch_tile_index_binned_workspace_bytes": [_bp, _i64, _szp],
     "ss_batch_tile_index_count": [_bp, _vp, _i64, _int, _f32, _vp, _vp, ctypes.c_size_t, _vp,
                                   _vp],
     "ss_batch_tile_index_fill": [_bp, _vp, _i64, _int, _f32, _vp, _vp, _i64, _vp,

@@ -176,7 +176,8 @@ class FitPlan:
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, **f32)
         self.offsets = torch.zeros(batch.tiles + 1, device=d, dtype=torch.int32)
         self.status = torch.zeros(1, device=d, dtype=torch.int32)
-        self.idx_ws_bytes = _native.size_query("ss_batch_tile_index_workspace_bytes", batch.ref, n)
+        self.idx_ws_bytes = _native.size_query("ss_batch_tile_index_binned_workspace_bytes",
+                                               batch.ref, n)
         self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=d, dtype=torch.uint8)
         if capacity <= 0:
             capacity = self.measure_entries() * 3 // 2 + 4096

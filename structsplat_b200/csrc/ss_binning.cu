@@ -4,13 +4,20 @@
 // whose clipped support rectangle touches it, offsets[t]..offsets[t+1]; the lists are sorted by
 // ascending Gaussian id, which is the order the reference's stable radix sort leaves and makes
 // every downstream sum deterministic.  No sort over all pairs is needed: per-tile counts come
-// from atomics, a device-wide scan gives the offsets, the fill claims slots with per-tile atomic
-// cursors, and a per-tile bitonic sort in shared memory restores ascending ids.  The scan is one
-// single-CTA kernel for up to 16,384 tiles and CUB's device scan beyond.
+// from atomics, a scan gives the offsets, and each tile's ids are put into ascending order by
+// one CTA.  Two forms, by the size of the caller's workspace:
+//
+//   binned (a workspace of ss_tile_index_binned_workspace_bytes): the count's atomics return each
+//     pair's rank in its tile, so the same kernel drops the id into the tile's bin, and
+//     bin_sort_kernel orders each bin into the list.  At 100k Gaussians on 1024x1024 (213k pairs)
+//     the fill, warp-sort and block-sort launches after the count took 12 + 6.4 + 4.2 us; this one
+//     takes their place.
+//   plain (a workspace of ss_tile_index_workspace_bytes, which depends on the tiles only): the
+//     fill enumerates the pairs again and claims slots with per-tile atomic cursors, then a
+//     warp or a CTA sorts each list.
 #include <climits>
 
 #include <cub/block/block_radix_sort.cuh>
-#include <cub/block/block_scan.cuh>
 #include <cub/device/device_scan.cuh>
 #include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
@@ -61,7 +68,21 @@ struct IndexWorkspace {
   int* big_count;         // 1
   void* scan_temp;
   size_t scan_bytes;
+  int32_t* bins;          // T x bin_ids, or NULL: ids by tile in arrival order
+  int bin_ids;            // K, ids a bin holds
 };
+
+// Ids per bin: 32 times the Gaussians per tile (lists average 2 to 8 times them; a tile beyond
+// that is rebuilt from the records by bin_sort_kernel).  0, no bins, without Gaussians or tiles and
+// where very many tiles would make them larger than 256 MB + 256 B per Gaussian.
+int bin_ids_for(int64_t n, int64_t T) {
+  if (n <= 0 || T <= 0) return 0;
+  int64_t k = 32 * ((n + T - 1) / T) + 32;
+  if (k > n) k = n;
+  k = (k + 7) & ~int64_t(7);  // every bin starts on a 32-byte sector
+  if (T * k * (int64_t)sizeof(int32_t) > ((int64_t)256 << 20) + 256 * n) return 0;
+  return (int)k;
+}
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -79,7 +100,12 @@ size_t index_workspace_bytes(int64_t T) {
          align256(scan_temp_bytes(T + 1));
 }
 
-IndexWorkspace carve(void* base, int64_t T) {
+size_t binned_workspace_bytes(int64_t n, int64_t T) {
+  return index_workspace_bytes(T) +
+         align256((size_t)T * (size_t)bin_ids_for(n, T) * sizeof(int32_t));
+}
+
+IndexWorkspace carve(void* base, size_t bytes, int64_t n, int64_t T) {
   IndexWorkspace w;
   char* p = static_cast<char*>(base);
   w.tile_count = reinterpret_cast<int*>(p);
@@ -92,6 +118,9 @@ IndexWorkspace carve(void* base, int64_t T) {
   p += align256(sizeof(int));
   w.scan_temp = p;
   w.scan_bytes = align256(scan_temp_bytes(T + 1));
+  p += w.scan_bytes;
+  w.bin_ids = bytes >= binned_workspace_bytes(n, T) ? bin_ids_for(n, T) : 0;
+  w.bins = w.bin_ids > 0 ? reinterpret_cast<int32_t*>(p) : nullptr;
   return w;
 }
 
@@ -99,9 +128,8 @@ struct TileRect {
   int gx0, gy0, gw, gh;
 };
 
-__device__ __forceinline__ TileRect tile_rect_of(const Splat* rec, int64_t i, int ts) {
+__device__ __forceinline__ TileRect tile_rect(const int4& b, int ts) {
   TileRect r{0, 0, 0, 0};
-  int4 b = reinterpret_cast<const int4*>(rec + i)[3];
   if (b.z > b.x && b.w > b.y) {
     r.gx0 = b.x / ts;
     r.gy0 = b.y / ts;
@@ -120,6 +148,10 @@ __device__ __forceinline__ Splat load_splat(const Splat* rec, int64_t i) {
   d[2] = src[2];
   d[3] = src[3];
   return s;
+}
+
+__device__ __forceinline__ TileRect tile_rect_of(const Splat* rec, int64_t i, int ts) {
+  return tile_rect(reinterpret_cast<const int4*>(rec + i)[3], ts);
 }
 
 // Calls visit(gaussian, tile) for every (tile, Gaussian) pair of the index, in any order.
@@ -185,101 +217,185 @@ __device__ __forceinline__ void enumerate_pairs(const Splat* rec, int64_t n, int
   }
 }
 
-// Exclusive scan of the T+1 counters into int64 and int32 offsets by one CTA of kThreads
-// threads, in rounds of kScanItems kThreads items (one round for up to 2,047 tiles); the counters
-// are read from L2 (other CTAs' atomics), every load of a round in flight before the scan.
-constexpr int kScanItems = 8;
-__device__ void block_scan_counts(const int* tile_count, int64_t items, long long* off64,
-                                  int32_t* off32) {
-  using Scan = cub::BlockScan<long long, kThreads>;
-  __shared__ typename Scan::TempStorage tmp;
-  long long carry = 0;
-  for (int64_t b0 = 0; b0 < items; b0 += kScanItems * kThreads) {
-    long long v[kScanItems];
+// Counts one CTA's pairs: thread l holds Gaussian `first + l` with record s (`in`: there is one).
+// The threads share the CTA's pairs evenly, whatever the rectangles' sizes: pair e belongs to
+// the last thread whose exclusive prefix of tile counts is <= e.  (Shared by warps only, the warp
+// with the widest Gaussians of a heavy-tailed field sets the kernel's time: 69 us for 250k
+// Gaussians and 2 M pairs.)  BINS: each pair's rank in its tile, which its atomic returns, is its
+// slot in the tile's bin (a full bin drops the id; the count still tells the list's length).  What
+// is left is the L2's rate of atomics and of scattered 4-byte stores, ~70 and ~100 per ns.
+// Rectangles of more than kHugeRect tiles take the whole CTA one after the other, so the prefix
+// stays small.
+constexpr int kHugeRect = 1 << 20;
+
+struct PairShare {
+  int excl[kThreads], tile0[kThreads], gw[kThreads], gh[kThreads], tiles_x[kThreads];
+  int warp_total[kThreads / 32];
+  unsigned huge[kThreads / 32];
+};
+struct CullShare {  // the ellipse cull's inputs
+  float mx[kThreads], my[kThreads], a[kThreads], b[kThreads], c[kThreads];
+  int4 rect[kThreads];
+};
+
+template <bool CULL, bool BINS>
+__device__ __forceinline__ void count_pairs(const Splat& s, bool in, int first, int ts,
+                                            int tiles_x, int first_tile, float cutoff2,
+                                            int* tile_count, int32_t* bins, int K) {
+  __shared__ PairShare sh;
+  __shared__ CullShare cs[1];
+  const unsigned all = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  TileRect r{0, 0, 0, 0};
+  if (in) r = tile_rect(make_int4(s.x0, s.y0, s.x1, s.y1), ts);
+  const int cnt = r.gw * r.gh;
+  const int own = cnt > kHugeRect ? 0 : cnt;
+  int incl = own;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      const int64_t idx = b0 + kScanItems * threadIdx.x + k;
-      v[k] = idx < items ? __ldcg(tile_count + idx * kCounterStride) : 0;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(all, incl, o);
+    if (lane >= o) incl += v;
+  }
+  const unsigned huge_mask = __ballot_sync(all, cnt > kHugeRect);
+  if (lane == 31) sh.warp_total[warp] = incl;
+  if (lane == 0) sh.huge[warp] = huge_mask;
+  sh.tile0[tid] = first_tile + r.gy0 * tiles_x + r.gx0;
+  sh.gw[tid] = r.gw;
+  sh.gh[tid] = r.gh;
+  sh.tiles_x[tid] = tiles_x;
+  if (CULL) {
+    cs[0].mx[tid] = s.mx;
+    cs[0].my[tid] = s.my;
+    cs[0].a[tid] = s.a;
+    cs[0].b[tid] = s.b;
+    cs[0].c[tid] = s.c;
+    cs[0].rect[tid] = make_int4(s.x0, s.y0, s.x1, s.y1);
+  }
+  __syncthreads();
+  int base = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) {
+    const int t = sh.warp_total[w];
+    base += w < warp ? t : 0;
+    total += t;
+  }
+  sh.excl[tid] = base + incl - own;
+  __syncthreads();
+  auto tile_of = [&](int l, unsigned k) {  // -1: culled
+    const unsigned gw = (unsigned)sh.gw[l];
+    const int row = (int)(k / gw), col = (int)(k - (unsigned)row * gw);
+    if (CULL) {
+      Splat o;
+      o.mx = cs[0].mx[l];
+      o.my = cs[0].my[l];
+      o.a = cs[0].a[l];
+      o.b = cs[0].b[l];
+      o.c = cs[0].c[l];
+      const int4 b = cs[0].rect[l];
+      o.x0 = b.x;
+      o.y0 = b.y;
+      o.x1 = b.z;
+      o.y1 = b.w;
+      if (culled(o, b.x / ts + col, b.y / ts + row, ts, cutoff2)) return -1;
     }
-    long long total;
-    Scan(tmp).ExclusiveSum(v, v, total);
+    return sh.tile0[l] + row * sh.tiles_x[l] + col;
+  };
+  for (int e0 = tid; e0 < total; e0 += 2 * kThreads) {  // two pairs per thread in flight
+    int tile[2] = {-1, -1}, owner[2] = {0, 0}, rank[2] = {0, 0};
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
-      const int64_t idx = b0 + kScanItems * threadIdx.x + k;
-      if (idx < items) {
-        const long long o = carry + v[k];
-        off64[idx] = o;
-        off32[idx] = (int32_t)(o < 2147483647LL ? o : 2147483647LL);
+    for (int u = 0; u < 2; ++u) {
+      const int e = e0 + u * kThreads;
+      if (e < total) {
+        int l = 0;
+#pragma unroll
+        for (int step = kThreads / 2; step > 0; step >>= 1)
+          if (sh.excl[l + step] <= e) l += step;
+        owner[u] = l;
+        tile[u] = tile_of(l, (unsigned)(e - sh.excl[l]));
       }
     }
-    carry += total;
-    __syncthreads();  // tmp is reused by the next round
-  }
-}
-
-// Per-tile counts by atomics.  SCAN: the last CTA to finish (a ticket in the padding word after
-// counter 0, zeroed with the counters) also scans the counts into the offsets, which saves the
-// separate scan launch for small tile sets.
-template <bool CULL, bool SCAN>
-__global__ void tile_count_kernel(const Splat* __restrict__ rec, int64_t n, int ts, Frames frames,
-                                  float cutoff2, int* __restrict__ tile_count, int64_t items,
-                                  long long* __restrict__ off64, int32_t* __restrict__ off32) {
-  pdl_wait();
-  pdl_trigger();
-  enumerate_pairs<CULL>(rec, n, ts, frames, cutoff2,
-                        [&](int, int, int t) { atomicAdd(tile_count + (int64_t)t * kCounterStride, 1); });
-  if constexpr (SCAN) {
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();  // this CTA's counts before its ticket
-      const unsigned ticket = atomicAdd(reinterpret_cast<unsigned*>(tile_count + 1), 1u);
-      last = ticket == gridDim.x - 1;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (tile[u] >= 0) rank[u] = atomicAdd(tile_count + (int64_t)tile[u] * kCounterStride, 1);
+    if (BINS) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (tile[u] >= 0 && rank[u] < K) bins[(int64_t)tile[u] * K + rank[u]] = first + owner[u];
     }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();  // every other CTA's counts are visible after its ticket
-    block_scan_counts(tile_count, items, off64, off32);
+  }
+  for (int w = 0; w < kThreads / 32; ++w) {
+    for (unsigned huge = sh.huge[w]; huge; huge &= huge - 1) {
+      const int l = 32 * w + __ffs(huge) - 1;
+      const unsigned n = (unsigned)sh.gw[l] * (unsigned)sh.gh[l];
+      for (unsigned k = tid; k < n; k += kThreads) {
+        const int t = tile_of(l, k);
+        if (t < 0) continue;
+        const int rank = atomicAdd(tile_count + (int64_t)t * kCounterStride, 1);
+        if (BINS && rank < K) bins[(int64_t)t * K + rank] = first + l;
+      }
+    }
   }
 }
 
-// The RS projection (rs_project_one, as project_rs_kernel) and the per-tile counts in one pass:
-// each thread stores its Gaussian's record and counts its tiles from it, so the counts need no
-// second read of the records from DRAM.  The record is read back by its own thread (and, for a
-// rectangle the warp enumerates together, by the warp after __syncwarp), so `out` carries no
-// read-only qualifier.  SCAN as in tile_count_kernel.  The grid also zeroes `clear_vec` 16-byte
-// words at `clear` (a caller's per-step scratch, such as the next backward's moments).
-template <bool CULL, bool SCAN>
-__global__ void project_count_kernel(RSField field, int64_t n, int ts, Frames frames,
-                                     float cutoff2, Splat* out, int* __restrict__ tile_count,
-                                     int64_t items, long long* __restrict__ off64,
-                                     int32_t* __restrict__ off32, uint4* __restrict__ clear,
-                                     int64_t clear_vec) {
+// Per-tile counts by atomics, and with BINS the bins.  The second padding word after counter 0
+// (zeroed with the counters) tells bin_sort_kernel that the bins belong to these counts.
+template <bool CULL, bool BINS>
+__global__ void tile_count_kernel(const Splat* __restrict__ rec, int64_t n, int ts, Frames frames,
+                                  float cutoff2, int* __restrict__ tile_count,
+                                  int32_t* __restrict__ bins, int K) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (BINS && i == 0) tile_count[2] = K;
+  Splat s{};
+  int tiles_x = 0, first_tile = 0;
+  if (i < n) {
+    if (CULL) {
+      s = load_splat(rec, i);
+    } else {
+      const int4 b = reinterpret_cast<const int4*>(rec + i)[3];
+      s.x0 = b.x;
+      s.y0 = b.y;
+      s.x1 = b.z;
+      s.y1 = b.w;
+    }
+    const Frame fr = frame_of_gaussian(frames, i, n);
+    tiles_x = fr.tiles_x;
+    first_tile = fr.first_tile;
+  }
+  count_pairs<CULL, BINS>(s, i < n, blockIdx.x * kThreads, ts, tiles_x, first_tile, cutoff2,
+                          tile_count, bins, K);
+}
+
+// The RS projection (rs_project_one, as project_rs_kernel) and the per-tile counts in one pass:
+// each thread stores its Gaussian's record and counts its tiles from the registers that hold it.
+// BINS as in tile_count_kernel.  The grid also zeroes `clear_vec` 16-byte words at
+// `clear` (a caller's per-step scratch, such as the next backward's moments).
+template <bool CULL, bool BINS>
+__global__ void project_count_kernel(RSField field, int64_t n, int ts, Frames frames,
+                                     float cutoff2, Splat* __restrict__ out,
+                                     int* __restrict__ tile_count, uint4* __restrict__ clear,
+                                     int64_t clear_vec,
+                                     int32_t* __restrict__ bins, int K) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (BINS && i == 0) tile_count[2] = K;
   for (int64_t v = i; v < clear_vec; v += (int64_t)gridDim.x * blockDim.x)
     clear[v] = make_uint4(0u, 0u, 0u, 0u);
+  Splat s{};
+  int tiles_x = 0, first_tile = 0;
   if (i < n) {
-    long long rx, ry;
-    store_splat(out + i, rs_project_one(field, i, frame_of_gaussian(frames, i, n), rx, ry));
+    const RSParams p = rs_load(field, i);
+    const Frame fr = frame_of_gaussian(frames, i, n);
+    float rx, ry;
+    s = rs_project_one(field, p, fr.H, fr.W, rx, ry);
+    store_splat(out + i, s);
+    tiles_x = fr.tiles_x;
+    first_tile = fr.first_tile;
   }
-  __syncwarp();
-  enumerate_pairs<CULL>(out, n, ts, frames, cutoff2,
-                        [&](int, int, int t) { atomicAdd(tile_count + (int64_t)t * kCounterStride, 1); });
-  if constexpr (SCAN) {
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      const unsigned ticket = atomicAdd(reinterpret_cast<unsigned*>(tile_count + 1), 1u);
-      last = ticket == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    block_scan_counts(tile_count, items, off64, off32);
-  }
+  count_pairs<CULL, BINS>(s, i < n, blockIdx.x * kThreads, ts, tiles_x, first_tile, cutoff2,
+                          tile_count, bins, K);
 }
 
 // Writes int32 offsets, checks capacity, then claims one slot per pair.  Slots are claimed by
@@ -322,58 +438,57 @@ __global__ void tile_fill_kernel(const Splat* __restrict__ rec, int64_t n, int t
     if (pos[k] >= 0 && pos[k] < cap) gids[pos[k]] = owner;
 }
 
-// Offsets of small tile sets in one launch: a single CTA scans up to kSingleScanMax per-tile
-// counts (each thread a contiguous run of kScanPerThread, then a block scan of the run totals)
-// and writes the int64 and the int32 offsets.  Larger tile sets use CUB's device scan.
+// Offsets of up to kScanMax tiles in one launch: each CTA sums the counters before its own 1,024
+// (coalesced, one sector each, from L2) and scans its own, so no CTA waits for another.  8,161
+// counters took 19 us and 13,297 took 26 us in one CTA, and take 6 us here (cold caches); up to
+// 4,095 used to be scanned by the count's last CTA, but the fence and ticket that tells it so
+// costs every CTA of the count more than this launch: 2 M Gaussians on 2,040 tiles 103 -> 85 us
+// together, 100k on 1,024 tiles 16.9 -> 14.8 us.  The re-reads grow with the square of the tile
+// count, hence CUB's device scan beyond kScanMax.
 constexpr int kScanThreads = 1024;
-constexpr int kScanPerThread = 16;
-constexpr int64_t kSingleScanMax = (int64_t)kScanThreads * kScanPerThread;
-constexpr int64_t kFusedScanMax = 16 * kThreads;
+constexpr int64_t kScanMax = 1 << 16;
+
+__device__ __forceinline__ long long warp_inclusive(long long v, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
+  }
+  return v;
+}
 
 __global__ void __launch_bounds__(kScanThreads)
-    single_scan_kernel(const int* __restrict__ tile_count, int64_t items,
+    scan_counts_kernel(const int* __restrict__ tile_count, int64_t items,
                        long long* __restrict__ off64, int32_t* __restrict__ off32) {
   pdl_wait();
   pdl_trigger();
-  __shared__ long long warp_total[kScanThreads / 32];
+  __shared__ long long before[kScanThreads / 32], warp_total[kScanThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t base = (int64_t)tid * kScanPerThread;
-  long long run[kScanPerThread];
-  long long sum = 0;
+  const int64_t first = (int64_t)blockIdx.x * kScanThreads, idx = first + tid;
+  const long long own = idx < items ? tile_count[idx * kCounterStride] : 0;
+  long long pre = 0;
+#pragma unroll 4
+  for (int64_t k = tid; k < first; k += kScanThreads) pre += tile_count[k * kCounterStride];
 #pragma unroll
-  for (int k = 0; k < kScanPerThread; ++k) {
-    const int64_t idx = base + k;
-    run[k] = sum;
-    sum += idx < items ? tile_count[idx * kCounterStride] : 0;
+  for (int o = 16; o > 0; o >>= 1) pre += __shfl_xor_sync(0xffffffffu, pre, o);
+  const long long incl = warp_inclusive(own, lane);
+  if (lane == 31) {
+    before[warp] = pre;
+    warp_total[warp] = incl;
   }
-  long long incl = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) warp_total[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    const long long v = warp_total[lane];
-    long long w = v;
+    long long b = before[lane];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    warp_total[lane] = w - v;  // exclusive prefix of the warp totals
+    for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+    const long long v = warp_total[lane];
+    warp_total[lane] = b + warp_inclusive(v, lane) - v;  // offset of the warp's first counter
   }
   __syncthreads();
-  const long long prefix = warp_total[warp] + (incl - sum);
-#pragma unroll
-  for (int k = 0; k < kScanPerThread; ++k) {
-    const int64_t idx = base + k;
-    if (idx < items) {
-      const long long o = prefix + run[k];
-      off64[idx] = o;
-      off32[idx] = (int32_t)(o < 2147483647LL ? o : 2147483647LL);
-    }
+  if (idx < items) {
+    const long long o = warp_total[warp] + (incl - own);
+    off64[idx] = o;
+    off32[idx] = (int32_t)(o < 2147483647LL ? o : 2147483647LL);
   }
 }
 
@@ -444,10 +559,10 @@ __device__ __forceinline__ void warp_bitonic(int (&v)[K], int lane) {
 }
 
 template <int K>
-__device__ __forceinline__ void warp_sort_list(int32_t* __restrict__ g, int len, int lane) {
+__device__ __forceinline__ void warp_sort_list(const int32_t* src, int32_t* g, int len, int lane) {
   int v[K];
 #pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = 32 * k + lane < len ? g[32 * k + lane] : INT_MAX;
+  for (int k = 0; k < K; ++k) v[k] = 32 * k + lane < len ? src[32 * k + lane] : INT_MAX;
   warp_bitonic<K>(v, lane);
 #pragma unroll
   for (int k = 0; k < K; ++k)
@@ -471,17 +586,17 @@ __global__ void __launch_bounds__(kThreads) tile_sort_kernel(const int32_t* __re
   if (len <= 1) return;
   int32_t* g = gids + lo;
   if (len <= 32) {
-    warp_sort_list<1>(g, len, lane);
+    warp_sort_list<1>(g, g, len, lane);
   } else if (len <= 64) {
-    warp_sort_list<2>(g, len, lane);
+    warp_sort_list<2>(g, g, len, lane);
   } else if (len <= 128) {
-    warp_sort_list<4>(g, len, lane);
+    warp_sort_list<4>(g, g, len, lane);
   } else if (len <= 256) {
-    warp_sort_list<8>(g, len, lane);
+    warp_sort_list<8>(g, g, len, lane);
   } else if (len <= 512) {
-    warp_sort_list<16>(g, len, lane);
+    warp_sort_list<16>(g, g, len, lane);
   } else if (len <= kWarpSortMax) {
-    warp_sort_list<32>(g, len, lane);
+    warp_sort_list<32>(g, g, len, lane);
   } else if (lane == 0) {
     big_tiles[atomicAdd(big_count, 1)] = (int)t;
   }
@@ -555,6 +670,280 @@ __global__ void __launch_bounds__(1024) tile_sort_big_kernel(const int32_t* __re
   }
 }
 
+// The binned index's second stage puts each bin's ids into ascending order.  The ids of a list are
+// distinct, so there is one result whatever the way:
+//
+//   warp      short lists of a sparse tile set (see bin_sort_kernel): one warp's registers.
+//   buckets   up to kSortIds ids: spread over about as many buckets of equal id width (128 to
+//             1,024), each bucket finished by insertion, when no bucket holds more than kBucketIds.
+//   windows   long lists and clustered ids (a field in Morton order, as decoded ones are, has a
+//             tile's ids side by side): a bit per Gaussian of the image in shared memory, set from
+//             the bin and read back in order, one window of ids after the other, windows without
+//             ids skipped.  Costs the list plus 1/32 of the window, however the ids lie.
+//   rebuilt   a tile whose bin overflowed: the windows again, set by testing every record of the
+//             image instead.
+//
+// Bound by latency (a few dependent L2 reads and block-wide steps per tile), hence small CTAs, 10 to
+// an SM.  Lists of ~1,100 of 2 M ids on 2,040 tiles took 39 + 161 us in the warp and block sorts of
+// the plain form, lists of ~2,000 of 250 k on 1,024 tiles 35 + 81 us; here 29 and 22 us.
+constexpr int kSortThreads = 128;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortIds = 4096;
+constexpr int kBuckets = 1024;
+constexpr int kBucketIds = 24;
+constexpr int kWindowWords = kSortIds + kBuckets;
+constexpr int kWindowIds = 32 * kWindowWords;  // 163,840
+constexpr int kBitmapIds = 32 * kSortIds;      // a window below the bucket prefixes: 131,072
+
+// Exclusive prefix of v over the CTA's threads (tmp: kSortWarps + 1 words, ends holding the total
+// in tmp[kSortWarps]); holds two barriers.
+__device__ __forceinline__ int block_exclusive(int v, int* tmp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  __syncthreads();  // tmp may still be read from an earlier call
+  if (lane == 31) tmp[warp] = incl;
+  __syncthreads();
+  int base = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) {
+    const int t = tmp[w];
+    base += w < warp ? t : 0;
+    total += t;
+  }
+  if (threadIdx.x == 0) tmp[kSortWarps] = total;
+  return base + incl - v;
+}
+
+// Writes the ids of the set bits of words[0..nw) (bit b of word w is id first + 32 w + b) to g in
+// ascending order (at most `room` of them) and returns their number.  An odd run of words per thread
+// keeps the warp's reads on distinct banks.  Ends with a barrier.
+__device__ __forceinline__ int emit_bits(const uint32_t* words, int nw, int first, int32_t* g,
+                                         int room, int* tmp) {
+  const int per = ((nw + kSortThreads - 1) / kSortThreads) | 1;
+  const int w0 = min(nw, (int)threadIdx.x * per), w1 = min(nw, w0 + per);
+  int c = 0;
+  for (int w = w0; w < w1; ++w) c += __popc(words[w]);
+  int at = block_exclusive(c, tmp);
+  for (int w = w0; w < w1; ++w) {
+    uint32_t x = words[w];
+    while (x) {
+      if (at < room) g[at] = first + 32 * w + __ffs(x) - 1;
+      ++at;
+      x &= x - 1;
+    }
+  }
+  __syncthreads();
+  return tmp[kSortWarps];
+}
+
+// Orders a bin of len <= kSortIds ids by NB buckets of 2^shift ids and writes it to g; false,
+// with nothing written and the buckets' prefixes in hist, when some bucket is too full.  Called by
+// every thread.
+template <int NB>
+__device__ __forceinline__ bool bucket_sort(const int32_t* __restrict__ bin, int len, int first,
+                                            int count, int* buf, int* hist, int* tmp,
+                                            int32_t* __restrict__ g, int& shift) {
+  constexpr int kOwn = NB / kSortThreads;
+  shift = 0;
+  while (((count - 1) >> shift) >= NB) ++shift;
+#pragma unroll
+  for (int k = 0; k < kOwn; ++k) hist[k * kSortThreads + threadIdx.x] = 0;
+  __syncthreads();
+  for (int e = threadIdx.x; e < len; e += kSortThreads)
+    atomicAdd(&hist[(bin[e] - first) >> shift], 1);
+  __syncthreads();
+  int own[kOwn], sum = 0, most = 0;
+#pragma unroll
+  for (int k = 0; k < kOwn; ++k) {
+    own[k] = hist[kOwn * threadIdx.x + k];
+    sum += own[k];
+    most = max(most, own[k]);
+  }
+  int at = block_exclusive(sum, tmp);
+#pragma unroll
+  for (int k = 0; k < kOwn; ++k) {
+    hist[kOwn * threadIdx.x + k] = at;
+    at += own[k];
+  }
+  at -= sum;
+  if (!__syncthreads_and(most <= kBucketIds && len <= kSortIds)) return false;
+  for (int e = threadIdx.x; e < len; e += kSortThreads) {
+    const int id = bin[e];
+    buf[atomicAdd(&hist[(id - first) >> shift], 1)] = id;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kOwn; ++k) {  // the thread's own buckets, each by insertion
+    for (int x = at + 1; x < at + own[k]; ++x) {
+      const int v = buf[x];
+      int y = x;
+      for (; y > at && buf[y - 1] > v; --y) buf[y] = buf[y - 1];
+      buf[y] = v;
+    }
+    at += own[k];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < len; e += kSortThreads) g[e] = buf[e];
+  return true;
+}
+
+// One tile by the whole CTA (see above).  Every thread calls it.
+template <bool CULL>
+__device__ __noinline__ void cta_sort_bin(const Splat* __restrict__ rec, int64_t n, int ts,
+                                          const Frames& frames, float cutoff2, int t,
+                                          long long lo, int len, bool rebuild,
+                                          const int32_t* __restrict__ bin,
+                                          int32_t* __restrict__ gids, uint32_t* smem, int* tmp) {
+  const Frame fr = frame_of_tile(frames, t, n);
+  const int first = fr.gauss_first, count = fr.gauss_count;
+  int32_t* g = gids + lo;
+  auto set_bit = [&](int rel) { atomicOr(&smem[rel >> 5], 1u << (rel & 31)); };
+  auto clear = [&](int nw) {
+    for (int w = threadIdx.x; w < nw; w += kSortThreads) smem[w] = 0u;
+    __syncthreads();
+  };
+  if (rebuild) {
+    const int local = t - fr.first_tile;
+    const int gx = local % fr.tiles_x, gy = local / fr.tiles_x;
+    const int px0 = gx * ts, py0 = gy * ts;
+    int done = 0;
+    for (int w0 = 0; w0 < count; w0 += kWindowIds) {
+      const int ids = min(count - w0, kWindowIds), nw = (ids + 31) >> 5;
+      // a warp tests 32 consecutive records: their ballot is the bitmap's word
+#pragma unroll 4
+      for (int w = threadIdx.x >> 5; w < nw; w += kSortWarps) {
+        const int rel = 32 * w + (threadIdx.x & 31);
+        bool hit = false;
+        if (rel < ids) {
+          const int64_t i = (int64_t)first + w0 + rel;
+          const int4 b = reinterpret_cast<const int4*>(rec + i)[3];
+          hit = b.z > b.x && b.w > b.y && b.x < px0 + ts && b.z > px0 && b.y < py0 + ts &&
+                b.w > py0;
+          if (CULL && hit) hit = !culled(load_splat(rec, i), gx, gy, ts, cutoff2);
+        }
+        const unsigned word = __ballot_sync(0xffffffffu, hit);
+        if ((threadIdx.x & 31) == 0) smem[w] = word;
+      }
+      __syncthreads();
+      done += emit_bits(smem, nw, first + w0, g + done, len - done, tmp);
+    }
+    return;
+  }
+  int* buf = reinterpret_cast<int*>(smem);
+  int* hist = buf + kSortIds;
+  int shift = 0;
+  if (len <= 128) {
+    if (bucket_sort<128>(bin, len, first, count, buf, hist, tmp, g, shift)) return;
+  } else if (len <= 256) {
+    if (bucket_sort<256>(bin, len, first, count, buf, hist, tmp, g, shift)) return;
+  } else if (len <= 512) {
+    if (bucket_sort<512>(bin, len, first, count, buf, hist, tmp, g, shift)) return;
+  } else {
+    if (bucket_sort<kBuckets>(bin, len, first, count, buf, hist, tmp, g, shift)) return;
+  }
+  if (count <= kWindowIds) {  // one window
+    __syncthreads();  // every thread has left the buckets
+    const int nw = (count + 31) >> 5;
+    clear(nw);
+    for (int e = threadIdx.x; e < len; e += kSortThreads) set_bit(bin[e] - first);
+    __syncthreads();
+    emit_bits(smem, nw, first, g, len, tmp);
+    return;
+  }
+  const int nb = ((count - 1) >> shift) + 1;  // buckets in use
+  // windows of whole buckets; the bucket prefixes tell where each one's ids go.  The bitmap takes
+  // the shared memory below the buckets.
+  const int buckets = max(1, kBitmapIds >> shift);
+  for (int b0 = 0; b0 < nb; b0 += buckets) {
+    const int b1 = min(nb, b0 + buckets);
+    const int beg = hist[b0], end = b1 < nb ? hist[b1] : len;
+    if (beg == end) continue;  // the same in every thread
+    // a bucket wider than the bitmap (few buckets, or very many Gaussians) is cut in pieces
+    const int64_t r0 = (int64_t)b0 << shift, r1 = min((int64_t)count, (int64_t)b1 << shift);
+    int done = beg;
+    for (int64_t w0 = r0; w0 < r1; w0 += kBitmapIds) {
+      const int ids = (int)min(r1 - w0, (int64_t)kBitmapIds), nw = (ids + 31) >> 5;
+      clear(nw);
+      for (int e = threadIdx.x; e < len; e += kSortThreads) {
+        const int64_t rel = (int64_t)(bin[e] - first) - w0;
+        if (rel >= 0 && rel < ids) set_bit((int)rel);
+      }
+      __syncthreads();
+      done += emit_bits(smem, nw, first + (int)w0, g + done, len - done, tmp);
+    }
+  }
+}
+
+// Tiles per CTA: with up to kWarpTilesMax Gaussians per tile on average most lists are short, and a
+// CTA takes four tiles, each warp sorting its own in registers (lists up to kWarpIds; bitonic, no
+// block-wide step), longer ones then by the whole CTA in turn; beyond that one tile, by the CTA.
+// Lists of ~210 on 1,024 and 8,160 tiles: 8.5 and 27 us one tile at a time, 6 and 16 us by fours.
+constexpr int kWarpIds = 256;
+constexpr int64_t kWarpTilesMax = 128;
+
+template <bool CULL>
+__global__ void __launch_bounds__(kSortThreads)
+    bin_sort_kernel(const Splat* __restrict__ rec, int64_t n, int ts, Frames frames,
+                    float cutoff2, int64_t T, int tiles_per_cta,
+                    const long long* __restrict__ off64, const int* __restrict__ tile_count,
+                    const int32_t* __restrict__ bins, int K, int32_t* __restrict__ gids,
+                    int64_t cap, uint32_t* status) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ __align__(16) uint32_t smem[kWindowWords];  // a bitmap, or ids and buckets
+  __shared__ int tmp[kSortWarps + 1];
+  const int64_t t0 = (int64_t)blockIdx.x * tiles_per_cta;
+  const bool trusted = tile_count[2] == K;  // the bins belong to these counts
+  if (t0 == 0 && threadIdx.x == 0) {
+    const long long total = off64[T];
+    if (total > 2147483647LL) raise_status(status, SS_STATUS_INDEX_INT32);
+    if (total > cap) raise_status(status, SS_STATUS_INDEX_OVERFLOW);
+  }
+  bool mine = true;  // the CTA path takes the tile
+  if (tiles_per_cta > 1) {
+    const int lane = threadIdx.x & 31;
+    const int64_t t = t0 + (threadIdx.x >> 5);
+    mine = false;
+    if (t < T) {
+      const long long lo = off64[t], hi = off64[t + 1];
+      const int len = (int)(hi - lo);
+      if (hi <= cap && len > 0) {  // else truncated: the renderers scan all Gaussians
+        mine = len > kWarpIds || len > K || !trusted;
+        if (!mine) {
+          const int32_t* bin = bins + t * K;
+          int32_t* g = gids + lo;
+          if (len <= 32)
+            warp_sort_list<1>(bin, g, len, lane);
+          else if (len <= 64)
+            warp_sort_list<2>(bin, g, len, lane);
+          else if (len <= 128)
+            warp_sort_list<4>(bin, g, len, lane);
+          else
+            warp_sort_list<8>(bin, g, len, lane);
+        }
+      }
+    }
+    if (!__syncthreads_or(mine)) return;
+  }
+  for (int u = 0; u < tiles_per_cta; ++u) {
+    const int64_t t = t0 + u;
+    if (t >= T) break;
+    const long long lo = off64[t], hi = off64[t + 1];
+    const int len = (int)(hi - lo);  // at most the image's Gaussians
+    if (hi > cap || len == 0) continue;
+    const bool rebuild = len > K || !trusted;
+    if (tiles_per_cta > 1 && len <= kWarpIds && !rebuild) continue;  // a warp has sorted it
+    cta_sort_bin<CULL>(rec, n, ts, frames, cutoff2, (int)t, lo, len, rebuild, bins + t * K, gids,
+                       smem, tmp);
+    __syncthreads();
+  }
+}
+
 // Bits that hold every id below n and the pad 2^bits - 1 above them.
 int sort_key_bits(int64_t n) {
   int b = 1;
@@ -603,16 +992,14 @@ int index_count(const Frames& frames, int ts, int64_t T, const void* records, in
     return fail(SS_ERR_INVALID_ARGUMENT, "tile index workspace too small (%zu < %zu)",
                 workspace_bytes, index_workspace_bytes(T));
   cudaStream_t s = as_stream(stream);
-  IndexWorkspace w = carve(workspace, T);
+  IndexWorkspace w = carve(workspace, workspace_bytes, n, T);
   if (cudaMemsetAsync(w.tile_count, 0, sizeof(int) * kCounterStride * (T + 1), s) !=
       cudaSuccess)
     return check_launch("tile_index_count memset");
   const Splat* rec = static_cast<const Splat*>(records);
   float cutoff2 = sigma_cutoff * sigma_cutoff;
-  // the count kernel's last CTA scans up to kFusedScanMax counters (two rounds); larger sets
-  // up to kSingleScanMax take the 1024-thread scan kernel, beyond that CUB's device scan
-  const bool fused_scan = T + 1 <= kFusedScanMax;
-  const bool single_scan = T + 1 <= kSingleScanMax;
+  const bool one_scan = T + 1 <= kScanMax;
+  const bool binned = w.bins != nullptr;
   if (clear_bytes && (!clear || reinterpret_cast<uintptr_t>(clear) % 16 || clear_bytes % 16))
     return fail(SS_ERR_INVALID_ARGUMENT,
                 "clear region must be 16-byte aligned and a multiple of 16 bytes");
@@ -623,36 +1010,35 @@ int index_count(const Frames& frames, int ts, int64_t T, const void* records, in
       return fail(SS_ERR_INVALID_ARGUMENT, "records must be 16-byte aligned");
     int blocks = (int)((n + kThreads - 1) / kThreads);
     Splat* out = static_cast<Splat*>(const_cast<void*>(records));
-#define SS_PCOUNT(C, S)                                                                       \
-  launch("project_count_kernel", project_count_kernel<C, S>, blocks, kThreads, 0, s, *rs, n,   \
-         ts, frames, cutoff2, out, w.tile_count, T + 1, w.offsets64, tile_offsets,           \
-         static_cast<uint4*>(clear), (int64_t)(clear_bytes / 16))
+#define SS_PCOUNT(C, B)                                                                       \
+  launch("project_count_kernel", project_count_kernel<C, B>, blocks, kThreads, 0, s, *rs, n,   \
+         ts, frames, cutoff2, out, w.tile_count, static_cast<uint4*>(clear),                  \
+         (int64_t)(clear_bytes / 16), w.bins, w.bin_ids)
     if (ellipse_cull) {
-      if (fused_scan) SS_PCOUNT(true, true); else SS_PCOUNT(true, false);
+      if (binned) SS_PCOUNT(true, true); else SS_PCOUNT(true, false);
     } else {
-      if (fused_scan) SS_PCOUNT(false, true); else SS_PCOUNT(false, false);
+      if (binned) SS_PCOUNT(false, true); else SS_PCOUNT(false, false);
     }
 #undef SS_PCOUNT
     if ((rc = check_launch("project_count"))) return rc;
-    if (fused_scan) return SS_OK;
   } else if (n > 0 && T > 0) {
     int blocks = (int)((n + kThreads - 1) / kThreads);
-#define SS_COUNT(C, S)                                                                        \
-  launch("tile_count_kernel", tile_count_kernel<C, S>, blocks, kThreads, 0, s, rec, n, ts,     \
-         frames, cutoff2, w.tile_count, T + 1, w.offsets64, tile_offsets)
+#define SS_COUNT(C, B)                                                                        \
+  launch("tile_count_kernel", tile_count_kernel<C, B>, blocks, kThreads, 0, s, rec, n, ts,      \
+         frames, cutoff2, w.tile_count, w.bins, w.bin_ids)
     if (ellipse_cull) {
-      if (fused_scan) SS_COUNT(true, true); else SS_COUNT(true, false);
+      if (binned) SS_COUNT(true, true); else SS_COUNT(true, false);
     } else {
-      if (fused_scan) SS_COUNT(false, true); else SS_COUNT(false, false);
+      if (binned) SS_COUNT(false, true); else SS_COUNT(false, false);
     }
 #undef SS_COUNT
     if ((rc = check_launch("tile_count"))) return rc;
-    if (fused_scan) return SS_OK;
   }
   (void)status;
-  if (single_scan) {
-    launch("single_scan_kernel", single_scan_kernel, 1, kScanThreads, 0, s, w.tile_count, T + 1, w.offsets64,
-                                                  tile_offsets);
+  if (one_scan) {
+    launch("scan_counts_kernel", scan_counts_kernel,
+           (unsigned)((T + kScanThreads) / kScanThreads), kScanThreads, 0, s, w.tile_count, T + 1,
+           w.offsets64, tile_offsets);
     return check_launch("tile_offsets scan");
   }
   size_t sb = w.scan_bytes;
@@ -681,9 +1067,19 @@ int index_fill(const Frames& frames, int ts, int64_t T, const void* records, int
     return fail(SS_ERR_INVALID_ARGUMENT, "tile index workspace too small");
   if (T == 0) return SS_OK;
   cudaStream_t s = as_stream(stream);
-  IndexWorkspace w = carve(workspace, T);
+  IndexWorkspace w = carve(workspace, workspace_bytes, n, T);
   const Splat* rec = static_cast<const Splat*>(records);
   float cutoff2 = sigma_cutoff * sigma_cutoff;
+  if (w.bins) {  // the count left every tile's ids in its bin
+    const int per = n <= kWarpTilesMax * T ? kSortWarps : 1;
+#define SS_BIN(C)                                                                             \
+  launch("bin_sort_kernel", bin_sort_kernel<C>, (unsigned)((T + per - 1) / per), kSortThreads,  \
+         0, s, rec, n, ts, frames, cutoff2, T, per, w.offsets64, w.tile_count, w.bins,          \
+         w.bin_ids, tile_gids, gid_capacity, status)
+    if (ellipse_cull) SS_BIN(true); else SS_BIN(false);
+#undef SS_BIN
+    return check_launch("bin_sort");
+  }
   int64_t threads_needed = n > T + 1 ? n : T + 1;
   int blocks = (int)((threads_needed + kThreads - 1) / kThreads);
   int32_t* offsets32 = const_cast<int32_t*>(tile_offsets);
@@ -722,6 +1118,24 @@ int ss_tile_index_workspace_bytes(int64_t n, int height, int width, int tile_siz
   if (rc) return rc;
   if (!bytes) return fail(SS_ERR_INVALID_ARGUMENT, "null bytes pointer");
   *bytes = index_workspace_bytes(make_grid(height, width, tile_size).T);
+  return SS_OK;
+}
+
+int ss_tile_index_binned_workspace_bytes(int64_t n, int height, int width, int tile_size,
+                                         size_t* bytes) {
+  int rc = check_index_args(n, height, width, tile_size);
+  if (rc) return rc;
+  if (!bytes) return fail(SS_ERR_INVALID_ARGUMENT, "null bytes pointer");
+  *bytes = binned_workspace_bytes(n, make_grid(height, width, tile_size).T);
+  return SS_OK;
+}
+
+int ss_batch_tile_index_binned_workspace_bytes(const ss_batch* batch, int64_t n, size_t* bytes) {
+  Frames f;
+  int rc = frames_of_batch(batch, n, &f);
+  if (rc) return rc;
+  if (!bytes) return fail(SS_ERR_INVALID_ARGUMENT, "null bytes pointer");
+  *bytes = binned_workspace_bytes(n, batch->tiles);
   return SS_OK;
 }
 

@@ -118,6 +118,29 @@ __device__ __forceinline__ void support_rect(float mx, float my, long long rx, l
   y1 = (int)yh + 1;
 }
 
+// The same for radii that are whole floats >= 1 (a projection's), in 32-bit arithmetic where the
+// centre and radii are small enough for it to be exact: conversions to int64 run at a fraction
+// of the rate, and every Gaussian near an image takes the short way.
+__device__ __forceinline__ void support_rect_f(float mx, float my, float rx, float ry, int H,
+                                               int W, int& x0, int& y0, int& x1, int& y1) {
+  const float fx = rintf(mx), fy = rintf(my);
+  constexpr float kSmall = 536870912.0f;  // 2^29: sums of two stay below 2^31
+  if (fabsf(fx) < kSmall && fabsf(fy) < kSmall && rx < kSmall && ry < kSmall) {
+    const int ix = (int)fx, iy = (int)fy, ax = (int)rx, ay = (int)ry;
+    const int xl = max(ix - ax, 0), xh = min(ix + ax, W - 1);
+    const int yl = max(iy - ay, 0), yh = min(iy + ay, H - 1);
+    const bool any = xh >= xl && yh >= yl;
+    x0 = any ? xl : 0;
+    x1 = any ? xh + 1 : 0;
+    y0 = any ? yl : 0;
+    y1 = any ? yh + 1 : 0;
+    return;
+  }
+  const long long lim = 1LL << 40;
+  support_rect(mx, my, rx < 1e12f ? (long long)rx : lim, ry < 1e12f ? (long long)ry : lim, H, W,
+               x0, y0, x1, y1);
+}
+
 __device__ __forceinline__ Splat make_splat(float mx, float my, float a, float b, float c,
                                             float op, float cr, float cg, float cb, int x0,
                                             int y0, int x1, int y1) {
@@ -290,38 +313,60 @@ struct RSField {
   float dilation, cutoff;
 };
 
-// RS -> splat record of Gaussian i of frame fr, with its radii.  The conic follows
-// gaussians.py:275-300 and the radii gaussians.py:302-321; every product and sum is rounded
-// separately (no FMA contraction) so the radii's ceil() sees the same float the reference's
-// elementwise torch ops produce.
-__device__ __forceinline__ Splat rs_project_one(const RSField& f, int64_t i, const Frame& fr,
-                                                long long& rx, long long& ry) {
+// One Gaussian's parameters; loaded together, before the sine and cosine's branches, so that the
+// loads are in flight at once.
+struct RSParams {
+  float mx, my, ls0, ls1, th, cr, cg, cb, lg;
+};
+__device__ __forceinline__ RSParams rs_load(const RSField& f, int64_t i) {
+  RSParams p;
+  p.ls0 = __ldg(f.log_scales + 2 * i);
+  p.ls1 = __ldg(f.log_scales + 2 * i + 1);
+  p.th = __ldg(f.rotations + i);
+  p.mx = __ldg(f.means + 2 * i);
+  p.my = __ldg(f.means + 2 * i + 1);
+  p.cr = __ldg(f.colors + 3 * i);
+  p.cg = __ldg(f.colors + 3 * i + 1);
+  p.cb = __ldg(f.colors + 3 * i + 2);
+  p.lg = f.logits ? __ldg(f.logits + i) : 0.f;
+  return p;
+}
+
+// RS -> splat record of one Gaussian in an image of H x W, with its radii as whole floats (infinite
+// or NaN ones have a support without bound).  The conic follows gaussians.py:275-300 and the radii
+// gaussians.py:302-321; every product and sum is rounded separately (no FMA contraction) so the
+// radii's ceil() sees the same float the reference's elementwise torch ops produce.
+__device__ __forceinline__ Splat rs_project_one(const RSField& f, const RSParams& p, int H, int W,
+                                                float& rx, float& ry) {
   const float dilation = f.dilation, cutoff = f.cutoff;
-  float sx = expf(f.log_scales[2 * i]), sy = expf(f.log_scales[2 * i + 1]);
+  float sx = expf(p.ls0), sy = expf(p.ls1);
   float sx2 = __fmul_rn(sx, sx), sy2 = __fmul_rn(sy, sy);
-  float th = f.rotations[i];
-  float cs = cosf(th), sn = sinf(th);
+  float cs = cosf(p.th), sn = sinf(p.th);
   float cc = __fmul_rn(cs, cs), ss2 = __fmul_rn(sn, sn);
   // conic
-  float ix = __fdiv_rn(1.0f, __fadd_rn(sx2, dilation));
-  float iy = __fdiv_rn(1.0f, __fadd_rn(sy2, dilation));
+  float vx2 = __fadd_rn(sx2, dilation), vy2 = __fadd_rn(sy2, dilation);
+  float ix = __frcp_rn(vx2);
+  float iy = __frcp_rn(vy2);
   float a = __fadd_rn(__fmul_rn(cc, ix), __fmul_rn(ss2, iy));
   float b = __fmul_rn(__fmul_rn(cs, sn), __fsub_rn(ix, iy));
   float c = __fadd_rn(__fmul_rn(ss2, ix), __fmul_rn(cc, iy));
   // radii: ceil(cutoff * sqrt(var)) clamped >= 1
-  float vx2 = __fadd_rn(sx2, dilation), vy2 = __fadd_rn(sy2, dilation);
   float varx = __fadd_rn(__fmul_rn(cc, vx2), __fmul_rn(ss2, vy2));
   float vary = __fadd_rn(__fmul_rn(ss2, vx2), __fmul_rn(cc, vy2));
-  float fr_x = ceilf(__fmul_rn(cutoff, __fsqrt_rn(varx)));
-  float fr_y = ceilf(__fmul_rn(cutoff, __fsqrt_rn(vary)));
-  rx = isfinite(fr_x) ? (long long)fmaxf(fminf(fr_x, 1e15f), 1.0f) : (1LL << 40);
-  ry = isfinite(fr_y) ? (long long)fmaxf(fminf(fr_y, 1e15f), 1.0f) : (1LL << 40);
-  float op = f.logits ? 1.0f / (1.0f + expf(-f.logits[i])) : 1.0f;
-  float mx = f.means[2 * i], my = f.means[2 * i + 1];
+  const float fr_x = ceilf(__fmul_rn(cutoff, __fsqrt_rn(varx)));
+  const float fr_y = ceilf(__fmul_rn(cutoff, __fsqrt_rn(vary)));
+  const float unbounded = __int_as_float(0x7f800000);
+  rx = isfinite(fr_x) ? fmaxf(fminf(fr_x, 1e15f), 1.0f) : unbounded;
+  ry = isfinite(fr_y) ? fmaxf(fminf(fr_y, 1e15f), 1.0f) : unbounded;
+  float op = f.logits ? 1.0f / (1.0f + expf(-p.lg)) : 1.0f;
   int x0, y0, x1, y1;
-  support_rect(mx, my, rx, ry, fr.H, fr.W, x0, y0, x1, y1);
-  return make_splat(mx, my, a, b, c, op, f.colors[3 * i], f.colors[3 * i + 1],
-                    f.colors[3 * i + 2], x0, y0, x1, y1);
+  support_rect_f(p.mx, p.my, rx, ry, H, W, x0, y0, x1, y1);
+  return make_splat(p.mx, p.my, a, b, c, op, p.cr, p.cg, p.cb, x0, y0, x1, y1);
+}
+
+// Radius as the int64 the callers' radii tensors hold.
+__device__ __forceinline__ long long radius_i64(float r) {
+  return r <= 1e15f ? (long long)r : (1LL << 40);
 }
 
 // The backward's per-(tile, Gaussian) record in deterministic mode: nine moments, padded.

@@ -116,8 +116,10 @@ __global__ void project_rs_kernel(const float* __restrict__ means,
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const RSField f{means, log_scales, rotations, colors, logits, dilation, cutoff};
-  long long rx, ry;
-  const Splat sp = rs_project_one(f, i, frame_of_gaussian(frames, i, n), rx, ry);
+  const RSParams p = rs_load(f, i);
+  const Frame fr = frame_of_gaussian(frames, i, n);
+  float rx, ry;
+  const Splat sp = rs_project_one(f, p, fr.H, fr.W, rx, ry);
   store_splat(out + i, sp);
   if (conics_out) {
     conics_out[3 * i] = sp.a;
@@ -125,8 +127,8 @@ __global__ void project_rs_kernel(const float* __restrict__ means,
     conics_out[3 * i + 2] = sp.c;
   }
   if (radii_out) {
-    radii_out[2 * i] = rx;
-    radii_out[2 * i + 1] = ry;
+    radii_out[2 * i] = radius_i64(rx);
+    radii_out[2 * i + 1] = radius_i64(ry);
   }
 }
 

@@ -60,7 +60,7 @@ class RenderPlan:
         f32 = dict(device=d, dtype=torch.float32)
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, **f32)
         self.offsets = torch.zeros(self.T + 1, device=d, dtype=torch.int32)
-        self.idx_ws_bytes = _native.size_query("ss_tile_index_workspace_bytes", n, self.H, self.W,
+        self.idx_ws_bytes = _native.size_query("ss_tile_index_binned_workspace_bytes", n, self.H, self.W,
                                                self.tile_size)
         self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=d, dtype=torch.uint8)
         if self.capacity <= 0:

@@ -189,7 +189,7 @@ class EagerPlan:
         d = device
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, device=d, dtype=torch.float32)
         self.offsets = torch.zeros(self.T + 1, device=d, dtype=torch.int32)
-        self.idx_ws_bytes = _native.size_query("ss_tile_index_workspace_bytes", n, H, W,
+        self.idx_ws_bytes = _native.size_query("ss_tile_index_binned_workspace_bytes", n, H, W,
                                                tile_size)
         self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=d, dtype=torch.uint8)
         self.capacity = 0
@@ -262,7 +262,7 @@ def index_from_records(records, n: int, H: int, W: int, tile_size: int = 16,
     dev = records.device
     offsets = torch.empty(T + 1, device=dev, dtype=torch.int32)
     status = torch.zeros(1, device=dev, dtype=torch.int32)
-    ws_bytes = _native.size_query("ss_tile_index_workspace_bytes", n, H, W, tile_size)
+    ws_bytes = _native.size_query("ss_tile_index_binned_workspace_bytes", n, H, W, tile_size)
     ws = torch.empty(max(ws_bytes, 1), device=dev, dtype=torch.uint8)
     _native.call("ss_tile_index_count", _p(records), n, H, W, tile_size, int(ellipse_cull),
                  float(sigma_cutoff), _p(offsets), _p(ws), ws_bytes, _p(status), _stream())
