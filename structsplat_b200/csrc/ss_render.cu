@@ -44,8 +44,6 @@ constexpr int kEpilogueThreads = 256;
 
 template <int TS>
 struct Tiling {
-  // forward: one warp per 8x8 block of the tile
-  static constexpr int kFwdThreads = 32 * (TS / 8) * (TS / 8);
   // backward whole-list stage: what fits in 48 KB of static shared memory beside the pixels
   static constexpr int kBwdStageAll = TS == 16 ? 512 : 448;
 };
@@ -114,16 +112,19 @@ __device__ __forceinline__ unsigned block_cover(const float4 (*st)[4], int j, co
   return xm | (ym << 8);
 }
 
-// Ballot of the staged entries [0, min(m, 32)) covering the block at (sx0, sy0); lane l also
-// gets entry l's cover.  The rectangles come from `rects` when given, else from the records.
-__device__ __forceinline__ unsigned hit_cover(const float4 (*st)[4], const int4* rects, int m,
-                                              int sx0, int sy0, int lane, unsigned& cover) {
-  cover = 0u;
-  if (lane < m) {
-    const int4 b = rects ? rects[lane] : *reinterpret_cast<const int4*>(&st[lane][3]);
-    cover = block_cover(st, lane, b, sx0, sy0);
-  }
-  return __ballot_sync(0xffffffffu, cover != 0u);
+// The 8x8 blocks of the TS x TS tile at (tx0, ty0) that rectangle b touches: bit (TS / 8) row + col.
+template <int TS>
+__device__ __forceinline__ uint16_t block_mask(const int4& b, int tx0, int ty0) {
+  constexpr int kSide = TS / 8;
+  const int x0 = max(b.x - tx0, 0), x1 = min(b.z - tx0, TS);
+  const int y0 = max(b.y - ty0, 0), y1 = min(b.w - ty0, TS);
+  if (x1 <= x0 || y1 <= y0) return 0;
+  const unsigned cols = (2u << ((x1 - 1) >> 3)) - (1u << (x0 >> 3));
+  const unsigned rows = (2u << ((y1 - 1) >> 3)) - (1u << (y0 >> 3));
+  unsigned spread = 0;  // row r's bit at the first column of row r
+#pragma unroll
+  for (int r = 0; r < kSide; ++r) spread |= ((rows >> r) & 1u) << (kSide * r);
+  return (uint16_t)(spread * cols);
 }
 
 // Lists up to kStageAll Gaussians are staged whole (one barrier per tile; the warps then run
@@ -149,13 +150,64 @@ __device__ __forceinline__ void stage_range(float4 (*dst)[4], const Splat* rec,
   }
 }
 
+// stage_range of entries [0, m), m <= SLOTS, with the rectangles loaded through registers and
+// their block masks noted; the other three pieces are copies in flight.
+template <int TS, int NT, int SLOTS>
+__device__ __forceinline__ void stage_with_masks(float4 (*dst)[4], const Splat* rec,
+                                                 const TileList& L, int m, int4* rects,
+                                                 uint16_t* masks, int tx0, int ty0) {
+  constexpr int kIters = 4 * SLOTS / NT;
+  static_assert(kIters * NT == 4 * SLOTS && NT % 4 == 0, "pieces per thread");
+  const int piece = threadIdx.x & 3;
+  if constexpr (kIters <= 8) {
+    int4 r[kIters];
+#pragma unroll
+    for (int k = 0; k < kIters; ++k) {
+      const int slot = (threadIdx.x + k * NT) >> 2;
+      if (slot < m) {
+        const float4* from = reinterpret_cast<const float4*>(rec + L.gid(slot)) + piece;
+        if (piece == 3)
+          r[k] = *reinterpret_cast<const int4*>(from);
+        else
+          cp_async16(&dst[slot][piece], from);
+      }
+    }
+    if (piece == 3) {
+#pragma unroll
+      for (int k = 0; k < kIters; ++k) {
+        const int slot = (threadIdx.x + k * NT) >> 2;
+        if (slot < m) {
+          rects[slot] = r[k];
+          masks[slot] = block_mask<TS>(r[k], tx0, ty0);
+        }
+      }
+    }
+  } else {
+    for (int q = threadIdx.x; q < 4 * m; q += NT) {
+      const int slot = q >> 2;
+      const float4* from = reinterpret_cast<const float4*>(rec + L.gid(slot)) + piece;
+      if (piece == 3) {
+        const int4 r = *reinterpret_cast<const int4*>(from);
+        rects[slot] = r;
+        masks[slot] = block_mask<TS>(r, tx0, ty0);
+      } else {
+        cp_async16(&dst[slot][piece], from);
+      }
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Forward evaluation of one 8x8 pixel block by one warp, four Gaussians at a time.
 //
-// The block's hits (staged entries whose rectangle touches it and is not wholly underflowed, in
-// ascending list order) are listed per warp in shared memory; an entry is the staged slot
-// (bits 0-14) and its cover of the block (bits 16-23 block columns, 24-31 block rows).  The
-// lanes form four groups of eight: group g = lane >> 3 evaluates hit 4i + g, lane (c, g) the
+// When a tile's records are staged, the thread that looks at a record also finds the blocks its
+// rectangle touches (block_mask).  Each warp lists its block's hits from those masks, 32 entries
+// per step (a load, a ballot, a store), and only the hits, a quarter of the entries or fewer, get
+// the block's cover and the underflow test (cover_hits).  (Every warp used to find the cover of
+// every entry: at 3840x2160 with 800k Gaussians 84 of the forward's 342 us.)  An entry of the list
+// is the staged slot (bits 0-14) and its cover of the block (bits 16-23 block columns, 24-31 block
+// rows), in ascending list order.
+// The lanes form four groups of eight: group g = lane >> 3 evaluates hit 4i + g, lane (c, g) the
 // eight pixels of block column c, so the setup of a Gaussian (record loads, dx terms) serves
 // eight pixels, and rows k and k + 4 share packed (f32x2) arithmetic.  Each lane keeps a
 // partial sum per pixel and channel; the k-th hit of a block always goes to partial k mod 4,
@@ -163,8 +215,21 @@ __device__ __forceinline__ void stage_range(float4 (*dst)[4], const Splat* rec,
 // (p0 + p1) + (p2 + p3).  Every kernel that renders a tile (forward, fused render pass, fused
 // fit pass) evaluates its blocks this way, so their images agree bitwise.  A list is padded to
 // a multiple of four with the null record (opacity 0, no cover).
-constexpr int kQueueLen = 40;   // per-batch queue: ≥ 3 pending + 32 new hits + 3 padding
 constexpr int kCarrySlots = 4;  // per warp: staged slots for pending hits across a refill
+
+// A warp's hit list: entries in consecutive words.
+struct LinearList {
+  uint32_t* q;
+  __device__ __forceinline__ uint32_t* at(int i) const { return q + i; }
+};
+// The same in the tile's pixel inputs: the 1 KB of the block that the warp is working on, which
+// it writes only after the list is done with: eight runs of 32 words, one per pixel row.
+struct PixelList {
+  uint32_t* q;
+  int pitch;  // words from one pixel row to the next
+  __device__ __forceinline__ uint32_t* at(int i) const { return q + (i >> 5) * pitch + (i & 31); }
+};
+constexpr int kPixelListLen = 256;
 
 // Row offsets of the fast evaluation: for row pair k (rows k and k + 4) the row's index when
 // the 8-bit row mask covers it, and kRowMasked when not.  Added to dy0, a masked
@@ -197,12 +262,18 @@ __device__ __forceinline__ bool regular_record(const float4& p0, const float4& p
          fabsf(p1.y) + fabsf(p1.z) + fabsf(p1.w) + fabsf(cb) < 3.0e38f;
 }
 
-// Staged slots [0, m): true when every record is regular.  A CTA-wide barrier: every thread
-// of the CTA calls it.
-template <int NT>
-__device__ __forceinline__ bool all_regular(const float4 (*st)[4], int m) {
+// Looks at the staged slots [0, m): notes each rectangle's block mask (masks NULL: known already)
+// and returns true when every record is regular.  A CTA-wide barrier: every thread calls it.
+template <int TS, int NT>
+__device__ __forceinline__ bool check_records(const float4 (*st)[4], const int4* rects,
+                                              uint16_t* masks, int m, int tx0, int ty0) {
   bool ok = true;
-  for (int t = threadIdx.x; t < m; t += NT) ok = ok && regular_record(st[t][0], st[t][1], st[t][2].x);
+  for (int t = threadIdx.x; t < m; t += NT) {
+    ok = ok && regular_record(st[t][0], st[t][1], st[t][2].x);
+    if (masks)
+      masks[t] = block_mask<TS>(rects ? rects[t] : *reinterpret_cast<const int4*>(&st[t][3]), tx0,
+                                ty0);
+  }
   return __syncthreads_and(ok) != 0;
 }
 
@@ -254,57 +325,99 @@ __device__ __forceinline__ void eval4(const float4 (*st)[4], const uint32_t* q, 
   }
 }
 
-// Appends the hits among staged slots [slot0, slot0 + min(cnt, 32)) to the list q[0..qn).
-__device__ __forceinline__ int enqueue_hits(const float4 (*st)[4], const int4* rects, int slot0,
-                                            int cnt, int sx0, int sy0, int lane, uint32_t* q,
-                                            int qn) {
-  unsigned cover;
-  const unsigned hits = hit_cover(st + slot0, rects ? rects + slot0 : nullptr, cnt, sx0, sy0,
-                                  lane, cover);
-  if (cover) q[qn + __popc(hits & ((1u << lane) - 1u))] = (uint32_t)(slot0 + lane) | (cover << 16);
+// Appends the staged slots among [slot0, slot0 + min(cnt, 32)) whose mask has the block's bit to
+// the list [0, qn); their covers follow in cover_hits.
+template <typename List>
+__device__ __forceinline__ int enqueue_hits(const uint16_t* masks, int slot0, int cnt,
+                                            unsigned block_bit, int lane, const List& q, int qn) {
+  const bool hit = lane < cnt && (masks[slot0 + lane] & block_bit);
+  const unsigned hits = __ballot_sync(0xffffffffu, hit);
+  if (hit) *q.at(qn + __popc(hits & ((1u << lane) - 1u))) = (uint32_t)(slot0 + lane);
   return qn + __popc(hits);
+}
+
+// Both in one go, without masks: appends the entries among the staged slots [slot0, slot0 +
+// min(cnt, 32)) that cover the block, each lane finding its entry's cover.
+template <typename List>
+__device__ __forceinline__ int enqueue_covered(const float4 (*st)[4], const int4* rects,
+                                               int slot0, int cnt, int sx0, int sy0, int lane,
+                                               const List& q, int qn) {
+  unsigned cover = 0u;
+  if (lane < cnt) {
+    const int j = slot0 + lane;
+    cover = block_cover(st, j, rects ? rects[j] : *reinterpret_cast<const int4*>(&st[j][3]), sx0,
+                        sy0);
+  }
+  const unsigned hits = __ballot_sync(0xffffffffu, cover != 0u);
+  if (cover)
+    *q.at(qn + __popc(hits & ((1u << lane) - 1u))) = (uint32_t)(slot0 + lane) | (cover << 16);
+  return qn + __popc(hits);
+}
+
+// Gives the entries [p, qn) of the list their covers; those of no cover (block_cover) leave it.
+// Returns the new length.  The rectangles come from `rects` when given, else from the records.
+template <typename List>
+__device__ __forceinline__ int cover_hits(const float4 (*st)[4], const int4* rects, const List& q,
+                                          int p, int qn, int sx0, int sy0, int lane) {
+  __syncwarp();
+  int w = p;
+  for (int i = p; i < qn; i += 32) {
+    unsigned cover = 0u;
+    int slot = 0;
+    if (i + lane < qn) {
+      slot = (int)*q.at(i + lane);
+      const int4 b = rects ? rects[slot] : *reinterpret_cast<const int4*>(&st[slot][3]);
+      cover = block_cover(st, slot, b, sx0, sy0);
+    }
+    const unsigned hits = __ballot_sync(0xffffffffu, cover != 0u);  // all have read theirs
+    if (cover)
+      *q.at(w + __popc(hits & ((1u << lane) - 1u))) = (uint32_t)slot | (cover << 16);
+    w += __popc(hits);
+  }
+  return w;
 }
 
 // Evaluates the listed hits four at a time.  `all`: the last partial group too, padded with the
 // null record (the list ends empty); otherwise the remainder (< 4) moves to the front.  Returns
 // the new length.  The list needs room for 3 entries of padding.
-template <bool FADE>
-__device__ __forceinline__ int drain(const float4 (*st)[4], uint32_t* q, int qn, bool all,
+template <bool FADE, typename List>
+__device__ __forceinline__ int drain(const float4 (*st)[4], const List& q, int qn, bool all,
                                      bool exact, int null_slot, int lane, float fx, float fy0,
                                      float tail, float2 (&acc)[4][4]) {
   if (all && (qn & 3)) {
-    if (lane < 4 && lane >= (qn & 3)) q[(qn & ~3) + lane] = (uint32_t)null_slot;
+    if (lane < 4 && lane >= (qn & 3)) *q.at((qn & ~3) + lane) = (uint32_t)null_slot;
     qn = (qn + 3) & ~3;
   }
   __syncwarp();
   const int full = qn & ~3;
   if (exact) {
 #pragma unroll 1
-    for (int i = 0; i < full; i += 4) eval4<FADE, true>(st, q + i, lane, fx, fy0, tail, acc);
+    for (int i = 0; i < full; i += 4) eval4<FADE, true>(st, q.at(i), lane, fx, fy0, tail, acc);
   } else {
 #pragma unroll 1
-    for (int i = 0; i < full; i += 4) eval4<FADE, false>(st, q + i, lane, fx, fy0, tail, acc);
+    for (int i = 0; i < full; i += 4) eval4<FADE, false>(st, q.at(i), lane, fx, fy0, tail, acc);
   }
   const int r = qn - full;
   if (r == 0) return 0;
-  const uint32_t keep = lane < r ? q[full + lane] : 0u;
+  const uint32_t keep = lane < r ? *q.at(full + lane) : 0u;
   __syncwarp();
-  if (lane < r) q[lane] = keep;
+  if (lane < r) *q.at(lane) = keep;
   __syncwarp();
   return r;
 }
 
 // Before a staged chunk is refilled: the records of the pending hits q[0..qn) (qn < 4) move to
 // the warp's carry slots carry0 + i (a hit already there stays), and the list points at them.
-__device__ __forceinline__ void carry_pending(float4 (*st)[4], uint32_t* q, int qn, int carry0,
+template <typename List>
+__device__ __forceinline__ void carry_pending(float4 (*st)[4], const List& q, int qn, int carry0,
                                               int lane) {
   if (lane < 3 * qn) {  // pieces 0-2 hold what the evaluation reads
     const int i = lane / 3, piece = lane - 3 * i;
-    const int src = (int)(q[i] & 0x7fffu);
+    const int src = (int)(*q.at(i) & 0x7fffu);
     if (src != carry0 + i) st[carry0 + i][piece] = st[src][piece];
   }
   __syncwarp();
-  if (lane < qn) q[lane] = (q[lane] & 0xffff0000u) | (uint32_t)(carry0 + lane);
+  if (lane < qn) *q.at(lane) = (*q.at(lane) & 0xffff0000u) | (uint32_t)(carry0 + lane);
   __syncwarp();
 }
 
@@ -426,61 +539,84 @@ __device__ __forceinline__ void add_tile_loss(float loss_sum, float sq_sum, floa
 
 // Shared memory of the forward kernel (dynamic): the stage (whole lists up to kStageAll
 // records, or two halves of it for a streamed list) followed by every warp's carry slots and
-// the null record; the staged records' rectangles, packed; and every warp's hit list, which
+// the null record; the staged records' rectangles, packed, and block masks; and every warp's hit
+// list, which
 // after the block's last evaluation holds the block's 8x8 pixels (RGB rows, then den) on their
 // way out as whole float4 image rows.  One warp per 8x8 block.
 template <int TS>
 struct FwdSmem {
-  static constexpr int kWarps = (TS / 8) * (TS / 8);
-  static constexpr int kNullSlot = kStageAll + kWarps * kCarrySlots;
+  static constexpr int kThreads = 32 * (TS / 8) * (TS / 8);
+  static constexpr int kWarps = kThreads / 32;
+  // Two CTAs of a 32-px tile's 16 warps share an SM, eight of a 16-px tile's four (64 registers a
+  // thread either way), the stage as large as that leaves.  16-px tiles used to stage 512 records
+  // too, four CTAs to an SM: 18.0 -> 15.7 us for 20k Gaussians on 517x389.  Eight warps with two
+  // blocks each, four CTAs to an SM, were no gain for 32-px tiles: alone 312 us against 318 at
+  // 3840x2160, but the 1024x1024 step 125 us against 117, the kernel overlapping its neighbours
+  // less.
+  static constexpr int kCtas = 1024 / kThreads;
+  static constexpr int kStage = TS == 32 ? kStageAll : 256;
+  static constexpr int kNullSlot = kStage + kWarps * kCarrySlots;
   static constexpr int kSlots = kNullSlot + 1;
-  static constexpr int kListLen = kStageAll + 4;  // a whole stage's hits and padding
+  static constexpr int kListLen = kStage + 4;  // a whole stage's hits and padding
   static constexpr size_t kStageBytes = (size_t)kSlots * 4 * sizeof(float4);
-  static constexpr size_t kRectBytes = (size_t)kStageAll * sizeof(int4);
+  static constexpr size_t kRectBytes = (size_t)kStage * sizeof(int4);
   static constexpr size_t kListBytes = (size_t)kWarps * kListLen * sizeof(uint32_t);
   static constexpr size_t kRectOff = kStageBytes;
-  static constexpr size_t kListOff = kRectOff + kRectBytes;
+  static constexpr size_t kMaskBytes = (size_t)kStage * sizeof(uint16_t);
+  static constexpr size_t kMaskOff = kRectOff + kRectBytes;
+  static constexpr size_t kListOff = kMaskOff + kMaskBytes;
   static constexpr size_t kBytes = kListOff + kListBytes;
   static_assert(kListLen * sizeof(uint32_t) >= 8 * 32 * sizeof(float), "a block's pixels fit");
   static_assert(kListLen * sizeof(uint32_t) % 16 == 0 && kListOff % 16 == 0, "float4 rows");
 };
 
-// Accumulates one warp's 8x8 block over a tile's list, staged whole by the caller (who also
-// passed the barrier after it), or streamed here through two halves of the stage with the
-// pending hits carried across each refill (chunk 0 already in flight when `chunk0_issued`; the
-// stream ends with a barrier, after which the stage may be refilled).  `qcap` is the capacity
-// of the warp's list q: with room for a whole stage (or half) plus padding the hits are listed
-// first and evaluated in one run, otherwise batch by batch.  `exact`: the staged records were
-// checked (all_regular) and some is not regular.  Every thread of the CTA calls it: it holds
-// the CTA's barriers.
-template <int NT, bool FADE>
-__device__ __forceinline__ void accumulate_block(float4 (*stage)[4], int stage_slots,
-                                                 const Splat* __restrict__ rec,
-                                                 const TileList& L, uint32_t* q, int qcap,
-                                                 int carry0, int null_slot, bool active, int sx0,
-                                                 int sy0, int lane, float tail,
-                                                 float2 (&acc)[4][4], bool staged_whole,
-                                                 bool exact, bool chunk0_issued = false,
-                                                 int4* rects = nullptr) {
+// Lists the hits of block `block_bit` among staged slots [s0, s0 + m) after the p pending ones and
+// evaluates them four at a time (`all`: the last group padded), in runs as long as the list's
+// qcap entries allow.  Returns the hits left pending.  Without masks (NULL) every entry's cover is
+// found as it is listed.
+template <bool FADE, typename List>
+__device__ __forceinline__ int block_hits(const float4 (*st)[4], const int4* rects,
+                                          const uint16_t* masks, int s0, int m,
+                                          unsigned block_bit, const List& q, int qcap, int p,
+                                          bool all, bool exact, int null_slot, int sx0, int sy0,
+                                          int lane, float tail, float2 (&acc)[4][4]) {
   const float fx = (float)(sx0 + (lane & 7)), fy0 = (float)sy0;
-  int qn = 0;
-  if (staged_whole) {  // the caller staged the list and passed the barrier
-    const int m = (int)L.count;
-    if (active) {
-      const bool listed = qcap >= m + 4;
-      for (int base = 0; base < m; base += 32) {
-        qn = enqueue_hits(stage, rects, base, m - base, sx0, sy0, lane, q, qn);
-        if (!listed) qn = drain<FADE>(stage, q, qn, false, exact, null_slot, lane, fx, fy0, tail, acc);
-      }
-      drain<FADE>(stage, q, qn, true, exact, null_slot, lane, fx, fy0, tail, acc);
+  int qn = p;
+  for (int base = 0; base < m; base += 32) {
+    if (masks)
+      qn = enqueue_hits(masks, s0 + base, m - base, block_bit, lane, q, qn);
+    else
+      qn = enqueue_covered(st, rects, s0 + base, m - base, sx0, sy0, lane, q, qn);
+    if (qn + 32 + 3 > qcap && base + 32 < m) {
+      if (masks) qn = cover_hits(st, rects, q, p, qn, sx0, sy0, lane);
+      qn = p = drain<FADE>(st, q, qn, false, exact, null_slot, lane, fx, fy0, tail, acc);
     }
-    return;
   }
+  if (masks) qn = cover_hits(st, rects, q, p, qn, sx0, sy0, lane);
+  return drain<FADE>(st, q, qn, all, exact, null_slot, lane, fx, fy0, tail, acc);
+}
+
+// Accumulates one warp's 8x8 block (bit `block_bit` of the masks) over a tile's list that streams
+// through two halves of the stage, with the pending hits carried across each refill (chunk 0
+// already in flight when `chunk0_issued`; the stream ends with a barrier, after which the stage may
+// be refilled).  MASKS: by block masks; long lists are often of wide Gaussians that hit most blocks
+// (1024x1024, 250k heavy-tailed: 673 us for the forward without them, 710 us with), so only the
+// fused pass, whose streamed lists are mostly dense fields of small ones, uses them (1920x1080,
+// 2 M around 1 px: 945 -> 884 us).  Every thread of the CTA calls it: it holds the CTA's barriers.
+template <int TS, int NT, bool FADE, bool MASKS, typename List>
+__device__ __forceinline__ void stream_block(float4 (*stage)[4], int stage_slots,
+                                             const Splat* __restrict__ rec, const TileList& L,
+                                             const List& q, int qcap, int carry0, int null_slot,
+                                             bool active, unsigned block_bit, int tx0, int ty0,
+                                             int sx0, int sy0, int lane, float tail,
+                                             float2 (&acc)[4][4], uint16_t* masks,
+                                             bool chunk0_issued, int4* rects) {
   const int half = stage_slots / 2;
-  const bool listed = qcap >= half + 8;
   const int64_t count = L.count;
   const int nchunks = (int)((count + half - 1) / half);
   auto len = [&](int64_t k0) { return (int)(count - k0 < half ? count - k0 : half); };
+  bool exact = false;
+  int qn = 0;
   if (!chunk0_issued) {
     stage_range<NT>(stage, rec, L, 0, len(0), nullptr, rects);
     cp_async_commit();
@@ -494,29 +630,26 @@ __device__ __forceinline__ void accumulate_block(float4 (*stage)[4], int stage_s
     cp_async_wait_one();
     __syncthreads();
     const int m = len(k0), s0 = (c & 1) * half;
-    exact = exact || !all_regular<NT>(stage + s0, m);
+    exact = !check_records<TS, NT>(stage + s0, rects ? rects + s0 : nullptr,
+                                   MASKS ? masks + s0 : nullptr, m, tx0, ty0) || exact;
     if (active) {
-      for (int base = 0; base < m; base += 32) {
-        qn = enqueue_hits(stage, rects, s0 + base, m - base, sx0, sy0, lane, q, qn);
-        if (!listed) qn = drain<FADE>(stage, q, qn, false, exact, null_slot, lane, fx, fy0, tail, acc);
-      }
-      if (listed) qn = drain<FADE>(stage, q, qn, false, exact, null_slot, lane, fx, fy0, tail, acc);
-      if (c + 1 < nchunks) carry_pending(stage, q, qn, carry0, lane);
+      const bool last = c + 1 == nchunks;
+      qn = block_hits<FADE>(stage, rects, MASKS ? masks : nullptr, s0, m, block_bit, q, qcap, qn, last, exact,
+                            null_slot, sx0, sy0, lane, tail, acc);
+      if (!last) carry_pending(stage, q, qn, carry0, lane);
     }
     __syncthreads();
   }
-  if (active) drain<FADE>(stage, q, qn, true, exact, null_slot, lane, fx, fy0, tail, acc);
-  __syncthreads();
 }
 
 // Forward of one tile, one warp per 8x8 block.  LOSS == kNoLoss: writes out and den.
 // Otherwise (a fit iteration) it also evaluates the pixel loss against target and writes the
 // backward's per-pixel input pixel_grad = (dL/dnum_rgb, dL/dden) (out and den only when given)
 // and adds each image's loss and mean squared error into loss[2 b], loss[2 b + 1]
-// (finish_pixel).  Each warp lists its block's hits (accumulate_block), per staged chunk when
+// (finish_pixel).  Each warp lists its block's hits (enqueue_hits), per staged chunk when
 // the list streams.
 template <int TS, bool NORMALIZE, bool FADE, int LOSS>
-__global__ void __launch_bounds__(Tiling<TS>::kFwdThreads, 2)
+__global__ void __launch_bounds__(FwdSmem<TS>::kThreads, FwdSmem<TS>::kCtas)
     forward_kernel(const Splat* __restrict__ rec, int64_t n, const int32_t* __restrict__ gids,
                    int64_t cap, const int32_t* __restrict__ offsets, Frames frames, float eps,
                    float tail, float* __restrict__ out, float* __restrict__ den,
@@ -525,7 +658,7 @@ __global__ void __launch_bounds__(Tiling<TS>::kFwdThreads, 2)
   pdl_wait();
   pdl_trigger();
   using S = FwdSmem<TS>;
-  constexpr int NT = Tiling<TS>::kFwdThreads;
+  constexpr int NT = S::kThreads;
   extern __shared__ __align__(16) unsigned char fwd_smem[];
   float4(*stage)[4] = reinterpret_cast<float4(*)[4]>(fwd_smem);
   const int tile = blockIdx.x;
@@ -534,29 +667,42 @@ __global__ void __launch_bounds__(Tiling<TS>::kFwdThreads, 2)
   const int tx0 = (local % fr.tiles_x) * TS, ty0 = (local / fr.tiles_x) * TS;
   const int H = fr.H, W = fr.W;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int sx0 = tx0 + (warp % (TS / 8)) * 8, sy0 = ty0 + (warp / (TS / 8)) * 8;
   uint32_t* q = reinterpret_cast<uint32_t*>(fwd_smem + S::kListOff) + warp * S::kListLen;
   int4* rects = reinterpret_cast<int4*>(fwd_smem + S::kRectOff);
+  uint16_t* masks = reinterpret_cast<uint16_t*>(fwd_smem + S::kMaskOff);
+  const LinearList list{q};
   const TileList L = tile_list(gids, offsets, cap, fr, tile);
-  const bool whole = L.count <= kStageAll;
   if (threadIdx.x == 0) write_null_record(stage, S::kNullSlot);
+  const unsigned block_bit = 1u << warp;
+  const int sx0 = tx0 + (warp % (TS / 8)) * 8, sy0 = ty0 + (warp / (TS / 8)) * 8;
   float2 acc[4][4];
 #pragma unroll
   for (int k = 0; k < 4; ++k)
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch) acc[k][ch] = make_float2(0.f, 0.f);
-  bool exact = false;
-  if (whole) {
-    stage_range<NT>(stage, rec, L, 0, (int)L.count, nullptr, rects);
+  if (L.count <= S::kStage) {
+    // The rectangles come through registers, so that the block masks are known, and the hits
+    // listed, while the records are still on their way.
+    const int m = (int)L.count;
+    stage_with_masks<TS, NT, S::kStage>(stage, rec, L, m, rects, masks, tx0, ty0);
     cp_async_commit();
+    __syncthreads();
+    int qn = 0;
+    for (int base = 0; base < m; base += 32)
+      qn = enqueue_hits(masks, base, m - base, block_bit, lane, list, qn);
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    exact = !all_regular<NT>(stage, (int)L.count);
+    const bool exact = !check_records<TS, NT>(stage, rects, nullptr, m, tx0, ty0);
+    qn = cover_hits(stage, rects, list, 0, qn, sx0, sy0, lane);
+    drain<FADE>(stage, list, qn, true, exact, S::kNullSlot, lane, (float)(sx0 + (lane & 7)),
+                (float)sy0, tail, acc);
+  } else {
+    // a streamed list moves through two chunks of `chunk` records (at most half the stage)
+    stream_block<TS, NT, FADE, false>(stage, 2 * min(chunk, S::kStage / 2), rec, L, list,
+                                      S::kListLen, S::kStage + warp * kCarrySlots, S::kNullSlot,
+                                      true, block_bit, tx0, ty0, sx0, sy0, lane, tail, acc, masks,
+                                      false, rects);
   }
-  // a streamed list moves through two chunks of `chunk` records (at most half the stage)
-  accumulate_block<NT, FADE>(stage, 2 * chunk, rec, L, q, S::kListLen,
-                             kStageAll + warp * kCarrySlots, S::kNullSlot, true, sx0, sy0, lane,
-                             tail, acc, whole, exact, false, rects);
   float v[2][4];
   combine_groups(acc, lane, v);
   const int cx = lane & 7, r0 = block_first_row(lane);
@@ -686,7 +832,7 @@ __device__ __forceinline__ float4 finish_pixel_rt(int normalize, int loss_kind, 
 
 // Shared memory of the backward tile kernel (dynamic): the stage (plus, in the fused pass, every
 // warp's carry slots for the forward phase), the tile's per-pixel inputs, the staged ids, the
-// cost-class order and counters, and in the fused pass the warps' hit queues.
+// cost-class order and counters, and in the fused pass the staged records' block masks.
 template <int TS, int NT, bool FUSED>
 struct BwdSmem {
   static constexpr int kStageMax = Tiling<TS>::kBwdStageAll;
@@ -698,9 +844,8 @@ struct BwdSmem {
   static constexpr size_t kOrderOff = kGidOff + (size_t)kStageMax * sizeof(int);
   static constexpr size_t kClassOff = kOrderOff + (size_t)kStageMax * sizeof(int);
   static constexpr size_t kNextOff = kClassOff + 256 * sizeof(int);
-  static constexpr size_t kQueueOff = kNextOff + 16;
-  static constexpr size_t kBytes =
-      kQueueOff + (FUSED ? (size_t)kWarps * kQueueLen * sizeof(uint32_t) : 0);
+  static constexpr size_t kMaskOff = kNextOff + 16;
+  static constexpr size_t kBytes = kMaskOff + (FUSED ? (size_t)kStageMax * sizeof(uint16_t) : 0);
 };
 
 template <int TS, int NT>
@@ -959,15 +1104,15 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
     constexpr int kBlocks = (TS / 8) * (TS / 8);
     constexpr int kWarps = NT / 32;
     constexpr int kPer = (kBlocks + kWarps - 1) / kWarps;
-    uint32_t* q = reinterpret_cast<uint32_t*>(bwd_smem + S::kQueueOff) + warp * kQueueLen;
     const bool whole = L.count <= kStageMax;
+    uint16_t* masks = reinterpret_cast<uint16_t*>(bwd_smem + S::kMaskOff);
     constexpr int kNullSlot = S::kSlots - 1;
     if (threadIdx.x == 0) write_null_record(stage, kNullSlot);
     bool exact = false;
     if (whole) {
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
       __syncthreads();
-      exact = !all_regular<NT>(stage, (int)L.count);
+      exact = !check_records<TS, NT>(stage, nullptr, masks, (int)L.count, tx0, ty0);
     }
     const float per_value = pixel_loss_scale(H, W);
     float loss_sum = 0.f, sq_sum = 0.f;
@@ -981,12 +1126,18 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
       for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) acc[k][ch] = make_float2(0.f, 0.f);
-      accumulate_block<NT, FADE>(stage, kStageMax, rec, L, q, kQueueLen,
-                                 kStageMax + warp * kCarrySlots, kNullSlot, active, tx0 + bx,
-                                 ty0 + by, lane, tail, acc, whole, exact, i == 0);
+      const PixelList list{reinterpret_cast<uint32_t*>(pix + by * TS + bx), TS * 4};
+      if (!whole)
+        stream_block<TS, NT, FADE, true>(stage, kStageMax, rec, L, list, kPixelListLen,
+                                   kStageMax + warp * kCarrySlots, kNullSlot, active, 1u << b,
+                                   tx0, ty0, tx0 + bx, ty0 + by, lane, tail, acc, masks, i == 0,
+                                   nullptr);
+      else if (active)
+        block_hits<FADE>(stage, nullptr, masks, 0, (int)L.count, 1u << b, list, kPixelListLen, 0,
+                         true, exact, kNullSlot, tx0 + bx, ty0 + by, lane, tail, acc);
       if (!active) continue;
       float v[2][4];
-      combine_groups(acc, lane, v);
+      combine_groups(acc, lane, v);  // warp-synchronous: the list has been read
       const int lx = bx + (lane & 7), px = tx0 + lx;
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
@@ -1226,7 +1377,7 @@ void launch_forward_loss(int loss_kind, unsigned T, cudaStream_t s, const Splat*
                          const int32_t* gids, int64_t cap, const int32_t* offsets,
                          const Frames& f, float eps, float tail, float* out, float* den,
                          const float* target, float4* pixel_grad, float* loss, float ce2) {
-  constexpr int NT = Tiling<TS>::kFwdThreads;
+  constexpr int NT = FwdSmem<TS>::kThreads;
   const int c = g_forward_chunk[TS == 16 ? 0 : 1].load(std::memory_order_relaxed);
   const int chunk = c ? c : kStageAll / 2;
 #define SS_FWD(LOSS)                                                                          \
