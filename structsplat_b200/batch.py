@@ -22,7 +22,8 @@ from dataclasses import dataclass
 import torch
 
 from . import _native
-from .render import DEFAULT_EPS, RECORD_FLOATS, RENDER_TILE, _p, _stream, fade_tail, validate_eps
+from .render import (DEFAULT_EPS, RECORD_FLOATS, RENDER_TILE, _p, _stream, deterministic_mode,
+                     fade_tail, validate_eps)
 
 PARAM_NAMES = ("means", "log_scales", "rotations", "colors", "opacity_logits")
 LOSS_KINDS = {"l1": 0, "l2": 1, "charbonnier": 2}
@@ -172,6 +173,7 @@ class FitPlan:
         self.n = n
         self.tail = fade_tail(s.sigma_cutoff, s.fade_alpha)
         self.cull = s.fade_alpha >= 1.0
+        self.det = deterministic_mode(s.deterministic, self.cull)
         f32 = dict(device=d, dtype=torch.float32)
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, **f32)
         self.offsets = torch.zeros(batch.tiles + 1, device=d, dtype=torch.int32)
@@ -261,13 +263,17 @@ class FitPlan:
                      float(s.charbonnier_eps), _p(self.pixel_grad), _p(image), _p(den),
                      _p(self.loss), _p(self.status), _stream())
 
-    def backward(self):
+    # ``det``: the deterministic mode of a backward and its update when not the library's plain one
+    def _det(self, det):
+        return int(self.s.deterministic) if det is None else det
+
+    def backward(self, det=None):
         _native.call("ss_fit_backward", self.batch.ref, _p(self.records), self.n, _p(self.gids),
                      self.capacity, _p(self.offsets), float(self.tail), _p(self.pixel_grad),
-                     int(self.s.deterministic), _p(self.bwd_ws), self.bwd_ws_bytes,
-                     _p(self.status), _stream())
+                     self._det(det), _p(self.bwd_ws), self.bwd_ws_bytes, _p(self.status),
+                     _stream())
 
-    def forward_backward(self):
+    def forward_backward(self, det=None):
         """Forward, pixel loss and backward of every tile in one kernel (the loss gradient stays
         on chip); the same images, losses and moments as forward_loss() + backward()."""
         s = self.s
@@ -275,7 +281,7 @@ class FitPlan:
                      _p(self.gids), self.capacity, _p(self.offsets), int(s.normalize),
                      float(s.eps), float(self.tail), _p(self.target), LOSS_KINDS[s.pixel_loss],
                      float(s.charbonnier_eps), None, None, _p(self.loss),
-                     int(s.deterministic), _p(self.bwd_ws), self.bwd_ws_bytes, _p(self.status),
+                     self._det(det), _p(self.bwd_ws), self.bwd_ws_bytes, _p(self.status),
                      _stream())
 
     def ssim_term(self):
@@ -286,10 +292,10 @@ class FitPlan:
                      float(s.ssim_weight), _p(self.pixel_grad), _p(self.ssim), _p(self.ssim_ws),
                      self.ssim_ws_bytes, _stream())
 
-    def update(self):
+    def update(self, det=None):
         s = self.s
         _native.call("ss_fit_adam_update", self.batch.ref, _p(self.records), self.n,
-                     _p(self.gids), self.capacity, _p(self.offsets), int(s.deterministic),
+                     _p(self.gids), self.capacity, _p(self.offsets), self._det(det),
                      _p(self.bwd_ws), float(s.dilation), self._p_params, self._p_m, self._p_v,
                      self._lrs, float(s.betas[0]), float(s.betas[1]), float(s.adam_eps),
                      float(math.log(s.scale_min)), _p(self.log_hi), _p(self.step_state),
@@ -304,13 +310,13 @@ class FitPlan:
             self.ssim.zero_()
             self.forward_loss(image=self.image, den=self.den)
             self.ssim_term()
-            self.backward()
+            self.backward(self.det)
         elif self.s.use_fused():
-            self.forward_backward()
+            self.forward_backward(self.det)
         else:
             self.forward_loss()
-            self.backward()
-        self.update()
+            self.backward(self.det)
+        self.update(self.det)
 
     def render(self):
         """Current images (P,3) and the per-image [loss, mse] of the current field."""

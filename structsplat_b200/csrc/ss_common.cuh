@@ -380,6 +380,9 @@ constexpr int kPartialFloats = 12;
 //   partials  cap x 12 floats       keys_in / keys   cap uint32 (ids; n marks unused slots)
 //   order_in / order  cap int32      seg              2n int32 (segment begin, end)
 //   temp      the radix sort's scratch
+// In slot mode (kEntrySlots) no sort is needed: a Gaussian's partials have consecutive slots, one per
+// tile of its rectangle in ascending tile order, so seg alone tells where they lie.
+constexpr int kEntrySlots = SS_DETERMINISTIC_SLOTS;
 struct EntryOrder {
   float* partials;
   uint32_t* keys_in;
@@ -462,7 +465,8 @@ __device__ __forceinline__ void add_partial(const float* partials, int32_t e,
 // the warp calls it (active = false for a lane without a Gaussian).  A segment of at most
 // kLaneSegment entries is summed serially by its lane; a longer one by the whole warp (lane l
 // takes entries l, l + 32, ..., then a butterfly over the lanes), so one huge Gaussian does not
-// serialise its warp.  The order depends only on the segment's length.
+// serialise its warp.  The order depends only on the segment's length.  order NULL: the entries lie
+// at the segment's positions themselves.
 __device__ __forceinline__ void sum_entry_partials(const float* __restrict__ partials,
                                                    const int32_t* __restrict__ order,
                                                    const int32_t* __restrict__ seg, int64_t n,
@@ -476,7 +480,7 @@ __device__ __forceinline__ void sum_entry_partials(const float* __restrict__ par
     end = seg[n + g];
   }
   if (end - beg <= kLaneSegment)
-    for (int i = beg; i < end; ++i) add_partial(partials, order[i], acc);
+    for (int i = beg; i < end; ++i) add_partial(partials, order ? order[i] : i, acc);
   const int lane = threadIdx.x & 31;
   unsigned big = __ballot_sync(0xffffffffu, end - beg > kLaneSegment);
   while (big) {
@@ -486,7 +490,7 @@ __device__ __forceinline__ void sum_entry_partials(const float* __restrict__ par
     float t[kMoments];
 #pragma unroll
     for (int k = 0; k < kMoments; ++k) t[k] = 0.f;
-    for (int i = b + lane; i < e; i += 32) add_partial(partials, order[i], t);
+    for (int i = b + lane; i < e; i += 32) add_partial(partials, order ? order[i] : i, t);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll

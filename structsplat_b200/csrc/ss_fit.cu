@@ -280,7 +280,8 @@ int ss_fit_adam_update(const ss_batch* batch, const void* records, int64_t n,
   const unsigned blocks = (unsigned)(want < cap_blocks ? want : cap_blocks);
   if (deterministic) {
     const EntryOrder eo = entry_order_layout(workspace, n, gid_capacity);
-    launch("fit_grad_kernel", fit_grad_kernel<true>, blocks, kThreads, 0, s, rec, n, nullptr, eo.partials, eo.order,
+    launch("fit_grad_kernel", fit_grad_kernel<true>, blocks, kThreads, 0, s, rec, n, nullptr, eo.partials,
+                                                      deterministic == kEntrySlots ? nullptr : eo.order,
                                                       eo.seg, p.log_scales, p.rotations,
                                                       p.logits, dilation, gp);
   } else {

@@ -52,6 +52,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -136,17 +140,24 @@ constexpr int kStageAll = 512;
 // (piece 3) go to that packed array instead: the lanes of a warp reading 32 consecutive
 // entries' rectangles then hit distinct banks (at the 64-byte record stride every fourth
 // entry shares a bank group).
+// gid_dst receives the entries' ids, or with slot_base the first slot of each one's Gaussian.
 template <int NT>
 __device__ __forceinline__ void stage_range(float4 (*dst)[4], const Splat* rec,
                                             const TileList& L, int64_t k0, int m,
-                                            int* gid_dst = nullptr, int4* rect_dst = nullptr) {
+                                            int* gid_dst = nullptr, int4* rect_dst = nullptr,
+                                            const int32_t* slot_base = nullptr) {
   for (int q = threadIdx.x; q < 4 * m; q += NT) {
     const int slot = q >> 2, piece = q & 3;
     const int g = L.gid(k0 + slot);
     void* to = (rect_dst && piece == 3) ? static_cast<void*>(&rect_dst[slot])
                                         : static_cast<void*>(&dst[slot][piece]);
     cp_async16(to, reinterpret_cast<const float4*>(rec + g) + piece);
-    if (gid_dst && piece == 0) gid_dst[slot] = g;  // the backward's atomics need the id
+    if (gid_dst && piece == 0) {
+      if (slot_base)
+        cp_async4(&gid_dst[slot], slot_base + g);
+      else
+        gid_dst[slot] = g;  // the backward's atomics need the id
+    }
   }
 }
 
@@ -862,7 +873,8 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
                     const float4* __restrict__ pixel_grad, const int32_t* __restrict__ gids,
                     int64_t cap, const int32_t* __restrict__ offsets, Frames frames,
                     int normalize, float eps, float tail, float* __restrict__ moments,
-                    float* __restrict__ partials, uint32_t* status, FusedFit ff) {
+                    float* __restrict__ partials, const int32_t* __restrict__ slot_base,
+                    uint32_t* status, FusedFit ff) {
   pdl_wait();
   pdl_trigger();
   using S = BwdSmem<TS, NT, FUSED>;
@@ -885,11 +897,13 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
     if (threadIdx.x == 0) raise_status(status, SS_STATUS_DETERMINISTIC_TRUNCATED);
     return;
   }
+  if (!DETERMINISTIC) slot_base = nullptr;
   // the first records' copies are in flight while the pixel inputs load
   if (L.count <= kStageMax)
-    stage_range<NT>(stage, rec, L, 0, (int)L.count, stage_gid);
+    stage_range<NT>(stage, rec, L, 0, (int)L.count, stage_gid, nullptr, slot_base);
   else
-    stage_range<NT>(stage, rec, L, 0, (int)(L.count < kHalf ? L.count : kHalf), stage_gid);
+    stage_range<NT>(stage, rec, L, 0, (int)(L.count < kHalf ? L.count : kHalf), stage_gid, nullptr,
+                    slot_base);
   cp_async_commit();
   // every pixel input this thread wrote is finite (the underflowed-entry skip below needs it)
   bool pix_ok = true;
@@ -971,8 +985,8 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
               isfinite(p2.x) &&
               rect_min_q(p0.x, p0.y, p2.y, p2.z, p2.w, (float)rx0, (float)rx1, (float)ry0,
                          (float)ry1) > kUnderflowQ) {
-            r.z = r.x;
-            reinterpret_cast<int4*>(&st[t][3])->z = r.x;
+            r.w = r.y;  // the columns still tell the entry's slot
+            reinterpret_cast<int4*>(&st[t][3])->w = r.y;
           }
         }
         const int w = min(r.z - tx0, TS) - max(r.x - tx0, 0);
@@ -1070,13 +1084,19 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
     if (active && (DETERMINISTIC || walked)) {
       const int base = ((quad & 2) ? 5 : 0) + ((quad & 1) ? 3 : 0);
       const int cnt = (quad & 1) ? 2 : 3;
+      int64_t entry = L.first + k0 + j;
+      if (DETERMINISTIC && slot_base) {  // the tile's place among the tiles of the rectangle
+        const int4 r = *reinterpret_cast<const int4*>(&st[j][3]);
+        const int gx0 = r.x / TS, gw = (r.z - 1) / TS - gx0 + 1;
+        entry = gsm[j] + (int64_t)(ty0 / TS - r.y / TS) * gw + (tx0 / TS - gx0);
+      }
 #pragma unroll
       for (int s = 0; s < 3; ++s) {
         const int mo = base + s;
         if (s < cnt && mo < kMoments) {
-          if (DETERMINISTIC)
-            partials[(L.first + k0 + j) * kPartialFloats + mo] = b[s];
-          else
+          if (DETERMINISTIC) {
+            if (entry < cap) partials[entry * kPartialFloats + mo] = b[s];
+          } else
             atomicAdd(moments + (int64_t)mo * n + gsm[j], b[s]);
         }
       }
@@ -1160,7 +1180,8 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
       }
     }
     if (!whole) {  // chunk 0 again, with its ids, for the backward
-      stage_range<NT>(stage, rec, L, 0, (int)(L.count < kHalf ? L.count : kHalf), stage_gid);
+      stage_range<NT>(stage, rec, L, 0, (int)(L.count < kHalf ? L.count : kHalf), stage_gid,
+                      nullptr, slot_base);
       cp_async_commit();
     }
     if (ff.loss) add_tile_loss<NT>(loss_sum, sq_sum, per_value, ff.loss + 2 * fr.image);
@@ -1180,7 +1201,7 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
       const int64_t k0 = (int64_t)c * kHalf;
       if (c + 1 < nchunks)
         stage_range<NT>(buf[(c + 1) & 1], rec, L, k0 + kHalf, len(k0 + kHalf),
-                        stage_gid + ((c + 1) & 1) * kHalf);
+                        stage_gid + ((c + 1) & 1) * kHalf, nullptr, slot_base);
       cp_async_commit();
       cp_async_wait_one();
       __syncthreads();
@@ -1318,6 +1339,75 @@ __global__ void entry_segments_kernel(const uint32_t* __restrict__ keys, int64_t
   }
 }
 
+// Slot mode, before the backward: each Gaussian's partials get consecutive slots, one per tile of
+// its rectangle (its entries, in an index built without the ellipse cull).  A CTA reserves its
+// Gaussians' slots with one atomic; where they land varies from run to run, the order of a
+// Gaussian's partials does not.  An index that overflowed its capacity leaves no slots (the
+// gradients are zero and the backward raises SS_STATUS_DETERMINISTIC_TRUNCATED).  One pass over the
+// rectangles in place of keys, a radix sort of the whole capacity and segments, nine launches: 9
+// us against 150 us for 250k Gaussians with 2 M entries.
+__global__ void __launch_bounds__(kEpilogueThreads)
+    entry_slots_kernel(const Splat* __restrict__ rec, int64_t n, int ts,
+                       const int32_t* __restrict__ offsets, int64_t T, int64_t cap,
+                       unsigned* __restrict__ cursor, int32_t* __restrict__ seg) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ int warp_total[kEpilogueThreads / 32];
+  __shared__ unsigned cta_first;
+  const int64_t g = (int64_t)blockIdx.x * kEpilogueThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool room = offsets[T] <= cap;
+  int cnt = 0;
+  if (g < n && room) {
+    const int4 r = reinterpret_cast<const int4*>(rec + g)[3];
+    if (r.z > r.x && r.w > r.y)
+      cnt = ((r.z - 1) / ts - r.x / ts + 1) * ((r.w - 1) / ts - r.y / ts + 1);
+  }
+  int incl = cnt;  // the total is at most the capacity, below 2^31
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_total[warp] = incl;
+  __syncthreads();
+  int before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kEpilogueThreads / 32; ++w) {
+    before += w < warp ? warp_total[w] : 0;
+    total += warp_total[w];
+  }
+  if (threadIdx.x == 0) cta_first = atomicAdd(cursor, (unsigned)total);
+  __syncthreads();
+  if (g >= n) return;
+  const int beg = room ? (int)cta_first + before + incl - cnt : 0;
+  seg[g] = beg;
+  seg[n + g] = beg + cnt;
+}
+
+int assign_entry_slots(const void* records, int64_t n, int ts, const int32_t* offsets, int64_t T,
+                       int64_t cap, void* ws, cudaStream_t s) {
+  const EntryOrder eo = entry_order_layout(ws, n, cap);
+  if (cap == 0) {
+    cudaMemsetAsync(eo.seg, 0, sizeof(int32_t) * 2 * n, s);
+    return check_launch("entry segments zero-fill");
+  }
+  cudaMemsetAsync(eo.keys_in, 0, sizeof(unsigned), s);  // the cursor: no keys in this mode
+  launch("entry_slots_kernel", entry_slots_kernel,
+         (unsigned)((n + kEpilogueThreads - 1) / kEpilogueThreads), kEpilogueThreads, 0, s,
+         static_cast<const Splat*>(records), n, ts, offsets, T, cap, eo.keys_in, eo.seg);
+  return check_launch("entry slots");
+}
+
+// First slot of each Gaussian (slot mode) or NULL.
+const int32_t* slot_base_of(void* ws, int64_t n, int64_t cap, int deterministic) {
+  return deterministic == kEntrySlots ? entry_order_layout(ws, n, cap).seg : nullptr;
+}
+// The partials' order for the per-Gaussian sums: NULL in slot mode.
+const int32_t* partial_order(const EntryOrder& eo, int deterministic) {
+  return deterministic == kEntrySlots ? nullptr : eo.order;
+}
+
 int key_bits(int64_t n) {
   int b = 1;
   while (b < 32 && ((int64_t)1 << b) <= n) ++b;
@@ -1414,16 +1504,17 @@ void launch_forward(int loss_kind, unsigned T, cudaStream_t s, const Splat* rec,
 std::atomic<int> g_backward_warps[2] = {{0}, {0}};
 
 template <int TS, int NT, bool PIXGRAD>
-void launch_backward_nt(unsigned T, cudaStream_t s, bool deterministic, const float* grad_out,
+void launch_backward_nt(unsigned T, cudaStream_t s, int deterministic, const float* grad_out,
                         const Splat* rec, int64_t n, const float* den, const float* out,
                         const float4* pixel_grad, const int32_t* gids, int64_t cap,
                         const int32_t* offsets, const Frames& f, int normalize, float eps,
                         float tail, float* ws, uint32_t* status) {
   const bool fade = tail > 0.0f;
+  const int32_t* slots = slot_base_of(ws, n, cap, deterministic);
 #define SS_BWD(FADE, DET)                                                                     \
   launch_smem("backward_kernel", backward_kernel<TS, NT, FADE, DET, PIXGRAD>, T, NT,         \
               (BwdSmem<TS, NT, false>::kBytes), s, grad_out, rec, n, den, out, pixel_grad,   \
-              gids, cap, offsets, f, normalize, eps, tail, ws, ws, status, FusedFit{})
+              gids, cap, offsets, f, normalize, eps, tail, ws, ws, slots, status, FusedFit{})
   if (deterministic) {
     if (fade) SS_BWD(true, true); else SS_BWD(false, true);
   } else {
@@ -1433,7 +1524,7 @@ void launch_backward_nt(unsigned T, cudaStream_t s, bool deterministic, const fl
 }
 
 template <int TS, bool PIXGRAD>
-void launch_backward(unsigned T, cudaStream_t s, bool deterministic, const float* grad_out,
+void launch_backward(unsigned T, cudaStream_t s, int deterministic, const float* grad_out,
                      const Splat* rec, int64_t n, const float* den, const float* out,
                      const float4* pixel_grad, const int32_t* gids, int64_t cap,
                      const int32_t* offsets, const Frames& f, int normalize, float eps,
@@ -1452,15 +1543,16 @@ void launch_backward(unsigned T, cudaStream_t s, bool deterministic, const float
 
 // The fused fit tile pass (forward + loss + backward in one CTA per tile).
 template <int TS, int NT>
-void launch_fused_nt(unsigned T, cudaStream_t s, bool deterministic, const Splat* rec, int64_t n,
+void launch_fused_nt(unsigned T, cudaStream_t s, int deterministic, const Splat* rec, int64_t n,
                      const int32_t* gids, int64_t cap, const int32_t* offsets, const Frames& f,
                      int normalize, float eps, float tail, float* ws, uint32_t* status,
                      const FusedFit& ff) {
   const bool fade = tail > 0.0f;
+  const int32_t* slots = slot_base_of(ws, n, cap, deterministic);
 #define SS_FUS(FADE, DET)                                                                       \
   launch_smem("fit_tile_kernel", backward_kernel<TS, NT, FADE, DET, false, true>, T, NT,     \
               (BwdSmem<TS, NT, true>::kBytes), s, nullptr, rec, n, nullptr, nullptr, nullptr, \
-              gids, cap, offsets, f, normalize, eps, tail, ws, ws, status, ff)
+              gids, cap, offsets, f, normalize, eps, tail, ws, ws, slots, status, ff)
   if (deterministic) {
     if (fade) SS_FUS(true, true); else SS_FUS(false, true);
   } else {
@@ -1470,7 +1562,7 @@ void launch_fused_nt(unsigned T, cudaStream_t s, bool deterministic, const Splat
 }
 
 template <int TS>
-void launch_fused(unsigned T, cudaStream_t s, bool deterministic, const Splat* rec, int64_t n,
+void launch_fused(unsigned T, cudaStream_t s, int deterministic, const Splat* rec, int64_t n,
                   const int32_t* gids, int64_t cap, const int32_t* offsets, const Frames& f,
                   int normalize, float eps, float tail, float* ws, uint32_t* status,
                   const FusedFit& ff) {
@@ -1517,6 +1609,10 @@ int render_backward_tiles(const Frames& f, int ts, int64_t T, const float* grad_
     return fail(SS_ERR_INVALID_ARGUMENT, "deterministic backward needs capacity < 2^31");
   const Splat* rec = static_cast<const Splat*>(records);
   const float4* pg = reinterpret_cast<const float4*>(pixel_grad);
+  int rc;
+  if (deterministic == kEntrySlots &&
+      (rc = assign_entry_slots(records, n, ts, offsets, T, cap, ws, s)))
+    return rc;
   if (pixel_grad) {
     if (ts == 16)
       launch_backward<16, true>((unsigned)T, s, deterministic, grad_out, rec, n, den, out, pg,
@@ -1532,8 +1628,8 @@ int render_backward_tiles(const Frames& f, int ts, int64_t T, const float* grad_
       launch_backward<32, false>((unsigned)T, s, deterministic, grad_out, rec, n, den, out, pg,
                                  gids, cap, offsets, f, normalize, eps, tail, ws, status);
   }
-  int rc = check_launch("render_backward");
-  if (rc || !deterministic) return rc;
+  rc = check_launch("render_backward");
+  if (rc || !deterministic || deterministic == kEntrySlots) return rc;
   return order_entries(gids, offsets, T, cap, n, ws, s);
 }
 
@@ -1580,7 +1676,7 @@ int render_backward(const Frames& f, int ts, int64_t T, int64_t npx, const float
   if (deterministic) {
     const EntryOrder eo = entry_order_layout(ws, n, cap);
     launch("reduce_partials_kernel", reduce_partials_kernel, gblocks, kEpilogueThreads, 0, s, 
-        rec, n, eo.partials, eo.order, eo.seg, has_opacity, grad_means, grad_conics,
+        rec, n, eo.partials, partial_order(eo, deterministic), eo.seg, has_opacity, grad_means, grad_conics,
         grad_colors, grad_opacities);
   } else
     launch("finalize_moments_kernel", finalize_moments_kernel, gblocks, kEpilogueThreads, 0, s, 
@@ -1755,7 +1851,7 @@ int ss_render_backward_finalize(const void* records, int64_t n, const int32_t* t
   if (deterministic) {
     const EntryOrder eo = entry_order_layout(const_cast<float*>(ws), n, gid_capacity);
     launch("reduce_partials_kernel", reduce_partials_kernel, gblocks, kEpilogueThreads, 0, s, 
-        rec, n, eo.partials, eo.order, eo.seg, has_opacity, grad_means, grad_conics,
+        rec, n, eo.partials, partial_order(eo, deterministic), eo.seg, has_opacity, grad_means, grad_conics,
         grad_colors, grad_opacities);
   } else
     launch("finalize_moments_kernel", finalize_moments_kernel, gblocks, kEpilogueThreads, 0, s, 
@@ -1785,7 +1881,7 @@ int ss_render_backward_finalize_rs(const void* records, int64_t n, const int32_t
   if (deterministic) {
     const EntryOrder eo = entry_order_layout(const_cast<float*>(ws), n, gid_capacity);
     launch("finalize_rs_kernel", finalize_rs_kernel<true>, gblocks, kEpilogueThreads, 0, s, 
-        rec, n, eo.partials, eo.order, eo.seg, log_scales, rotations, opacity_logits, dilation,
+        rec, n, eo.partials, partial_order(eo, deterministic), eo.seg, log_scales, rotations, opacity_logits, dilation,
         grad_means, grad_log_scales, grad_rotations, grad_colors, grad_opacity_logits);
   } else {
     launch("finalize_rs_kernel", finalize_rs_kernel<false>, gblocks, kEpilogueThreads, 0, s, 
@@ -1907,6 +2003,9 @@ int ss_fit_forward_backward(const ss_batch* batch, const void* records, int64_t 
   ff.grad_out = nullptr;
   const Splat* rec = static_cast<const Splat*>(records);
   float* ws = static_cast<float*>(workspace);
+  if (deterministic == kEntrySlots && n > 0 &&
+      (rc = assign_entry_slots(records, n, batch->tile_size, tile_offsets, T, gid_capacity, ws, s)))
+    return rc;
   if (batch->tile_size == 16)
     launch_fused<16>((unsigned)T, s, deterministic, rec, n, tile_gids, gid_capacity,
                      tile_offsets, f, normalize, eps, fade_tail, ws, status, ff);
@@ -1914,7 +2013,7 @@ int ss_fit_forward_backward(const ss_batch* batch, const void* records, int64_t 
     launch_fused<32>((unsigned)T, s, deterministic, rec, n, tile_gids, gid_capacity,
                      tile_offsets, f, normalize, eps, fade_tail, ws, status, ff);
   if ((rc = check_launch("fit forward + backward"))) return rc;
-  if (!deterministic || n == 0) return SS_OK;
+  if (!deterministic || deterministic == kEntrySlots || n == 0) return SS_OK;
   return order_entries(tile_gids, tile_offsets, T, gid_capacity, n, workspace, s);
 }
 
@@ -1948,6 +2047,9 @@ int ss_render_forward_backward(const void* records, int64_t n, const int32_t* ti
   const Frames f = single_frame(height, width, tile_size);
   const Splat* rec = static_cast<const Splat*>(records);
   float* ws = static_cast<float*>(workspace);
+  if (deterministic == kEntrySlots && n > 0 &&
+      (rc = assign_entry_slots(records, n, tile_size, tile_offsets, T, gid_capacity, ws, s)))
+    return rc;
   if (tile_size == 16)
     launch_fused<16>((unsigned)T, s, deterministic, rec, n, tile_gids, gid_capacity,
                      tile_offsets, f, normalize, eps, fade_tail, ws, status, ff);
@@ -1955,7 +2057,7 @@ int ss_render_forward_backward(const void* records, int64_t n, const int32_t* ti
     launch_fused<32>((unsigned)T, s, deterministic, rec, n, tile_gids, gid_capacity,
                      tile_offsets, f, normalize, eps, fade_tail, ws, status, ff);
   if ((rc = check_launch("render forward + backward"))) return rc;
-  if (!deterministic || n == 0) return SS_OK;
+  if (!deterministic || deterministic == kEntrySlots || n == 0) return SS_OK;
   return order_entries(tile_gids, tile_offsets, T, gid_capacity, n, workspace, s);
 }
 

@@ -14,8 +14,8 @@ from torch.autograd.function import once_differentiable
 
 from . import _native
 from .render import (DEFAULT_EPS, EAGER_PLANS, RECORD_FLOATS, RENDER_TILE, TileIndex, _backward,
-                     _forward, _p, _stream, fade_tail, index_from_records, resolve_fade_alpha,
-                     tile_grid, validate_eps)
+                     _forward, _p, _stream, deterministic_mode, fade_tail, index_from_records,
+                     resolve_fade_alpha, tile_grid, validate_eps)
 
 
 def project(means, log_scales, rotations, colors, opacity_logits, H: int, W: int,
@@ -119,8 +119,8 @@ class _B200RenderRS(Function):
                 rec, gids, offsets, status = saved[7:]
                 index = TileIndex(gids, offsets, ts, status)
             g_means, g_conics, g_colors, g_opac = _backward(
-                grad_out, rec, n, den, out, index, H, W, normalize, eps, tail, has_op, det,
-                grad_out.device)
+                grad_out, rec, n, den, out, index, H, W, normalize, eps, tail, has_op,
+                deterministic_mode(det, cull), grad_out.device)
             g_ls = torch.empty_like(log_scales)
             g_rot = torch.empty_like(rotations)
             g_logits = torch.empty_like(logits) if has_op else None

@@ -20,8 +20,8 @@ from dataclasses import dataclass, field
 import torch
 
 from . import _native
-from .render import (DEFAULT_EPS, RECORD_FLOATS, RENDER_TILE, _p, _stream, fade_tail, tile_grid,
-                     validate_eps)
+from .render import (DEFAULT_EPS, RECORD_FLOATS, RENDER_TILE, _p, _stream, deterministic_mode,
+                     fade_tail, tile_grid, validate_eps)
 
 PARAM_NAMES = ("means", "log_scales", "rotations", "colors", "opacity_logits")
 
@@ -56,6 +56,7 @@ class RenderPlan:
         self.T = tiles_x * tiles_y
         self.tail = fade_tail(self.sigma_cutoff, self.fade_alpha)
         self.cull = self.fade_alpha >= 1.0
+        self.det = deterministic_mode(self.deterministic, self.cull)
         d, n = self.device, self.n
         f32 = dict(device=d, dtype=torch.float32)
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, **f32)
@@ -145,8 +146,8 @@ class RenderPlan:
             return
         if not self.deterministic and not moments_zeroed:
             self.bwd_ws.zero_()
-        self.backward_tiles(grad_out)
-        self.finalize_rs(params)
+        self.backward_tiles(grad_out, self.det)
+        self.finalize_rs(params, self.det)
 
     def render_input_grads(self, grad_out):
         """Gradients w.r.t. the render inputs (means, conics, colours, opacities) into
@@ -160,12 +161,14 @@ class RenderPlan:
                      _p(self.status), _stream())
         return self.g_means, self.g_conics, self.g_colors, self.g_opac
 
-    def backward_tiles(self, grad_out):
-        """Only the backward tile kernel (fast mode: adds into the moments), for timing."""
+    def backward_tiles(self, grad_out, det=None):
+        """Only the backward tile kernel (fast mode: adds into the moments), for timing.  ``det``:
+        the deterministic mode when not the library's plain one; finalize_rs takes the same."""
+        det = int(self.deterministic) if det is None else det
         _native.call("ss_render_backward_moments", _p(grad_out), None, _p(self.records), self.n,
                      _p(self.den), _p(self.image), _p(self.gids), self.capacity,
                      _p(self.offsets), self.H, self.W, self.tile_size, int(self.normalize),
-                     float(self.eps), float(self.tail), int(self.deterministic), _p(self.bwd_ws),
+                     float(self.eps), float(self.tail), det, _p(self.bwd_ws),
                      self.bwd_ws_bytes, _p(self.status), _stream())
 
     def forward(self, params, clear_moments: bool = False):
@@ -191,24 +194,26 @@ class RenderPlan:
             return self.grads()
         self.project_count(params, clear_moments=True)
         self.fill()
-        self.tile_pass(grad_out)
+        self.tile_pass(grad_out, self.det)
         if self.n:
-            self.finalize_rs(params)
+            self.finalize_rs(params, self.det)
         return self.grads()
 
-    def tile_pass(self, grad_out):
+    def tile_pass(self, grad_out, det=None):
         """Only the fused forward + backward tile kernel (fast mode: adds into the moments)."""
+        det = int(self.deterministic) if det is None else det
         if self.H * self.W:
             _native.call("ss_render_forward_backward", _p(self.records), self.n, _p(self.gids),
                          self.capacity, _p(self.offsets), self.H, self.W, self.tile_size,
                          int(self.normalize), float(self.eps), float(self.tail), _p(grad_out),
-                         _p(self.image), _p(self.den), int(self.deterministic), _p(self.bwd_ws),
+                         _p(self.image), _p(self.den), det, _p(self.bwd_ws),
                          self.bwd_ws_bytes, _p(self.status), _stream())
 
-    def finalize_rs(self, params):
+    def finalize_rs(self, params, det=None):
+        det = int(self.deterministic) if det is None else det
         _native.call("ss_render_backward_finalize_rs", _p(self.records), self.n, _p(self.gids),
                      self.capacity, _p(self.offsets), self.H, self.W, self.tile_size,
-                     int(self.deterministic), _p(self.bwd_ws), _p(params["log_scales"]),
+                     det, _p(self.bwd_ws), _p(params["log_scales"]),
                      _p(params["rotations"]),
                      _p(params.get("opacity_logits") if self.has_opacity else None),
                      float(self.dilation), _p(self.g_means), _p(self.g_log_scales),

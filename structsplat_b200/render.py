@@ -75,6 +75,13 @@ def fade_tail(sigma_cutoff: float, alpha: float) -> float:
     return float(np.float32(alpha * math.exp(-0.5 * float(sigma_cutoff) ** 2)))
 
 
+def deterministic_mode(deterministic: bool, cull: bool) -> int:
+    """The library's ``deterministic`` argument: 0 fast, 2 (slots) where the tile index holds every
+    tile of each rectangle, 1 (sorted entries) where the ellipse cull drops some.  The gradients
+    of 1 and 2 are bitwise the same."""
+    return 0 if not deterministic else (1 if cull else 2)
+
+
 def tile_grid(H: int, W: int, tile_size: int) -> tuple[int, int]:
     if tile_size <= 0 or tile_size * tile_size > 1024:
         raise ValueError("tile_size must be positive with tile_size^2 <= 1024")
@@ -406,7 +413,8 @@ class _B200Render(Function):
                 rec, gids, offsets, status = saved[7:]
                 index = TileIndex(gids, offsets, ts, status)
             g_means, g_conics, g_colors, g_opac = _backward(
-                grad_out, rec, n, den, out, index, H, W, normalize, eps, tail, has_op, det, dev)
+                grad_out, rec, n, den, out, index, H, W, normalize, eps, tail, has_op,
+                deterministic_mode(det, cull), dev)
         return (g_means if need[0] else None, g_conics if need[1] else None,
                 g_colors if need[2] else None, None,
                 g_opac if (has_op and need[4]) else None) + (None,) * 9
