@@ -364,7 +364,7 @@ KERNELS_PER_CALL = {
     # kernels of this library launched by each entry point at 1,024 tiles (the index count's
     # second kernel scans the counts; the fill orders the bins)
     "ss_project_rs": 1, "ss_pack_splats": 1, "ss_tile_index_count": 2, "ss_tile_index_fill": 1,
-    "ss_project_rs_index_count": 2, "ss_batch_project_rs_index_count": 2,
+    "ss_pack_splats_index_count": 2, "ss_project_rs_index_count": 2, "ss_batch_project_rs_index_count": 2,
     "ss_render_forward": 1, "ss_render_backward": 2, "ss_project_rs_backward": 1,
     "ss_render_backward_moments": 1, "ss_render_backward_finalize_rs": 1,
     "ss_render_forward_backward": 1,

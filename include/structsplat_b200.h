@@ -123,6 +123,14 @@ int ss_project_rs_index_count(const float* means, const float* log_scales,
                               void* workspace, size_t workspace_bytes, void* clear,
                               size_t clear_bytes, uint32_t* status, ss_stream_t stream);
 
+/* ss_pack_splats followed by ss_tile_index_count in one kernel, with the same `clear` region. */
+int ss_pack_splats_index_count(const float* means, const float* conics, const float* colors,
+                               const int64_t* radii, const float* opacities, int64_t n,
+                               int height, int width, int tile_size, int ellipse_cull,
+                               float sigma_cutoff, void* records, int32_t* tile_offsets,
+                               void* workspace, size_t workspace_bytes, void* clear,
+                               size_t clear_bytes, uint32_t* status, ss_stream_t stream);
+
 /* The same over a batch (ss_batch_project_rs, then ss_batch_tile_index_count). */
 int ss_batch_project_rs_index_count(const ss_batch* batch, const float* means,
                                     const float* log_scales, const float* rotations,
@@ -424,9 +432,14 @@ int ss_render_backward_finalize_rs(const void* records, int64_t n, const int32_t
 /* ---------------------------------------------------------------- per-Gaussian passes
  * gaussian_activity (render.py:417-442): activity[g] = sum over the pixels of g's clipped
  * support rectangle of max(exp(-q/2) - fade_tail, 0) (opacity-free), from packed records.
- * lanes_per_gaussian: 8 (fields of small Gaussians) or 32.  Deterministic. */
+ * lanes_per_gaussian (8 or 32) is a hint of former versions without effect: each Gaussian gets the
+ * lanes its own rectangle needs.  Deterministic.  ss_splat_activity takes the render inputs
+ * (ss_pack_splats) instead of records. */
 int ss_gaussian_activity(const void* records, int64_t n, float fade_tail, int lanes_per_gaussian,
                          float* activity, ss_stream_t stream);
+int ss_splat_activity(const float* means, const float* conics, const int64_t* radii, int64_t n,
+                      int height, int width, float fade_tail, float* activity,
+                      ss_stream_t stream);
 
 /* ---------------------------------------------------------------- SSPL1 field decode
  * The integer streams of an SSPL1 container (codec.py:235-391), inflated on the host (zlib /

@@ -62,6 +62,9 @@ SIGNATURES = {
     "ss_project_rs_index_count": [_vp, _vp, _vp, _vp, _vp, _i64, _f32, _f32, _int, _int, _int,
                                   _int, _vp, _vp, _vp, ctypes.c_size_t, _vp, ctypes.c_size_t,
                                   _vp, _vp],
+    "ss_pack_splats_index_count": [_vp, _vp, _vp, _vp, _vp, _i64, _int, _int, _int, _int, _f32,
+                                   _vp, _vp, _vp, ctypes.c_size_t, _vp, ctypes.c_size_t, _vp,
+                                   _vp],
     "ss_build_tile_index_static": [_vp, _vp, _vp, _i64, _int, _int, _int, _int, _f32, _vp, _i64,
                                    _vp, _vp, _vp],
     "ss_render_forward": [_vp, _i64, _vp, _i64, _vp, _int, _int, _int, _int, _f32, _f32, _vp, _vp,
@@ -80,6 +83,7 @@ SIGNATURES = {
                                    _int, _int, _f32, _f32, _int, _vp, ctypes.c_size_t, _vp, _vp],
     "ss_render_backward_finalize_rs": [_vp, _i64, _vp, _i64, _vp, _int, _int, _int, _int, _vp,
                                        _vp, _vp, _vp, _f32, _vp, _vp, _vp, _vp, _vp, _vp],
+    "ss_splat_activity": [_vp, _vp, _vp, _i64, _int, _int, _f32, _vp, _vp],
     "ss_gaussian_activity": [_vp, _i64, _f32, _int, _vp, _vp],
     "ss_render_backward_finalize": [_vp, _i64, _vp, _i64, _vp, _int, _int, _int, _int, _int, _vp,
                                     _vp, _vp, _vp, _vp, _vp],

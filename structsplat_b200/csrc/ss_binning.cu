@@ -398,6 +398,34 @@ __global__ void project_count_kernel(RSField field, int64_t n, int ts, Frames fr
                           tile_count, bins, K);
 }
 
+// The render inputs (ss_pack_splats).
+struct PackField {
+  const float *means, *conics, *colors;
+  const int64_t* radii;
+  const float* opacities;
+};
+
+// Packing and the per-tile counts in one pass, as project_count_kernel.
+template <bool CULL, bool BINS>
+__global__ void pack_count_kernel(PackField f, int64_t n, int ts, Frames frames, float cutoff2,
+                                  Splat* __restrict__ out, int* __restrict__ tile_count,
+                                  uint4* __restrict__ clear, int64_t clear_vec,
+                                  int32_t* __restrict__ bins, int K) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (BINS && i == 0) tile_count[2] = K;
+  for (int64_t v = i; v < clear_vec; v += (int64_t)gridDim.x * blockDim.x)
+    clear[v] = make_uint4(0u, 0u, 0u, 0u);
+  Splat s{};
+  if (i < n) {
+    s = pack_one(f.means, f.conics, f.colors, f.radii, f.opacities, i, frames.H, frames.W);
+    store_splat(out + i, s);
+  }
+  count_pairs<CULL, BINS>(s, i < n, blockIdx.x * kThreads, ts, frames.tiles_x, 0, cutoff2,
+                          tile_count, bins, K);
+}
+
 // Writes int32 offsets, checks capacity, then claims one slot per pair.  Slots are claimed by
 // counting each tile's counter back down, which leaves the counters at zero.  A lane's own
 // (small) rectangle claims all its slots first and stores afterwards, so the atomics overlap.
@@ -980,11 +1008,12 @@ int check_index_args(int64_t n, int H, int W, int ts) {
 
 // Stage 1 over any tile set (one image or a batch): counts, scan, int32 offsets.
 // With `rs`, the records are first projected from that RS field in the same kernel
-// (project_count_kernel) and written to `records`.
+// (project_count_kernel) and written to `records`; with `pk` (one image) packed from those inputs.
 int index_count(const Frames& frames, int ts, int64_t T, const void* records, int64_t n,
                 int ellipse_cull, float sigma_cutoff, int32_t* tile_offsets, void* workspace,
                 size_t workspace_bytes, uint32_t* status, ss_stream_t stream,
-                const RSField* rs = nullptr, void* clear = nullptr, size_t clear_bytes = 0) {
+                const RSField* rs = nullptr, void* clear = nullptr, size_t clear_bytes = 0,
+                const PackField* pk = nullptr) {
   int rc;
   if (!tile_offsets || !workspace) return fail(SS_ERR_INVALID_ARGUMENT, "null pointer");
   if (n > 0 && !records) return fail(SS_ERR_INVALID_ARGUMENT, "null records");
@@ -1003,9 +1032,25 @@ int index_count(const Frames& frames, int ts, int64_t T, const void* records, in
   if (clear_bytes && (!clear || reinterpret_cast<uintptr_t>(clear) % 16 || clear_bytes % 16))
     return fail(SS_ERR_INVALID_ARGUMENT,
                 "clear region must be 16-byte aligned and a multiple of 16 bytes");
-  if (clear_bytes && !(rs && n > 0) && cudaMemsetAsync(clear, 0, clear_bytes, s) != cudaSuccess)
+  if (clear_bytes && !((rs || pk) && n > 0) && cudaMemsetAsync(clear, 0, clear_bytes, s) != cudaSuccess)
     return check_launch("clear region memset");
-  if (rs && n > 0) {  // project even when the tile set is empty: the records are an output
+  if (pk && n > 0) {  // pack even when the tile set is empty: the records are an output
+    if (reinterpret_cast<uintptr_t>(records) % 16)
+      return fail(SS_ERR_INVALID_ARGUMENT, "records must be 16-byte aligned");
+    int blocks = (int)((n + kThreads - 1) / kThreads);
+    Splat* out = static_cast<Splat*>(const_cast<void*>(records));
+#define SS_KCOUNT(C, B)                                                                       \
+  launch("pack_count_kernel", pack_count_kernel<C, B>, blocks, kThreads, 0, s, *pk, n, ts,      \
+         frames, cutoff2, out, w.tile_count, static_cast<uint4*>(clear),                      \
+         (int64_t)(clear_bytes / 16), w.bins, w.bin_ids)
+    if (ellipse_cull) {
+      if (binned) SS_KCOUNT(true, true); else SS_KCOUNT(true, false);
+    } else {
+      if (binned) SS_KCOUNT(false, true); else SS_KCOUNT(false, false);
+    }
+#undef SS_KCOUNT
+    if ((rc = check_launch("pack_count"))) return rc;
+  } else if (rs && n > 0) {  // project even when the tile set is empty
     if (reinterpret_cast<uintptr_t>(records) % 16)
       return fail(SS_ERR_INVALID_ARGUMENT, "records must be 16-byte aligned");
     int blocks = (int)((n + kThreads - 1) / kThreads);
@@ -1187,6 +1232,23 @@ int ss_project_rs_index_count(const float* means, const float* log_scales,
                      make_grid(height, width, tile_size).T, records, n, ellipse_cull,
                      sigma_cutoff, tile_offsets, workspace, workspace_bytes, status, stream, &f,
                      clear, clear_bytes);
+}
+
+int ss_pack_splats_index_count(const float* means, const float* conics, const float* colors,
+                               const int64_t* radii, const float* opacities, int64_t n,
+                               int height, int width, int tile_size, int ellipse_cull,
+                               float sigma_cutoff, void* records, int32_t* tile_offsets,
+                               void* workspace, size_t workspace_bytes, void* clear,
+                               size_t clear_bytes, uint32_t* status, ss_stream_t stream) {
+  int rc = check_index_args(n, height, width, tile_size);
+  if (rc) return rc;
+  if (n > 0 && (!means || !conics || !colors || !radii))
+    return fail(SS_ERR_INVALID_ARGUMENT, "null pointer");
+  const PackField f{means, conics, colors, radii, opacities};
+  return index_count(single_frame(height, width, tile_size), tile_size,
+                     make_grid(height, width, tile_size).T, records, n, ellipse_cull,
+                     sigma_cutoff, tile_offsets, workspace, workspace_bytes, status, stream,
+                     nullptr, clear, clear_bytes, &f);
 }
 
 int ss_batch_project_rs_index_count(const ss_batch* batch, const float* means,

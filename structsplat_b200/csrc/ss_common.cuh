@@ -164,6 +164,24 @@ __device__ __forceinline__ Splat make_splat(float mx, float my, float a, float b
   return s;
 }
 
+// Record of Gaussian i of the render inputs (ss_pack_splats); every load is issued before the first
+// is used.
+__device__ __forceinline__ Splat pack_one(const float* means, const float* conics,
+                                          const float* colors, const int64_t* radii,
+                                          const float* opacities, int64_t i, int H, int W) {
+  const float mx = __ldg(means + 2 * i), my = __ldg(means + 2 * i + 1);
+  const long long rx = __ldg(reinterpret_cast<const long long*>(radii) + 2 * i);
+  const long long ry = __ldg(reinterpret_cast<const long long*>(radii) + 2 * i + 1);
+  const float a = __ldg(conics + 3 * i), b = __ldg(conics + 3 * i + 1);
+  const float c = __ldg(conics + 3 * i + 2);
+  const float cr = __ldg(colors + 3 * i), cg = __ldg(colors + 3 * i + 1);
+  const float cb = __ldg(colors + 3 * i + 2);
+  const float op = opacities ? __ldg(opacities + i) : 1.0f;
+  int x0, y0, x1, y1;
+  support_rect(mx, my, rx, ry, H, W, x0, y0, x1, y1);
+  return make_splat(mx, my, a, b, c, op, cr, cg, cb, x0, y0, x1, y1);
+}
+
 __device__ __forceinline__ void store_splat(Splat* dst, const Splat& s) {
   const float4* src = reinterpret_cast<const float4*>(&s);
   float4* d = reinterpret_cast<float4*>(dst);

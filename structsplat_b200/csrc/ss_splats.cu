@@ -93,13 +93,7 @@ __global__ void pack_splats_kernel(const float* __restrict__ means,
   pdl_trigger();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float mx = means[2 * i], my = means[2 * i + 1];
-  int x0, y0, x1, y1;
-  support_rect(mx, my, radii[2 * i], radii[2 * i + 1], H, W, x0, y0, x1, y1);
-  float op = opacities ? opacities[i] : 1.0f;
-  store_splat(out + i, make_splat(mx, my, conics[3 * i], conics[3 * i + 1], conics[3 * i + 2],
-                                  op, colors[3 * i], colors[3 * i + 1], colors[3 * i + 2], x0,
-                                  y0, x1, y1));
+  store_splat(out + i, pack_one(means, conics, colors, radii, opacities, i, H, W));
 }
 
 // RS -> splat record (rs_project_one), plus the conic and radii where asked for.

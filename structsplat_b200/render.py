@@ -258,21 +258,23 @@ class _EagerPlans:
 EAGER_PLANS = _EagerPlans()
 
 
-def index_from_records(records, n: int, H: int, W: int, tile_size: int = 16,
-                       ellipse_cull: bool = False, sigma_cutoff: float = 3.0,
-                       capacity: int | None = None, exact: bool = False) -> TileIndex:
-    """Count → scan → fill → sort.  ``exact`` reads the entry total back (one device→host sync)
-    and sizes the list exactly; otherwise the capacity comes from ``capacity`` or the
-    per-problem cache."""
+def _index(n: int, H: int, W: int, tile_size: int, ellipse_cull: bool, sigma_cutoff: float,
+           capacity, exact: bool, dev, records, pack=None) -> TileIndex:
     tiles_x, tiles_y = tile_grid(H, W, tile_size)
     T = tiles_x * tiles_y
-    dev = records.device
     offsets = torch.empty(T + 1, device=dev, dtype=torch.int32)
-    status = torch.zeros(1, device=dev, dtype=torch.int32)
     ws_bytes = _native.size_query("ss_tile_index_binned_workspace_bytes", n, H, W, tile_size)
     ws = torch.empty(max(ws_bytes, 1), device=dev, dtype=torch.uint8)
-    _native.call("ss_tile_index_count", _p(records), n, H, W, tile_size, int(ellipse_cull),
-                 float(sigma_cutoff), _p(offsets), _p(ws), ws_bytes, _p(status), _stream())
+    if pack is None:
+        status = torch.zeros(1, device=dev, dtype=torch.int32)
+        _native.call("ss_tile_index_count", _p(records), n, H, W, tile_size, int(ellipse_cull),
+                     float(sigma_cutoff), _p(offsets), _p(ws), ws_bytes, _p(status), _stream())
+    else:
+        word = torch.empty(4, device=dev, dtype=torch.int32)  # cleared by the call, 16 bytes
+        status = word[:1]
+        _native.call("ss_pack_splats_index_count", *(_p(t) for t in pack), n, H, W, tile_size,
+                     int(ellipse_cull), float(sigma_cutoff), _p(records), _p(offsets), _p(ws),
+                     ws_bytes, _p(word), 16, _p(status), _stream())
     if T == 0:
         capacity = 0
     elif exact:
@@ -287,6 +289,26 @@ def index_from_records(records, n: int, H: int, W: int, tile_size: int = 16,
     return TileIndex(gids[:capacity], offsets, tile_size, status)
 
 
+def index_from_records(records, n: int, H: int, W: int, tile_size: int = 16,
+                       ellipse_cull: bool = False, sigma_cutoff: float = 3.0,
+                       capacity: int | None = None, exact: bool = False) -> TileIndex:
+    """Count → scan → fill → sort.  ``exact`` reads the entry total back (one device→host sync)
+    and sizes the list exactly; otherwise the capacity comes from ``capacity`` or the
+    per-problem cache."""
+    return _index(n, H, W, tile_size, ellipse_cull, sigma_cutoff, capacity, exact,
+                  records.device, records)
+
+
+def pack_and_index(means, conics, colors, radii, opacities, H: int, W: int, tile_size: int,
+                   ellipse_cull: bool, sigma_cutoff: float, exact: bool = False):
+    """pack_records and index_from_records with the packing and the count in one kernel."""
+    n = means.shape[0]
+    rec = torch.empty(max(n, 1) * RECORD_FLOATS, device=means.device, dtype=torch.float32)
+    index = _index(n, H, W, tile_size, ellipse_cull, sigma_cutoff, None, exact, means.device, rec,
+                   (means, conics, colors, radii, opacities))
+    return rec, index
+
+
 def build_tile_index(means, conics, radii, H: int, W: int, tile_size: int = 16,
                      ellipse_cull: bool = False, sigma_cutoff: float = 3.0):
     """``(gids int32 [entries], offsets int32 [T+1])`` like the extension's build_tile_index."""
@@ -296,9 +318,8 @@ def build_tile_index(means, conics, radii, H: int, W: int, tile_size: int = 16,
     means = means.detach().contiguous()
     conics = conics.detach().contiguous().to(torch.float32)
     radii = radii.contiguous()
-    rec = pack_records(means.to(torch.float32), conics, conics, radii, None, H, W)
-    idx = index_from_records(rec, means.shape[0], H, W, tile_size, ellipse_cull, sigma_cutoff,
-                             exact=True)
+    _, idx = pack_and_index(means.to(torch.float32), conics, conics, radii, None, H, W, tile_size,
+                            ellipse_cull, sigma_cutoff, exact=True)
     return idx.gids, idx.offsets
 
 
@@ -345,13 +366,12 @@ class _B200Render(Function):
         if not deterministic and n and H * W:
             # the fast path: the problem's buffers persist between calls (EagerPlan)
             plan = EAGER_PLANS.get(n, H, W, tile_size, cull, sigma_cutoff, means.device)
-            plan.step_block.zero_()  # fast moments and the status word
             stream = _stream()
-            _native.call("ss_pack_splats", _p(means), _p(conics), _p(colors), _p(radii), _p(op),
-                         n, H, W, _p(plan.records), stream)
-            _native.call("ss_tile_index_count", _p(plan.records), n, H, W, tile_size, int(cull),
-                         float(sigma_cutoff), _p(plan.offsets), _p(plan.idx_ws),
-                         plan.idx_ws_bytes, _p(plan.status), stream)
+            # clears the fast moments and the status word too
+            _native.call("ss_pack_splats_index_count", _p(means), _p(conics), _p(colors),
+                         _p(radii), _p(op), n, H, W, tile_size, int(cull), float(sigma_cutoff),
+                         _p(plan.records), _p(plan.offsets), _p(plan.idx_ws), plan.idx_ws_bytes,
+                         _p(plan.step_block), plan.step_block.numel(), _p(plan.status), stream)
             plan.ensure_capacity()
             _native.call("ss_tile_index_fill", _p(plan.records), n, H, W, tile_size, int(cull),
                          float(sigma_cutoff), _p(plan.offsets), _p(plan.gids), plan.capacity,
@@ -367,9 +387,8 @@ class _B200Render(Function):
             ctx.plan, ctx.generation = plan, plan.generation
             ctx.save_for_backward(out, den, means, conics, colors, radii, op)
             return out
-        rec = pack_records(means, conics, colors, radii, op, H, W)
-        index = index_from_records(rec, n, H, W, tile_size, cull, sigma_cutoff,
-                                   exact=bool(deterministic))
+        rec, index = pack_and_index(means, conics, colors, radii, op, H, W, tile_size, cull,
+                                    sigma_cutoff, exact=bool(deterministic))
         out, den = _forward(rec, n, index, H, W, normalize, eps, tail, means.device)
         ctx.plan = None
         ctx.save_for_backward(out, den, means, conics, colors, radii, op, rec, index.gids,
@@ -407,8 +426,8 @@ class _B200Render(Function):
                          stream)
         else:
             if plan is not None:  # the plan moved on to a later forward: rebuild this one's
-                rec = pack_records(means, conics, colors, radii, op, H, W)
-                index = index_from_records(rec, n, H, W, ts, cull, cutoff, exact=True)
+                rec, index = pack_and_index(means, conics, colors, radii, op, H, W, ts, cull,
+                                            cutoff, exact=True)
             else:
                 rec, gids, offsets, status = saved[7:]
                 index = TileIndex(gids, offsets, ts, status)
@@ -504,13 +523,11 @@ def gaussian_activity(means, conics, radii, H: int, W: int, chunk: int = 4096,
     tail = fade_tail(sigma_cutoff, alpha)
     means = means.detach().contiguous().to(torch.float32)
     conics = conics.detach().contiguous().to(torch.float32)
-    rec = pack_records(means, conics, conics, radii.contiguous(), None, H, W)
+    radii = radii.contiguous()
     act = torch.empty(n, device=means.device, dtype=torch.float32)
     if n:
-        r = radii.detach()
-        mean_side = float((2 * r + 1).to(torch.float32).mean()) if n else 0.0
-        lanes = 8 if mean_side * mean_side <= 96 else 32
-        _native.call("ss_gaussian_activity", _p(rec), n, float(tail), lanes, _p(act), _stream())
+        _native.call("ss_splat_activity", _p(means), _p(conics), _p(radii), n, H, W, float(tail),
+                     _p(act), _stream())
     return act
 
 
@@ -532,10 +549,10 @@ def render_cuda_exact_with_coverage(means, conics, colors, radii, H: int, W: int
     n = means.shape[0]
     alpha = resolve_fade_alpha(support_fade, None)
     tail = fade_tail(sigma_cutoff, alpha)
-    rec = pack_records(means.contiguous(), conics.contiguous(), colors.contiguous(),
-                       radii.contiguous(), None if opacities is None else opacities.contiguous(),
-                       H, W)
-    index = index_from_records(rec, n, H, W, tile_size, alpha >= 1.0, sigma_cutoff)
+    rec, index = pack_and_index(means.contiguous(), conics.contiguous(), colors.contiguous(),
+                                radii.contiguous(),
+                                None if opacities is None else opacities.contiguous(), H, W,
+                                tile_size, alpha >= 1.0, sigma_cutoff)
     return _forward(rec, n, index, H, W, True, eps, tail, means.device)
 
 
@@ -548,9 +565,9 @@ class _RawWeightMap(Function):
         n = means.shape[0]
         means, conics = means.contiguous(), conics.contiguous()
         has_op = opacities is not None
-        rec = pack_records(means, conics, conics, radii.contiguous(),
-                           opacities.contiguous() if has_op else None, H, W)
-        index = index_from_records(rec, n, H, W, tile_size, cull, sigma_cutoff)
+        rec, index = pack_and_index(means, conics, conics, radii.contiguous(),
+                                    opacities.contiguous() if has_op else None, H, W, tile_size,
+                                    cull, sigma_cutoff)
         _, den = _forward(rec, n, index, H, W, False, 1.0, tail, means.device)
         ctx.save_for_backward(rec, index.gids, index.offsets, index.status)
         ctx.meta = (n, H, W, tile_size, tail, has_op)
