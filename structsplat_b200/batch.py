@@ -189,14 +189,17 @@ class FitPlan:
                                                self.capacity, int(s.deterministic))
         self.bwd_ws = torch.zeros(max(self.bwd_ws_bytes // 4, 4), **f32)
         self.pixel_grad = torch.empty(max(batch.pixels, 1), 4, **f32)
-        self.loss = torch.zeros(batch.images, 2, **f32)
+        # loss and SSIM of every image in one block, which the projection kernel clears each step
+        B = batch.images
+        self._sums = torch.zeros((3 * B + 3) // 4 * 4, **f32)
+        self.loss = self._sums[:2 * B].view(B, 2)
         if not 0.0 <= s.ssim_weight <= 1.0:
             raise ValueError(f"ssim_weight must lie in [0, 1], got {s.ssim_weight}")
         if s.ssim_weight > 0.0:  # the SSIM term needs the whole image before the backward
             P = max(batch.pixels, 1)
             self.image = torch.empty(P, 3, **f32)
             self.den = torch.empty(P, **f32)
-            self.ssim = torch.zeros(batch.images, **f32)
+            self.ssim = self._sums[2 * B:3 * B]
             self.ssim_stats = torch.empty(6 * P, **f32)
             self.ssim_ws_bytes = _native.size_query("ss_ssim_workspace_bytes", batch.pixels)
             self.ssim_ws = torch.empty(max(self.ssim_ws_bytes // 4, 1), **f32)
@@ -239,15 +242,17 @@ class FitPlan:
                      int(self.cull), float(self.s.sigma_cutoff), _p(self.offsets), _p(self.idx_ws),
                      self.idx_ws_bytes, _p(self.status), _stream())
 
-    def project_count(self):
-        """project() and count() in one kernel (ss_batch_project_rs_index_count)."""
+    def project_count(self, clear_sums: bool = False):
+        """project() and count() in one kernel (ss_batch_project_rs_index_count), which also zeroes
+        the losses and SSIM values with ``clear_sums``."""
         p = self.params
+        clear = self._sums if clear_sums else None
         _native.call("ss_batch_project_rs_index_count", self.batch.ref, _p(p["means"]),
                      _p(p["log_scales"]), _p(p["rotations"]), _p(p["colors"]),
                      _p(p.get("opacity_logits")), self.n, float(self.s.dilation),
                      float(self.s.sigma_cutoff), int(self.cull), _p(self.records),
-                     _p(self.offsets), _p(self.idx_ws), self.idx_ws_bytes, None, 0,
-                     _p(self.status), _stream())
+                     _p(self.offsets), _p(self.idx_ws), self.idx_ws_bytes, _p(clear),
+                     4 * clear.numel() if clear_sums else 0, _p(self.status), _stream())
 
     def fill(self):
         _native.call("ss_batch_tile_index_fill", self.batch.ref, _p(self.records), self.n,
@@ -303,11 +308,9 @@ class FitPlan:
 
     def step(self):
         """One fit iteration for every image of the batch."""
-        self.loss.zero_()
-        self.project_count()
+        self.project_count(clear_sums=True)
         self.fill()
         if self.s.ssim_weight > 0.0:
-            self.ssim.zero_()
             self.forward_loss(image=self.image, den=self.den)
             self.ssim_term()
             self.backward(self.det)

@@ -47,11 +47,12 @@ __device__ __forceinline__ void pdl_trigger() {
 bool dependent_launch_enabled();
 void note_launch_error(cudaError_t e);
 
-// Launches `kern` on `s` with the programmatic-serialization attribute when enabled; returns
-// SS_OK or the launch error, which the next check_launch of the thread also reports.
+// Launches `kern` on `s`, with the programmatic-serialization attribute when `dependent` and
+// enabled; returns SS_OK or the launch error, which the next check_launch of the thread also
+// reports.
 template <typename... KArgs, typename... Args>
-int launch(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-           cudaStream_t s, Args... args) {
+int launch_as(bool dependent, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block,
+              size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -61,7 +62,7 @@ int launch(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = dependent_launch_enabled() ? 1 : 0;
+  cfg.numAttrs = dependent && dependent_launch_enabled() ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
   if (e != cudaSuccess) {
     note_launch_error(e);  // the caller's next check_launch reports it too
@@ -70,19 +71,37 @@ int launch(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size
   return SS_OK;
 }
 
+template <typename... KArgs, typename... Args>
+int launch(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+           cudaStream_t s, Args... args) {
+  return launch_as(true, what, kern, grid, block, smem, s, args...);
+}
+
+// Tile kernels of more CTAs than this are launched plainly.  Starting early saves a launch's latency,
+// a microsecond or two, but it hands out SMs as the kernel before drains: the CTAs crowd on the SMs
+// that come free first, and the kernel ends on those.  Measured with and without the attribute:
+// forward of 2,752 tiles in an SSIM fit 545 -> 519 us for the step, backward of 1,024 long lists
+// 12 us, fused pass of 2,040 tiles 12 us; nothing either way at 1,024 short lists.
+constexpr unsigned kDependentTiles = 592;  // two rounds of two CTAs per SM
+
 // Lets `kern` take `bytes` of dynamic shared memory (beyond the 48 KB default; the largest
 // size a kernel is launched with, set once per kernel and device).
 int allow_dynamic_smem(const void* kern, size_t bytes);
 
-// launch() of a kernel whose shared memory is dynamic: `smem` bytes, opted in first.
+// launch_as() and launch() of a kernel whose shared memory is dynamic: `smem` bytes, opted in first.
 template <typename... KArgs, typename... Args>
-int launch_smem(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                cudaStream_t s, Args... args) {
+int launch_smem_as(bool dependent, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block,
+                   size_t smem, cudaStream_t s, Args... args) {
   if (smem > 48 * 1024) {
     const int rc = allow_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
     if (rc) return rc;
   }
-  return launch(what, kern, grid, block, smem, s, args...);
+  return launch_as(dependent, what, kern, grid, block, smem, s, args...);
+}
+template <typename... KArgs, typename... Args>
+int launch_smem(const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                cudaStream_t s, Args... args) {
+  return launch_smem_as(true, what, kern, grid, block, smem, s, args...);
 }
 
 // 2^x on the SFU (PTX ex2.approx.ftz.f32: one MUFU operation, documented max relative error
@@ -497,8 +516,28 @@ __device__ __forceinline__ void sum_entry_partials(const float* __restrict__ par
     beg = seg[g];
     end = seg[n + g];
   }
-  if (end - beg <= kLaneSegment)
-    for (int i = beg; i < end; ++i) add_partial(partials, order ? order[i] : i, acc);
+  if (end - beg <= kLaneSegment) {
+    // four entries' loads in flight, added in order
+    for (int i = beg; i < end; i += 4) {
+      float4 u[4], v[4];
+      float w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (i + k >= end) break;
+        const float* p = partials + (int64_t)(order ? order[i + k] : i + k) * kPartialFloats;
+        u[k] = reinterpret_cast<const float4*>(p)[0];
+        v[k] = reinterpret_cast<const float4*>(p)[1];
+        w[k] = p[8];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (i + k >= end) break;
+        acc[0] += u[k].x; acc[1] += u[k].y; acc[2] += u[k].z; acc[3] += u[k].w;
+        acc[4] += v[k].x; acc[5] += v[k].y; acc[6] += v[k].z; acc[7] += v[k].w;
+        acc[8] += w[k];
+      }
+    }
+  }
   const int lane = threadIdx.x & 31;
   unsigned big = __ballot_sync(0xffffffffu, end - beg > kLaneSegment);
   while (big) {

@@ -1471,7 +1471,7 @@ void launch_forward_loss(int loss_kind, unsigned T, cudaStream_t s, const Splat*
   const int c = g_forward_chunk[TS == 16 ? 0 : 1].load(std::memory_order_relaxed);
   const int chunk = c ? c : kStageAll / 2;
 #define SS_FWD(LOSS)                                                                          \
-  launch_smem("forward_kernel", forward_kernel<TS, NORM, FADE, LOSS>, T, NT,                  \
+  launch_smem_as(T <= kDependentTiles, "forward_kernel", forward_kernel<TS, NORM, FADE, LOSS>, T, NT,                  \
               FwdSmem<TS>::kBytes, s, rec, n, gids, cap, offsets, f, eps, tail, out, den,      \
               target, pixel_grad, loss, ce2, chunk)
   switch (loss_kind) {
@@ -1512,7 +1512,7 @@ void launch_backward_nt(unsigned T, cudaStream_t s, int deterministic, const flo
   const bool fade = tail > 0.0f;
   const int32_t* slots = slot_base_of(ws, n, cap, deterministic);
 #define SS_BWD(FADE, DET)                                                                     \
-  launch_smem("backward_kernel", backward_kernel<TS, NT, FADE, DET, PIXGRAD>, T, NT,         \
+  launch_smem_as(T <= kDependentTiles, "backward_kernel", backward_kernel<TS, NT, FADE, DET, PIXGRAD>, T, NT,         \
               (BwdSmem<TS, NT, false>::kBytes), s, grad_out, rec, n, den, out, pixel_grad,   \
               gids, cap, offsets, f, normalize, eps, tail, ws, ws, slots, status, FusedFit{})
   if (deterministic) {
@@ -1550,7 +1550,7 @@ void launch_fused_nt(unsigned T, cudaStream_t s, int deterministic, const Splat*
   const bool fade = tail > 0.0f;
   const int32_t* slots = slot_base_of(ws, n, cap, deterministic);
 #define SS_FUS(FADE, DET)                                                                       \
-  launch_smem("fit_tile_kernel", backward_kernel<TS, NT, FADE, DET, false, true>, T, NT,     \
+  launch_smem_as(T <= kDependentTiles, "fit_tile_kernel", backward_kernel<TS, NT, FADE, DET, false, true>, T, NT,     \
               (BwdSmem<TS, NT, true>::kBytes), s, nullptr, rec, n, nullptr, nullptr, nullptr, \
               gids, cap, offsets, f, normalize, eps, tail, ws, ws, slots, status, ff)
   if (deterministic) {
