@@ -1503,6 +1503,16 @@ void launch_forward(int loss_kind, unsigned T, cudaStream_t s, const Splat* rec,
 // Warps per backward CTA: a process-wide tuning knob (0 = the default of the tile size).
 std::atomic<int> g_backward_warps[2] = {{0}, {0}};
 
+// Warps of a tile set's backward CTAs: as asked, else eight, or sixteen for a 32-px tile set of up to
+// kWideTiles, which leaves SMs idle or with one or two CTAs each: a tile's time is then the kernel's
+// (fit step of 64 tiles 45.0 -> 41.9 us).  Results do not depend on it.
+constexpr unsigned kWideTiles = 296;
+int backward_warps(int ts, unsigned T) {
+  const int asked = g_backward_warps[ts == 16 ? 0 : 1].load(std::memory_order_relaxed);
+  if (asked) return asked;
+  return ts == 32 && T <= kWideTiles ? 16 : 8;
+}
+
 template <int TS, int NT, bool PIXGRAD>
 void launch_backward_nt(unsigned T, cudaStream_t s, int deterministic, const float* grad_out,
                         const Splat* rec, int64_t n, const float* den, const float* out,
@@ -1529,9 +1539,9 @@ void launch_backward(unsigned T, cudaStream_t s, int deterministic, const float*
                      const float4* pixel_grad, const int32_t* gids, int64_t cap,
                      const int32_t* offsets, const Frames& f, int normalize, float eps,
                      float tail, float* ws, uint32_t* status) {
-  const int warps = g_backward_warps[TS == 16 ? 0 : 1].load(std::memory_order_relaxed);
+  const int warps = backward_warps(TS, T);
   constexpr int kSmall = TS == 16 ? 128 : 256, kLarge = TS == 16 ? 256 : 512;
-  if (warps * 32 == kSmall || (TS == 32 && warps == 0))  // tile 32: 8 warps unless asked
+  if (warps * 32 == kSmall)
     launch_backward_nt<TS, kSmall, PIXGRAD>(T, s, deterministic, grad_out, rec, n, den, out,
                                             pixel_grad, gids, cap, offsets, f, normalize, eps,
                                             tail, ws, status);
@@ -1566,9 +1576,9 @@ void launch_fused(unsigned T, cudaStream_t s, int deterministic, const Splat* re
                   const int32_t* gids, int64_t cap, const int32_t* offsets, const Frames& f,
                   int normalize, float eps, float tail, float* ws, uint32_t* status,
                   const FusedFit& ff) {
-  const int warps = g_backward_warps[TS == 16 ? 0 : 1].load(std::memory_order_relaxed);
+  const int warps = backward_warps(TS, T);
   constexpr int kSmall = TS == 16 ? 128 : 256, kLarge = TS == 16 ? 256 : 512;
-  if (warps * 32 == kSmall || (TS == 32 && warps == 0))
+  if (warps * 32 == kSmall)
     launch_fused_nt<TS, kSmall>(T, s, deterministic, rec, n, gids, cap, offsets, f, normalize,
                                 eps, tail, ws, status, ff);
   else
