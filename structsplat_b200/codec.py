@@ -12,8 +12,11 @@ from __future__ import annotations
 
 import ctypes
 import json
+import os
 import struct
+import threading
 import zlib
+from concurrent.futures import ThreadPoolExecutor
 from io import BytesIO
 
 import numpy as np
@@ -23,6 +26,9 @@ from . import _native
 from .render import ADDITIVE_MODES, DEFAULT_EPS, NORMALIZED_MODES, _p, _stream
 
 MAGIC = b"SSPL1"
+# Compressed bytes from which inflating in threads pays for the hand-over (~0.05 ms; a core inflates
+# 0.1 to 2 compressed bytes per ns).
+THREADED_BYTES = 1 << 17
 SCALE_LO = float(np.log(0.35))  # the fitter's log-scale floor, for headers without scale_lo
 
 
@@ -48,6 +54,35 @@ def _inflate(payload: bytes, codec: str, raw_len):
     raise ValueError(f"unknown stream_codec {codec!r}; expected 'zlib' or 'png'")
 
 
+_POOL: tuple | None = None  # (process id, executor)
+_POOL_LOCK = threading.Lock()
+
+
+def _pool() -> ThreadPoolExecutor:
+    """At most four threads, started on first use and kept by this process (a forked child, which
+    inherits none of them, starts its own); joined at exit."""
+    global _POOL
+    with _POOL_LOCK:
+        if _POOL is None or _POOL[0] != os.getpid():
+            _POOL = (os.getpid(), ThreadPoolExecutor(4, thread_name_prefix="sspl1-inflate"))
+        return _POOL[1]
+
+
+def _inflate_all(streams, codec: str):
+    """The inflated streams, in order.  zlib works outside the interpreter lock, so the streams of
+    all but small containers inflate side by side, the first on the calling thread (50k Gaussians:
+    0.6 + 0.8 ms for the means and scales, which compress, 0.15 ms for the rest).  The first
+    damaged stream's error is raised either way."""
+    if codec == "zlib" and len(streams) > 1 and sum(len(z) for z, _, _ in streams) >= THREADED_BYTES:
+        try:
+            rest = [_pool().submit(_inflate, *args) for args in streams[1:]]
+        except RuntimeError:  # the interpreter is shutting down: no more threads
+            rest = None
+        if rest is not None:
+            return [_inflate(*streams[0])] + [f.result() for f in rest]
+    return [_inflate(*args) for args in streams]
+
+
 def _streams(blob: bytes):
     """(header, inflated stream bytes in container order)."""
     h = blob_header(blob)
@@ -56,15 +91,19 @@ def _streams(blob: bytes):
     count = (5 if h.get("has_opacity", False) else 4) + (1 if h.get("has_alpha", False) else 0)
     raw_lengths = h.get("stream_raw_lengths", [])
     codec = h.get("stream_codec", "zlib")
-    raws = []
+    streams, cut = [], False
     for i in range(count):
         if off + 4 > len(blob):
-            raise ValueError("truncated structsplat codec stream framing")
+            cut = True
+            break
         (zlen,) = struct.unpack_from("<I", blob, off)
         off += 4
         raw_len = int(raw_lengths[i]) if i < len(raw_lengths) else None
-        raws.append(_inflate(blob[off:off + zlen], codec, raw_len))
+        streams.append((blob[off:off + zlen], codec, raw_len))
         off += zlen
+    raws = _inflate_all(streams, codec)
+    if cut:
+        raise ValueError("truncated structsplat codec stream framing")
     return h, raws
 
 
