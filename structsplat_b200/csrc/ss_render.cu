@@ -42,12 +42,6 @@ namespace {
 
 constexpr int kEpilogueThreads = 256;
 
-template <int TS>
-struct Tiling {
-  // backward whole-list stage: what fits in 48 KB of static shared memory beside the pixels
-  static constexpr int kBwdStageAll = TS == 16 ? 512 : 448;
-};
-
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
@@ -131,9 +125,12 @@ __device__ __forceinline__ uint16_t block_mask(const int4& b, int tx0, int ty0) 
   return (uint16_t)(spread * cols);
 }
 
-// Lists up to kStageAll Gaussians are staged whole (one barrier per tile; the warps then run
-// independently); longer lists stream through the two halves of the stage, double-buffered.
-constexpr int kStageAll = 512;
+// Lists up to a kernel's stage are staged whole (the warps then run independently); longer lists
+// stream through its two halves, double-buffered, the forward's at most this many records at a time.
+constexpr int kForwardChunk = 256;
+// Gaussians per 32-px tile beyond which a tile set counts as one of long lists (lists are 2 to 8 times
+// as long): the kernels then trade CTAs or cache for larger stages.
+constexpr int64_t kLongLists = 160;
 
 // Issues the copies of entries [k0, k0+m) into `dst` with NT threads: 16-byte piece (q & 3) of
 // entry (q >> 2) for q = threadIdx.x, threadIdx.x + NT, …  With `rect_dst` the rectangles
@@ -548,13 +545,12 @@ __device__ __forceinline__ void add_tile_loss(float loss_sum, float sq_sum, floa
   }
 }
 
-// Shared memory of the forward kernel (dynamic): the stage (whole lists up to kStageAll
+// Shared memory of the forward kernel (dynamic): the stage (whole lists up to kStage
 // records, or two halves of it for a streamed list) followed by every warp's carry slots and
 // the null record; the staged records' rectangles, packed, and block masks; and every warp's hit
-// list, which
-// after the block's last evaluation holds the block's 8x8 pixels (RGB rows, then den) on their
-// way out as whole float4 image rows.  One warp per 8x8 block.
-template <int TS>
+// list, which after the block's last evaluation holds the block's 8x8 pixels (RGB rows, then den)
+// on their way out as whole float4 image rows.  One warp per 8x8 block.
+template <int TS, bool LONG>
 struct FwdSmem {
   static constexpr int kThreads = 32 * (TS / 8) * (TS / 8);
   static constexpr int kWarps = kThreads / 32;
@@ -564,11 +560,15 @@ struct FwdSmem {
   // blocks each, four CTAs to an SM, were no gain for 32-px tiles: alone 312 us against 318 at
   // 3840x2160, but the 1024x1024 step 125 us against 117, the kernel overlapping its neighbours
   // less.
+  // LONG: for sets of long lists (kLongLists) the stage takes what is left of an SM's shared memory,
+  // so that fewer lists stream: the render of 500k Gaussians on 1920x1080 259 -> 223 us.  Lists of a
+  // hundred or two do better with the L1 cache that this costs (3840x2160 with 800k: 382 us against
+  // 393; the SSIM fit 566 against 595).
   static constexpr int kCtas = 1024 / kThreads;
-  static constexpr int kStage = TS == 32 ? kStageAll : 256;
+  static constexpr int kStage = TS == 32 ? (LONG ? 768 : 512) : 256;
   static constexpr int kNullSlot = kStage + kWarps * kCarrySlots;
   static constexpr int kSlots = kNullSlot + 1;
-  static constexpr int kListLen = kStage + 4;  // a whole stage's hits and padding
+  static constexpr int kListLen = (kStage < 512 ? kStage : 512) + 4;  // hits and padding
   static constexpr size_t kStageBytes = (size_t)kSlots * 4 * sizeof(float4);
   static constexpr size_t kRectBytes = (size_t)kStage * sizeof(int4);
   static constexpr size_t kListBytes = (size_t)kWarps * kListLen * sizeof(uint32_t);
@@ -659,8 +659,8 @@ __device__ __forceinline__ void stream_block(float4 (*stage)[4], int stage_slots
 // and adds each image's loss and mean squared error into loss[2 b], loss[2 b + 1]
 // (finish_pixel).  Each warp lists its block's hits (enqueue_hits), per staged chunk when
 // the list streams.
-template <int TS, bool NORMALIZE, bool FADE, int LOSS>
-__global__ void __launch_bounds__(FwdSmem<TS>::kThreads, FwdSmem<TS>::kCtas)
+template <int TS, bool LONG, bool NORMALIZE, bool FADE, int LOSS>
+__global__ void __launch_bounds__(FwdSmem<TS, LONG>::kThreads, (FwdSmem<TS, LONG>::kCtas))
     forward_kernel(const Splat* __restrict__ rec, int64_t n, const int32_t* __restrict__ gids,
                    int64_t cap, const int32_t* __restrict__ offsets, Frames frames, float eps,
                    float tail, float* __restrict__ out, float* __restrict__ den,
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(FwdSmem<TS>::kThreads, FwdSmem<TS>::kCtas)
                    float* __restrict__ loss, float charb_eps2, int chunk) {
   pdl_wait();
   pdl_trigger();
-  using S = FwdSmem<TS>;
+  using S = FwdSmem<TS, LONG>;
   constexpr int NT = S::kThreads;
   extern __shared__ __align__(16) unsigned char fwd_smem[];
   float4(*stage)[4] = reinterpret_cast<float4(*)[4]>(fwd_smem);
@@ -698,15 +698,18 @@ __global__ void __launch_bounds__(FwdSmem<TS>::kThreads, FwdSmem<TS>::kCtas)
     stage_with_masks<TS, NT, S::kStage>(stage, rec, L, m, rects, masks, tx0, ty0);
     cp_async_commit();
     __syncthreads();
-    int qn = 0;
-    for (int base = 0; base < m; base += 32)
+    int qn = 0, base = 0;
+    for (; base < m && qn + 32 + 3 <= S::kListLen; base += 32)
       qn = enqueue_hits(masks, base, m - base, block_bit, lane, list, qn);
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     const bool exact = !check_records<TS, NT>(stage, rects, nullptr, m, tx0, ty0);
     qn = cover_hits(stage, rects, list, 0, qn, sx0, sy0, lane);
-    drain<FADE>(stage, list, qn, true, exact, S::kNullSlot, lane, (float)(sx0 + (lane & 7)),
-                (float)sy0, tail, acc);
+    qn = drain<FADE>(stage, list, qn, base >= m, exact, S::kNullSlot, lane,
+                     (float)(sx0 + (lane & 7)), (float)sy0, tail, acc);
+    if (base < m)  // more hits than the list holds
+      block_hits<FADE>(stage, rects, masks, base, m - base, block_bit, list, S::kListLen, qn, true,
+                       exact, S::kNullSlot, sx0, sy0, lane, tail, acc);
   } else {
     // a streamed list moves through two chunks of `chunk` records (at most half the stage)
     stream_block<TS, NT, FADE, false>(stage, 2 * min(chunk, S::kStage / 2), rec, L, list,
@@ -846,7 +849,9 @@ __device__ __forceinline__ float4 finish_pixel_rt(int normalize, int loss_kind, 
 // cost-class order and counters, and in the fused pass the staged records' block masks.
 template <int TS, int NT, bool FUSED>
 struct BwdSmem {
-  static constexpr int kStageMax = Tiling<TS>::kBwdStageAll;
+  // whole-list stage: what the SM's shared memory holds beside the pixels, for four CTAs of a 32-px
+  // tile's eight warps or two of its sixteen
+  static constexpr int kStageMax = TS == 16 ? 512 : (NT == 512 ? 1152 : 448);
   static constexpr int kWarps = NT / 32;
   // fused pass only: every warp's carry slots, then the null record (slot kSlots - 1)
   static constexpr int kSlots = kStageMax + (FUSED ? kWarps * kCarrySlots + 1 : 0);
@@ -878,7 +883,7 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
   pdl_wait();
   pdl_trigger();
   using S = BwdSmem<TS, NT, FUSED>;
-  constexpr int kStageMax = Tiling<TS>::kBwdStageAll;
+  constexpr int kStageMax = S::kStageMax;
   constexpr int kHalf = kStageMax / 2;  // entries per chunk when a long list streams through
   extern __shared__ __align__(16) unsigned char bwd_smem[];
   float4(*stage)[4] = reinterpret_cast<float4(*)[4]>(bwd_smem);
@@ -1462,17 +1467,17 @@ int check_render_args(int64_t n, int H, int W, int ts, float eps) {
 // tuning knob per tile size (0 = half the stage).  Results do not depend on it.
 std::atomic<int> g_forward_chunk[2] = {{0}, {0}};
 
-template <int TS, bool NORM, bool FADE>
+template <int TS, bool LONG, bool NORM, bool FADE>
 void launch_forward_loss(int loss_kind, unsigned T, cudaStream_t s, const Splat* rec, int64_t n,
                          const int32_t* gids, int64_t cap, const int32_t* offsets,
                          const Frames& f, float eps, float tail, float* out, float* den,
                          const float* target, float4* pixel_grad, float* loss, float ce2) {
-  constexpr int NT = FwdSmem<TS>::kThreads;
+  constexpr int NT = FwdSmem<TS, LONG>::kThreads;
   const int c = g_forward_chunk[TS == 16 ? 0 : 1].load(std::memory_order_relaxed);
-  const int chunk = c ? c : kStageAll / 2;
+  const int chunk = c ? c : kForwardChunk;
 #define SS_FWD(LOSS)                                                                          \
-  launch_smem_as(T <= kDependentTiles, "forward_kernel", forward_kernel<TS, NORM, FADE, LOSS>, T, NT,                  \
-              FwdSmem<TS>::kBytes, s, rec, n, gids, cap, offsets, f, eps, tail, out, den,      \
+  launch_smem_as(T <= kDependentTiles, "forward_kernel", forward_kernel<TS, LONG, NORM, FADE, LOSS>, T, NT,                  \
+              (FwdSmem<TS, LONG>::kBytes), s, rec, n, gids, cap, offsets, f, eps, tail, out, den,      \
               target, pixel_grad, loss, ce2, chunk)
   switch (loss_kind) {
     case kL1: SS_FWD(kL1); break;
@@ -1489,13 +1494,19 @@ void launch_forward(int loss_kind, unsigned T, cudaStream_t s, const Splat* rec,
                     bool normalize, float eps, float tail, float* out, float* den,
                     const float* target, float4* pixel_grad, float* loss, float ce2) {
   const bool fade = tail > 0.0f;
+  const bool longer = TS == 32 && n > kLongLists * T;
 #define SS_FWD(NORM, FADE)                                                                     \
-  launch_forward_loss<TS, NORM, FADE>(loss_kind, T, s, rec, n, gids, cap, offsets, f, eps,     \
-                                      tail, out, den, target, pixel_grad, loss, ce2)
+  if (longer)                                                                                  \
+    launch_forward_loss<TS, TS == 32, NORM, FADE>(loss_kind, T, s, rec, n, gids, cap, offsets, \
+                                                  f, eps, tail, out, den, target, pixel_grad,  \
+                                                  loss, ce2);                                  \
+  else                                                                                         \
+    launch_forward_loss<TS, false, NORM, FADE>(loss_kind, T, s, rec, n, gids, cap, offsets, f, \
+                                               eps, tail, out, den, target, pixel_grad, loss, ce2)
   if (normalize) {
-    if (fade) SS_FWD(true, true); else SS_FWD(true, false);
+    if (fade) { SS_FWD(true, true); } else { SS_FWD(true, false); }
   } else {
-    if (fade) SS_FWD(false, true); else SS_FWD(false, false);
+    if (fade) { SS_FWD(false, true); } else { SS_FWD(false, false); }
   }
 #undef SS_FWD
 }
@@ -1503,14 +1514,20 @@ void launch_forward(int loss_kind, unsigned T, cudaStream_t s, const Splat* rec,
 // Warps per backward CTA: a process-wide tuning knob (0 = the default of the tile size).
 std::atomic<int> g_backward_warps[2] = {{0}, {0}};
 
-// Warps of a tile set's backward CTAs: as asked, else eight, or sixteen for a 32-px tile set of up to
-// kWideTiles, which leaves SMs idle or with one or two CTAs each: a tile's time is then the kernel's
-// (fit step of 64 tiles 45.0 -> 41.9 us).  Results do not depend on it.
+// Warps of a tile set's backward CTAs: as asked, else eight, or sixteen for 32-px tiles where
+//   there are up to kWideTiles, which leaves SMs idle or with one or two CTAs each: a tile's time is
+//   then the kernel's (fit step of 64 tiles 45.0 -> 41.9 us), or
+//   there are more than kLongLists Gaussians per tile: two CTAs instead of four share an SM's memory,
+//   so each stages 1,152 records instead of 448 and few lists stream; the fused pass's forward also
+//   streams once, not twice (2 M Gaussians on 2,040 tiles 1,103 -> 1,011 us a fit step, 250k
+//   heavy-tailed on 1,024 tiles 1,755 -> 1,671; at ~100 per tile eight warps win, 1,261 against
+//   1,524 us for the batched step).
+// Results do not depend on it.
 constexpr unsigned kWideTiles = 296;
-int backward_warps(int ts, unsigned T) {
+int backward_warps(int ts, unsigned T, int64_t n) {
   const int asked = g_backward_warps[ts == 16 ? 0 : 1].load(std::memory_order_relaxed);
   if (asked) return asked;
-  return ts == 32 && T <= kWideTiles ? 16 : 8;
+  return ts == 32 && (T <= kWideTiles || n > kLongLists * T) ? 16 : 8;
 }
 
 template <int TS, int NT, bool PIXGRAD>
@@ -1539,7 +1556,7 @@ void launch_backward(unsigned T, cudaStream_t s, int deterministic, const float*
                      const float4* pixel_grad, const int32_t* gids, int64_t cap,
                      const int32_t* offsets, const Frames& f, int normalize, float eps,
                      float tail, float* ws, uint32_t* status) {
-  const int warps = backward_warps(TS, T);
+  const int warps = backward_warps(TS, T, n);
   constexpr int kSmall = TS == 16 ? 128 : 256, kLarge = TS == 16 ? 256 : 512;
   if (warps * 32 == kSmall)
     launch_backward_nt<TS, kSmall, PIXGRAD>(T, s, deterministic, grad_out, rec, n, den, out,
@@ -1576,7 +1593,7 @@ void launch_fused(unsigned T, cudaStream_t s, int deterministic, const Splat* re
                   const int32_t* gids, int64_t cap, const int32_t* offsets, const Frames& f,
                   int normalize, float eps, float tail, float* ws, uint32_t* status,
                   const FusedFit& ff) {
-  const int warps = backward_warps(TS, T);
+  const int warps = backward_warps(TS, T, n);
   constexpr int kSmall = TS == 16 ? 128 : 256, kLarge = TS == 16 ? 256 : 512;
   if (warps * 32 == kSmall)
     launch_fused_nt<TS, kSmall>(T, s, deterministic, rec, n, gids, cap, offsets, f, normalize,
@@ -1768,9 +1785,9 @@ int ss_get_backward_warps(int tile_size) {
 int ss_set_forward_chunk(int tile_size, int records) {
   if (tile_size != 16 && tile_size != 32)
     return fail(SS_ERR_UNSUPPORTED, "render tile_size must be 16 or 32, got %d", tile_size);
-  if (records != 0 && records != 64 && records != 128 && records != kStageAll / 2)
+  if (records != 0 && records != 64 && records != 128 && records != kForwardChunk)
     return fail(SS_ERR_INVALID_ARGUMENT, "forward chunk must be 0, 64, 128 or %d records, got %d",
-                kStageAll / 2, records);
+                kForwardChunk, records);
   g_forward_chunk[tile_size == 16 ? 0 : 1].store(records, std::memory_order_relaxed);
   return SS_OK;
 }
@@ -1778,7 +1795,7 @@ int ss_set_forward_chunk(int tile_size, int records) {
 int ss_get_forward_chunk(int tile_size) {
   if (tile_size != 16 && tile_size != 32) return -1;
   const int c = g_forward_chunk[tile_size == 16 ? 0 : 1].load(std::memory_order_relaxed);
-  return c ? c : kStageAll / 2;
+  return c ? c : kForwardChunk;
 }
 
 int ss_render_backward_workspace_bytes(int64_t n, int64_t gid_capacity, int height, int width,
