@@ -19,6 +19,8 @@
 
 #include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 #include "ss_common.cuh"
 
@@ -58,18 +60,14 @@ __global__ void density_kernel(const float* __restrict__ energy, int64_t n,
   d[i] = __dadd_rn(base, __dmul_rn(1.0 - base, t));
 }
 
-__global__ void normalize_kernel(const double* d, double* out, int64_t n,
-                                 const double* __restrict__ sum, int uniform_if_empty) {
+__global__ void normalize_kernel(double* __restrict__ d, int64_t n,
+                                 const double* __restrict__ sum) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double s = *sum;
-  if (uniform_if_empty && !(s > 0.0)) {
-    out[i] = __ddiv_rn(1.0, (double)n);
-  } else {
-    out[i] = __ddiv_rn(d[i], s);
-  }
+  d[i] = s > 0.0 ? __ddiv_rn(d[i], s) : __ddiv_rn(1.0, (double)n);  // uniform without mass
 }
 
 __device__ __forceinline__ double reflect(double v, double hi) {
@@ -187,6 +185,28 @@ __device__ __forceinline__ float np_powerf(float x, float p) {
   return powf(x, p);
 }
 
+// Values at, at + 1, ..., at + 5 of an array of `len` (two neighbouring RGB pixels): the aligned
+// float4s that hold them, two or three loads instead of six.  Each lane of a warp reads somewhere
+// else, so a load costs the warp 32 cache lookups however little it fetches (2 M points on
+// 1920x1080: 85 -> 74 us).
+__device__ __forceinline__ void load_pair(const float* __restrict__ v, int64_t at, int64_t len,
+                                          float (&out)[6]) {
+  const int64_t base = at & ~int64_t(3);
+  const int shift = (int)(at - base);
+  if ((reinterpret_cast<uintptr_t>(v) & 15) || base + 12 > len) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) out[k] = __ldg(v + at + k);
+    return;
+  }
+  const float4* q = reinterpret_cast<const float4*>(v + base);
+  const float4 a = __ldg(q), b = __ldg(q + 1);
+  const float c = shift == 3 ? __ldg(v + base + 8) : 0.f;
+  const float w[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c};
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+    out[k] = shift == 0 ? w[k] : (shift == 1 ? w[k + 1] : (shift == 2 ? w[k + 2] : w[k + 3]));
+}
+
 struct PlaceParams {
   int anisotropic;
   float ratio_gain;        // max_axis_ratio - 1, as float (a weak Python scalar)
@@ -240,15 +260,15 @@ __global__ void place_kernel(const double* __restrict__ pts, int64_t n,
   // bilinear colour (init.py:39-49) in float64, left to right
   const double x = np_clip(px, 0.0, (double)W - 1.001), y = np_clip(py, 0.0, (double)H - 1.001);
   const int x0 = (int)floor(x), y0 = (int)floor(y);
-  const int x1 = x0 + 1, y1 = y0 + 1;
+  const int y1 = y0 + 1;
   const double fx = __dsub_rn(x, (double)x0), fy = __dsub_rn(y, (double)y0);
   const double gx = __dsub_rn(1.0, fx), gy = __dsub_rn(1.0, fy);
+  float up[6], down[6];
+  load_pair(image, ((int64_t)y0 * W + x0) * 3, (int64_t)H * W * 3, up);
+  load_pair(image, ((int64_t)y1 * W + x0) * 3, (int64_t)H * W * 3, down);
 #pragma unroll
   for (int ch = 0; ch < 3; ++ch) {
-    const double c00 = image[((int64_t)y0 * W + x0) * 3 + ch];
-    const double c01 = image[((int64_t)y0 * W + x1) * 3 + ch];
-    const double c10 = image[((int64_t)y1 * W + x0) * 3 + ch];
-    const double c11 = image[((int64_t)y1 * W + x1) * 3 + ch];
+    const double c00 = up[ch], c01 = up[3 + ch], c10 = down[ch], c11 = down[3 + ch];
     double c = __dmul_rn(__dmul_rn(c00, gx), gy);
     c = __dadd_rn(c, __dmul_rn(__dmul_rn(c01, fx), gy));
     c = __dadd_rn(c, __dmul_rn(__dmul_rn(c10, gx), fy));
@@ -267,10 +287,22 @@ struct PlaceWorkspace {
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// density[i] / *sum, divided as the scan reads it: a pass of 33 MB over a 1920x1080 density less.
+struct Scaled {
+  const double* density;
+  const double* sum;
+  __device__ double operator()(int64_t i) const { return __ddiv_rn(density[i], *sum); }
+};
+inline auto scaled_iter(const double* density, const double* sum) {
+  return thrust::make_transform_iterator(thrust::make_counting_iterator<int64_t>(0),
+                                         Scaled{density, sum});
+}
+
 size_t cub_bytes(int64_t npx) {
   size_t a = 0, b = 0;
   cub::DeviceReduce::Sum(nullptr, a, (const double*)nullptr, (double*)nullptr, (int)npx);
-  cub::DeviceScan::InclusiveSum(nullptr, b, (const double*)nullptr, (double*)nullptr, (int)npx);
+  cub::DeviceScan::InclusiveSum(nullptr, b, scaled_iter(nullptr, nullptr), (double*)nullptr,
+                                (int)npx);
   return a > b ? a : b;
 }
 
@@ -376,12 +408,13 @@ int ss_density_from_energy(const float* energy, int height, int width, double ba
     return fail(SS_ERR_INVALID_ARGUMENT, "placement workspace too small");
   PlaceWorkspace w = carve(workspace, npx);
   cudaStream_t s = as_stream(stream);
-  density_kernel<<<blocks_for(npx), kThreads, 0, s>>>(energy, npx, ref_dev, base, power, density);
+  launch("density_kernel", density_kernel, blocks_for(npx), kThreads, 0, s, energy, npx, ref_dev,
+         base, power, density);
   if ((rc = check_launch("density"))) return rc;
   size_t tb = w.temp_bytes;
   cudaError_t e = cub::DeviceReduce::Sum(w.temp, tb, density, w.sum, (int)npx, s);
   if (e != cudaSuccess) return fail(SS_ERR_CUDA, "density sum: %s", cudaGetErrorString(e));
-  normalize_kernel<<<blocks_for(npx), kThreads, 0, s>>>(density, density, npx, w.sum, 1);
+  normalize_kernel<<<blocks_for(npx), kThreads, 0, s>>>(density, npx, w.sum);
   return check_launch("density normalize");
 }
 
@@ -403,10 +436,8 @@ int ss_sample_candidates(const double* density, int height, int width, const dou
   size_t tb = w.temp_bytes;
   cudaError_t e = cub::DeviceReduce::Sum(w.temp, tb, density, w.sum, (int)npx, s);
   if (e != cudaSuccess) return fail(SS_ERR_CUDA, "sampler sum: %s", cudaGetErrorString(e));
-  normalize_kernel<<<blocks_for(npx), kThreads, 0, s>>>(density, w.cdf, npx, w.sum, 0);
-  if ((rc = check_launch("sampler normalize"))) return rc;
   tb = w.temp_bytes;
-  e = cub::DeviceScan::InclusiveSum(w.temp, tb, w.cdf, w.cdf, (int)npx, s);
+  e = cub::DeviceScan::InclusiveSum(w.temp, tb, scaled_iter(density, w.sum), w.cdf, (int)npx, s);
   if (e != cudaSuccess) return fail(SS_ERR_CUDA, "sampler cdf: %s", cudaGetErrorString(e));
   const int64_t buckets = guide_buckets(npx, n);
   if (buckets > 0) {
@@ -441,9 +472,9 @@ int ss_place_gaussians(const double* points, int64_t n, const double* density,
   pp.init_scale_mult = init_scale_mult;
   pp.n_points = (double)density_points;
   pp.quarter_turn = (float)(3.141592653589793 / 2.0);
-  place_kernel<<<blocks_for(n), kThreads, 0, as_stream(stream)>>>(
-      points, n, density, across_edge_angle, coherence, image, height, width, pp, means,
-      log_scales, rotations, colors);
+  launch("place_kernel", place_kernel, blocks_for(n), kThreads, 0, as_stream(stream), points, n,
+         density, across_edge_angle, coherence, image, height, width, pp, means, log_scales,
+         rotations, colors);
   return check_launch("place_gaussians");
 }
 
