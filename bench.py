@@ -675,7 +675,7 @@ def run_batched(args, dev, workload):
         "psnr_loop_mean": round(psum_loop / max(B_all, 1), 4),
         "psnr_max_abs_diff_vs_loop": round(dpsnr, 6),
         "psnr_after_steps": Wm + K, "index_overflow": overflow,
-        "gpu_launches_per_step": 8, "peak_mem_gb": round(mem_gb, 2), "clocks": clocks.summary(),
+        "gpu_launches_per_step": 6, "peak_mem_gb": round(mem_gb, 2), "clocks": clocks.summary(),
     }
     res["speedup_vs_loop_eager"] = round(res["batched_img_s"] / res["loop_eager_img_s"], 3)
     if tuned is not None:

@@ -4,12 +4,12 @@ The reference renders with one fixed shape (16x16 tiles, ``cuda_render.py:258``)
 workload picks, by timing on the GPU it runs on, among
 
 * render tile 16 or 32 (pixels per CTA; also the staging depth: a 32x32 tile stages its whole
-  list up to 512 Gaussians for the forward and 448 for the backward, a 16x16 tile up to 512,
-  longer lists stream through 64-record chunks), and
+  list up to 512 or 768 Gaussians for the forward and 448 or 1,152 for the backward, by its warps
+  and the Gaussians per tile, a 16x16 tile up to 256 and 512; longer lists stream), and
 * warps per backward CTA (4 or 8 for tile 16, 8 or 16 for tile 32), and
-* when the workload's longest tile list is longer than the forward's 512-record stage (the
-  list then streams through two chunks), the forward's chunk depth: 64, 128 or 256 records,
-  timed at the chosen shape.
+* when the workload's longest tile list is longer than 512 records (the forward then streams it
+  through two chunks, but for sets of long lists, which it stages up to 768), the forward's chunk
+  depth: 64, 128 or 256 records, timed at the chosen shape.
 
 The forward's threads follow the tile (one warp per 8x8 block).  Timing runs the render forward
 and backward of the actual workload (the field and images in hand), median of a few CUDA-event
@@ -33,7 +33,7 @@ from . import _native
 
 CANDIDATES = ((16, 4), (16, 8), (32, 8), (32, 16))
 CHUNKS = (64, 128, 256)  # forward records per streamed chunk
-STAGE_RECORDS = 512      # the forward's whole-list stage
+STAGE_RECORDS = 512      # the forward's whole-list stage at 32 px
 
 
 @dataclass

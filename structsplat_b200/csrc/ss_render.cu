@@ -1,15 +1,16 @@
 // Tiled forward and backward of the clipped-support normalized / additive renderer.
 //
 // Both kernels run one CTA per TS x TS tile (TS = 16 or 32) and stage the tile's Gaussian list
-// into shared memory with cp.async: whole when it fits (one barrier per tile), otherwise 64
-// records at a time, double-buffered, so the L2 gather of the next chunk overlaps the math on
+// into shared memory with cp.async: whole when it fits (one barrier per tile), otherwise in
+// double-buffered halves of the stage, so the L2 gather of the next chunk overlaps the math on
 // the current one.
 //
-// Forward (render_ext.cu:349-431 contract): each warp owns an 8x8 pixel block (two pixels per
-// lane, rows r and r+4).  For every 32 staged records a warp builds, with one ballot, the mask
-// of the Gaussians whose support rectangle touches its block and walks only those, in
-// ascending id; a lane masks its own pixels with the in-rectangle test.  The weight is 2^(qa dx^2 + qb dx dy + qc dy^2)
-// on the SFU.  The epilogue writes den raw and out = num / (den + eps) or num.
+// Forward (render_ext.cu:349-431 contract): each warp owns an 8x8 pixel block.  While the records
+// are copied, their rectangles become masks of the tile's blocks; from a ballot of its block's bit
+// over every 32 staged records a warp lists the Gaussians that touch the block, in ascending id,
+// with the columns and rows they cover.  It evaluates four of them at a time, eight lanes each, a
+// lane the eight pixels of one block column.  The weight is 2^(qa dx^2 + qb dx dy + qc dy^2) on the
+// SFU.  The epilogue writes den raw and out = num / (den + eps) or num.
 //
 // Backward (render_ext.cu:696-847 contract): a prologue turns grad_out, out and den into the
 // per-pixel (dnum_r, dnum_g, dnum_b, dden) of the tile in shared memory (the fit path hands
@@ -26,10 +27,11 @@
 // i.e. the reference's per-pixel formulas (render_ext.cu:785-818) summed over pixels.  Along a
 // column dx is constant, so S1, S3 and S4 fold into per-column products.  The moments are
 // reduce-scattered over the four lanes and added with one atomic per moment into per-Gaussian
-// accumulators (fast mode), or stored per (tile, Gaussian) entry, the entries ordered by
-// Gaussian with a stable radix sort, and summed per Gaussian in ascending tile order by a second
-// kernel (deterministic mode: every entry is computed by its own four lanes in a fixed order, so
-// the result does not depend on the scheduling).  A per-Gaussian epilogue applies o, a, b, c
+// accumulators (fast mode), or stored per (tile, Gaussian) entry and summed per Gaussian in
+// ascending tile order by a second kernel (deterministic mode: every entry is computed by its own
+// four lanes in a fixed order, so the result does not depend on the scheduling).  An entry's place
+// comes from its Gaussian's slots (entry_slots_kernel), or the entries are ordered by Gaussian
+// afterwards with a stable radix sort.  A per-Gaussian epilogue applies o, a, b, c
 // once.
 #include <atomic>
 
