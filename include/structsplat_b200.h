@@ -220,17 +220,20 @@ int ss_get_backward_warps(int tile_size);
 
 /* Launch tuning (process-wide): records per streamed chunk of the forward for a render tile
  * size — 64, 128 or 256, 0 restores the default (256).  Only tile lists longer than the
- * forward's 512-record stage stream; images do not depend on it.  ss_get_forward_chunk returns
+ * forward's stage (512 records, 768 for sets of long lists, 256 at 16 px) stream; images do not depend on it.  ss_get_forward_chunk returns
  * the value in effect (-1 for an unsupported tile size). */
 int ss_set_forward_chunk(int tile_size, int records);
 int ss_get_forward_chunk(int tile_size);
 
-/* `deterministic` of every backward, fit and finalize call: 0 adds with atomics; 1 and 2 are bitwise
+/* `deterministic` of every backward, fit and finalize call: 0 adds with atomics; 1 to 3 are bitwise
  * reproducible and give the same gradients.  1 takes any tile index and orders its entries by
  * Gaussian with a sort.  SS_DETERMINISTIC_SLOTS needs an index of whole images built without the
  * ellipse cull (each Gaussian listed in every tile of its rectangle) and no sort; with an index that
- * overflowed its capacity its gradients are zero.  One value for all calls on one workspace. */
+ * overflowed its capacity its gradients are zero.  SS_DETERMINISTIC_RUNS
+ * needs an index that this library built from these records, culled or not, and no sort.  One value
+ * for all calls on one workspace. */
 #define SS_DETERMINISTIC_SLOTS 2
+#define SS_DETERMINISTIC_RUNS 3
 /* Workspace of ss_render_backward: per-Gaussian moment accumulators (36 B per Gaussian) or,
  * deterministic, per-entry partials (48 B per entry of capacity); height and width are unused. */
 int ss_render_backward_workspace_bytes(int64_t n, int64_t gid_capacity, int height, int width,

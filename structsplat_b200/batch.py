@@ -130,8 +130,8 @@ class FitSettings:
     deterministic: bool = False
     # one tile kernel for forward, loss and backward (the same numbers as the two-kernel step);
     # None: fused in fast mode, two kernels in deterministic mode (where the fused kernel's extra
-    # registers spill: 9.75 vs 9.65 ms on the 2048^2 / 1 M stress step, 8.79 vs 9.20 ms fused
-    # on the 64-image batched step)
+    # registers spill: 1,728 against 1,675 us on a 1024^2 / 250k heavy-tailed step; a dense field of
+    # 2 M is faster fused, 1,057 against 1,117, most others are equal)
     fused: bool | None = None
 
     def use_fused(self) -> bool:

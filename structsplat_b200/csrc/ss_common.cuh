@@ -419,7 +419,9 @@ constexpr int kPartialFloats = 12;
 //   temp      the radix sort's scratch
 // In slot mode (kEntrySlots) no sort is needed: a Gaussian's partials have consecutive slots, one per
 // tile of its rectangle in ascending tile order, so seg alone tells where they lie.
+// kEntryRuns gives the sort's order without it, for an index of this library's own.
 constexpr int kEntrySlots = SS_DETERMINISTIC_SLOTS;
+constexpr int kEntryRuns = SS_DETERMINISTIC_RUNS;
 struct EntryOrder {
   float* partials;
   uint32_t* keys_in;

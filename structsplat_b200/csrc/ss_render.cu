@@ -31,7 +31,7 @@
 // ascending tile order by a second kernel (deterministic mode: every entry is computed by its own
 // four lanes in a fixed order, so the result does not depend on the scheduling).  An entry's place
 // comes from its Gaussian's slots (entry_slots_kernel), or the entries are ordered by Gaussian
-// afterwards with a stable radix sort.  A per-Gaussian epilogue applies o, a, b, c
+// afterwards (order_runs; for any index a stable radix sort).  A per-Gaussian epilogue applies o, a, b, c
 // once.
 #include <atomic>
 
@@ -1435,12 +1435,226 @@ int clear_entry_segments(void* ws, int64_t n, int64_t cap, cudaStream_t s) {
   return check_launch("entry segments zero-fill");
 }
 
-int order_entries(const int32_t* gids, const int32_t* offsets, int64_t T, int64_t cap,
+// kEntryRuns, after the backward: the same order without a sort, for an index of this library's own over
+// the same records (no Gaussian twice in a tile, and only in tiles that its rectangle touches).
+// An entry's rank among its Gaussian's is the number of the rectangle's earlier tiles that list it:
+// for a rectangle of up to kMaskTiles tiles the bits below its own in a mask of the tiles that do.
+// Larger rectangles' entries are ranked as they arrive, and their runs sorted by the entry's position.
+// Bound by the launches: these four in place of keys, a radix sort of the whole capacity, segments and
+// their memsets take a reproducible step with the fade from 85.7 to 59.8 us (20k Gaussians, 16-px
+// tiles), 69.5 to 39.0 (2k), 179 to 141 (100k on 1024x1024), 366 to 330 (250k); 250k heavy-tailed
+// Gaussians, whose long runs are sorted here, 1,393 and 1,386.
+constexpr int kMaskTiles = 32;
+constexpr int kMarkThreads = 128;
+constexpr int kWarpRun = 256;    // longest run sorted by one warp, in its share of shared memory
+constexpr int kWarpsPerCta = kEpilogueThreads / 32;
+
+// Tiles of rectangle r, and the place of tile (gx, gy) among them, row by row.
+__device__ __forceinline__ int rect_tiles(const int4& r, int ts) {
+  if (r.z <= r.x || r.w <= r.y) return 0;
+  const int64_t t = (int64_t)((r.z - 1) / ts - r.x / ts + 1) * ((r.w - 1) / ts - r.y / ts + 1);
+  return (int)min(t, (int64_t)INT32_MAX);
+}
+__device__ __forceinline__ int place_in_rect(const int4& r, int ts, int gx, int gy) {
+  const int gx0 = r.x / ts;
+  return (gy - r.y / ts) * ((r.z - 1) / ts - gx0 + 1) + (gx - gx0);
+}
+
+// Calls visit(gaussian, entry, rectangle, tile x, tile y) for the entries of this CTA's tile.  A tile
+// beyond the capacity has none: the backward left it out.
+template <typename Visit>
+__device__ __forceinline__ void for_entries(const Splat* rec, const int32_t* gids,
+                                            const int32_t* offsets, int64_t cap, int64_t n, int ts,
+                                            const Frames& frames, Visit visit) {
+  const int tile = blockIdx.x;
+  const Frame fr = frame_of_tile(frames, tile, n);
+  const TileList L = tile_list(gids, offsets, cap, fr, tile);
+  if (L.direct) return;
+  const int local = tile - fr.first_tile;
+  const int gx = local % fr.tiles_x, gy = local / fr.tiles_x;
+  for (int64_t k = threadIdx.x; k < L.count; k += kMarkThreads) {
+    const int g = gids[L.first + k];
+    visit(g, (int)(L.first + k), reinterpret_cast<const int4*>(rec + g)[3], gx, gy);
+  }
+}
+
+// seg[n + g]: the mask of Gaussian g's tiles, or how many entries it has; rank[entry] of the latter.
+__global__ void __launch_bounds__(kMarkThreads)
+    mark_entries_kernel(const Splat* __restrict__ rec, const int32_t* __restrict__ gids,
+                        const int32_t* __restrict__ offsets, int64_t cap, int64_t n, int ts,
+                        Frames frames, int32_t* __restrict__ seg, uint32_t* __restrict__ rank,
+                        unsigned* __restrict__ cursor) {
+  pdl_wait();
+  pdl_trigger();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *cursor = 0;
+  for_entries(rec, gids, offsets, cap, n, ts, frames,
+              [&](int g, int e, const int4& r, int gx, int gy) {
+                if (rect_tiles(r, ts) <= kMaskTiles)
+                  atomicOr(reinterpret_cast<unsigned*>(seg + n + g),
+                           1u << (place_in_rect(r, ts, gx, gy) & 31));
+                else
+                  rank[e] = (uint32_t)atomicAdd(seg + n + g, 1);
+              });
+}
+
+// Each Gaussian's run [seg[g], seg[n + g]), a CTA's side by side; masks[seg[g]] keeps its mask.
+__global__ void __launch_bounds__(kEpilogueThreads)
+    assign_runs_kernel(const Splat* __restrict__ rec, int64_t n, int ts,
+                       unsigned* __restrict__ cursor, uint32_t* __restrict__ masks,
+                       int32_t* __restrict__ seg) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ int warp_total[kWarpsPerCta];
+  __shared__ unsigned cta_first;
+  const int64_t g = (int64_t)blockIdx.x * kEpilogueThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int cnt = 0;
+  unsigned mask = 0;
+  if (g < n) {
+    cnt = seg[n + g];
+    if (rect_tiles(reinterpret_cast<const int4*>(rec + g)[3], ts) <= kMaskTiles) {
+      mask = (unsigned)cnt;
+      cnt = __popc(mask);
+    }
+  }
+  int incl = cnt;  // the total is at most the capacity, below 2^31
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_total[warp] = incl;
+  __syncthreads();
+  int before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kWarpsPerCta; ++w) {
+    before += w < warp ? warp_total[w] : 0;
+    total += warp_total[w];
+  }
+  if (threadIdx.x == 0) cta_first = atomicAdd(cursor, (unsigned)total);
+  __syncthreads();
+  if (g >= n) return;
+  const int beg = (int)cta_first + before + incl - cnt;
+  seg[g] = beg;
+  seg[n + g] = beg + cnt;
+  if (mask) masks[beg] = mask;
+}
+
+__global__ void __launch_bounds__(kMarkThreads)
+    place_entries_kernel(const Splat* __restrict__ rec, const int32_t* __restrict__ gids,
+                         const int32_t* __restrict__ offsets, int64_t cap, int64_t n, int ts,
+                         Frames frames, const int32_t* __restrict__ seg,
+                         const uint32_t* __restrict__ rank, const uint32_t* __restrict__ masks,
+                         int32_t* __restrict__ order) {
+  pdl_wait();
+  pdl_trigger();
+  for_entries(rec, gids, offsets, cap, n, ts, frames,
+              [&](int g, int e, const int4& r, int gx, int gy) {
+                const int beg = seg[g];
+                const int k = rect_tiles(r, ts) <= kMaskTiles
+                                  ? __popc(masks[beg] & ((1u << (place_in_rect(r, ts, gx, gy) & 31)) - 1u))
+                                  : (int)rank[e];
+                order[beg + k] = e;
+              });
+}
+
+// Ascending sort of v[0, m) by `threads` threads (t the caller's): a bitonic network whose every
+// exchange leaves the smaller value at the lower place, so the places from m up to the next power of
+// two need not exist.
+template <typename Sync>
+__device__ __forceinline__ void sort_ascending(int* v, int m, int t, int threads, Sync sync) {
+  int half = 1;  // pairs of the network: half the next power of two
+  while (2 * half < m) half <<= 1;
+  for (int size = 2; size <= 2 * half; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int p = t; p < half; p += threads) {
+        const int i = 2 * p - (p & (stride - 1));  // the lower of the pair's places
+        const int j = stride == (size >> 1) ? (i ^ (size - 1)) : i + stride;
+        if (j < m && v[i] > v[j]) {
+          const int x = v[i];
+          v[i] = v[j];
+          v[j] = x;
+        }
+      }
+      sync();
+    }
+  }
+}
+
+// The runs of rectangles of more than kMaskTiles tiles into ascending order: up to kWarpRun entries
+// by one warp, longer ones by the CTA, in shared memory where they fit.
+__global__ void __launch_bounds__(kEpilogueThreads)
+    sort_runs_kernel(const Splat* __restrict__ rec, int64_t n, int ts,
+                     const int32_t* __restrict__ seg, int32_t* __restrict__ order) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ int buf[kWarpsPerCta * kWarpRun];
+  __shared__ int longer[kEpilogueThreads], num_longer;
+  const int64_t g = (int64_t)blockIdx.x * kEpilogueThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) num_longer = 0;
+  __syncthreads();
+  int beg = 0, cnt = 0;
+  if (g < n && rect_tiles(reinterpret_cast<const int4*>(rec + g)[3], ts) > kMaskTiles) {
+    beg = seg[g];
+    cnt = seg[n + g] - beg;
+  }
+  if (cnt > kWarpRun) longer[atomicAdd(&num_longer, 1)] = threadIdx.x;
+  unsigned mine = __ballot_sync(0xffffffffu, cnt > 1 && cnt <= kWarpRun);
+  int* v = buf + warp * kWarpRun;
+  while (mine) {
+    const int l = __ffs(mine) - 1;
+    mine &= mine - 1;
+    const int b = __shfl_sync(0xffffffffu, beg, l), m = __shfl_sync(0xffffffffu, cnt, l);
+    for (int k = lane; k < m; k += 32) v[k] = order[b + k];
+    __syncwarp();
+    sort_ascending(v, m, lane, 32, [] { __syncwarp(); });
+    for (int k = lane; k < m; k += 32) order[b + k] = v[k];
+    __syncwarp();
+  }
+  __syncthreads();
+  const int todo = num_longer;
+  for (int i = 0; i < todo; ++i) {
+    const int64_t h = (int64_t)blockIdx.x * kEpilogueThreads + longer[i];
+    const int b = seg[h], m = seg[n + h] - b;
+    const bool fits = m <= kWarpsPerCta * kWarpRun;
+    int* w = fits ? buf : order + b;
+    if (fits)
+      for (int k = threadIdx.x; k < m; k += kEpilogueThreads) buf[k] = order[b + k];
+    __syncthreads();
+    sort_ascending(w, m, threadIdx.x, kEpilogueThreads, [] { __syncthreads(); });
+    if (fits)
+      for (int k = threadIdx.x; k < m; k += kEpilogueThreads) order[b + k] = buf[k];
+    __syncthreads();
+  }
+}
+
+int order_runs(const Frames& f, int ts, const void* records, const int32_t* gids,
+               const int32_t* offsets, int64_t T, int64_t cap, int64_t n, const EntryOrder& eo,
+               cudaStream_t s) {
+  const Splat* rec = static_cast<const Splat*>(records);
+  const unsigned gblocks = (unsigned)((n + kEpilogueThreads - 1) / kEpilogueThreads);
+  unsigned* cursor = reinterpret_cast<unsigned*>(eo.order_in);
+  launch("mark_entries_kernel", mark_entries_kernel, (unsigned)T, kMarkThreads, 0, s, rec, gids,
+         offsets, cap, n, ts, f, eo.seg, eo.keys_in, cursor);
+  launch("assign_runs_kernel", assign_runs_kernel, gblocks, kEpilogueThreads, 0, s, rec, n, ts, cursor,
+         eo.keys, eo.seg);
+  launch("place_entries_kernel", place_entries_kernel, (unsigned)T, kMarkThreads, 0, s, rec, gids,
+         offsets, cap, n, ts, f, eo.seg, eo.keys_in, eo.keys, eo.order);
+  launch("sort_runs_kernel", sort_runs_kernel, gblocks, kEpilogueThreads, 0, s, rec, n, ts, eo.seg,
+         eo.order);
+  return check_launch("entry runs");
+}
+
+int order_entries(const Frames& f, int ts, const void* records, int deterministic,
+                  const int32_t* gids, const int32_t* offsets, int64_t T, int64_t cap,
                   int64_t n, void* ws, cudaStream_t s) {
   int rc;
   if ((rc = clear_entry_segments(ws, n, cap, s))) return rc;
   if (cap == 0) return SS_OK;
   const EntryOrder eo = entry_order_layout(ws, n, cap);
+  if (deterministic == kEntryRuns)
+    return order_runs(f, ts, records, gids, offsets, T, cap, n, eo, s);
   const int64_t want = (cap + kEpilogueThreads - 1) / kEpilogueThreads;
   const unsigned blocks = (unsigned)(want < 148 * 16 ? want : 148 * 16);
   launch("entry_keys_kernel", entry_keys_kernel, blocks, kEpilogueThreads, 0, s, gids, offsets, T, cap, n, eo.keys_in,
@@ -1659,7 +1873,7 @@ int render_backward_tiles(const Frames& f, int ts, int64_t T, const float* grad_
   }
   rc = check_launch("render_backward");
   if (rc || !deterministic || deterministic == kEntrySlots) return rc;
-  return order_entries(gids, offsets, T, cap, n, ws, s);
+  return order_entries(f, ts, records, deterministic, gids, offsets, T, cap, n, ws, s);
 }
 
 size_t backward_ws_bytes(int64_t n, int64_t cap, int deterministic) {
@@ -2043,7 +2257,8 @@ int ss_fit_forward_backward(const ss_batch* batch, const void* records, int64_t 
                      tile_offsets, f, normalize, eps, fade_tail, ws, status, ff);
   if ((rc = check_launch("fit forward + backward"))) return rc;
   if (!deterministic || deterministic == kEntrySlots || n == 0) return SS_OK;
-  return order_entries(tile_gids, tile_offsets, T, gid_capacity, n, workspace, s);
+  return order_entries(f, batch->tile_size, records, deterministic, tile_gids, tile_offsets, T,
+                       gid_capacity, n, workspace, s);
 }
 
 int ss_render_forward_backward(const void* records, int64_t n, const int32_t* tile_gids,
@@ -2087,7 +2302,8 @@ int ss_render_forward_backward(const void* records, int64_t n, const int32_t* ti
                      tile_offsets, f, normalize, eps, fade_tail, ws, status, ff);
   if ((rc = check_launch("render forward + backward"))) return rc;
   if (!deterministic || deterministic == kEntrySlots || n == 0) return SS_OK;
-  return order_entries(tile_gids, tile_offsets, T, gid_capacity, n, workspace, s);
+  return order_entries(f, tile_size, records, deterministic, tile_gids, tile_offsets, T,
+                       gid_capacity, n, workspace, s);
 }
 
 }  // extern "C"

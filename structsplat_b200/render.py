@@ -77,9 +77,10 @@ def fade_tail(sigma_cutoff: float, alpha: float) -> float:
 
 def deterministic_mode(deterministic: bool, cull: bool) -> int:
     """The library's ``deterministic`` argument: 0 fast, 2 (slots) where the tile index holds every
-    tile of each rectangle, 1 (sorted entries) where the ellipse cull drops some.  The gradients
-    of 1 and 2 are bitwise the same."""
-    return 0 if not deterministic else (1 if cull else 2)
+    tile of each rectangle, 3 (runs) where the ellipse cull drops some.  Both need an index that
+    was built here from the same records; 1, which sorts, takes any.  The gradients of 1 to 3 are
+    bitwise the same."""
+    return 0 if not deterministic else (3 if cull else 2)
 
 
 def tile_grid(H: int, W: int, tile_size: int) -> tuple[int, int]:
