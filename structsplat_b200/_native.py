@@ -55,6 +55,7 @@ SIGNATURES = {
     "ss_project_rs_backward": [_vp, _vp, _vp, _i64, _f32, _vp, _vp, _vp, _vp, _vp, _vp],
     "ss_tile_index_workspace_bytes": [_i64, _int, _int, _int, _szp],
     "ss_tile_index_binned_workspace_bytes": [_i64, _int, _int, _int, _szp],
+    "ss_tile_index_entries_workspace_bytes": [_i64, _i64, _int, _i64, _szp],
     "ss_tile_index_count": [_vp, _i64, _int, _int, _int, _int, _f32, _vp, _vp, ctypes.c_size_t,
                             _vp, _vp],
     "ss_tile_index_fill": [_vp, _i64, _int, _int, _int, _int, _f32, _vp, _vp, _i64, _vp,

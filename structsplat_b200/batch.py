@@ -178,11 +178,11 @@ class FitPlan:
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, **f32)
         self.offsets = torch.zeros(batch.tiles + 1, device=d, dtype=torch.int32)
         self.status = torch.zeros(1, device=d, dtype=torch.int32)
-        self.idx_ws_bytes = _native.size_query("ss_batch_tile_index_binned_workspace_bytes",
-                                               batch.ref, n)
-        self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=d, dtype=torch.uint8)
+        self.entries = 0  # as measured last
+        self._size_index(0)
         if capacity <= 0:
             capacity = self.measure_entries() * 3 // 2 + 4096
+            self._size_index(self.entries)
         self.capacity = int(capacity)
         self.gids = torch.empty(self.capacity, device=d, dtype=torch.int32)
         self.bwd_ws_bytes = _native.size_query("ss_fit_backward_workspace_bytes", n,
@@ -227,7 +227,15 @@ class FitPlan:
         """Tile-list total of the current field (one host sync)."""
         self.project()
         self.count()
-        return int(self.offsets[-1].item())
+        self.entries = int(self.offsets[-1].item())
+        return self.entries
+
+    def _size_index(self, entries: int):
+        """The index workspace for about ``entries`` tile-list entries (0: not known)."""
+        self.idx_ws_bytes = _native.size_query("ss_tile_index_entries_workspace_bytes", self.n,
+                                               self.batch.tiles, self.batch.images, entries)
+        self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=self.batch.device,
+                                  dtype=torch.uint8)
 
     # -- stages ------------------------------------------------------------------------
     def project(self):
@@ -470,6 +478,7 @@ def fit_batch(fields, targets, iters: int = 100, settings: FitSettings | None = 
 
 def _replan(plan: FitPlan, capacity: int) -> FitPlan:
     new = FitPlan(plan.batch, plan.params, plan.target, plan.s, capacity=capacity)
+    new._size_index(plan.entries)
     for k in plan.exp_avg:
         new.exp_avg[k].copy_(plan.exp_avg[k])
         new.exp_avg_sq[k].copy_(plan.exp_avg_sq[k])

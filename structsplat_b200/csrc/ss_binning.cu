@@ -11,7 +11,7 @@
 //     pair's rank in its tile, so the same kernel drops the id into the tile's bin, and
 //     bin_sort_kernel orders each bin into the list.  At 100k Gaussians on 1024x1024 (213k pairs)
 //     the fill, warp-sort and block-sort launches after the count took 12 + 6.4 + 4.2 us; this one
-//     takes their place.
+//     takes their place, and lists the few tiles whose bins overflowed.
 //   plain (a workspace of ss_tile_index_workspace_bytes, which depends on the tiles only): the
 //     fill enumerates the pairs again and claims slots with per-tile atomic cursors, then a
 //     warp or a CTA sorts each list.
@@ -72,8 +72,9 @@ struct IndexWorkspace {
   int bin_ids;            // K, ids a bin holds
 };
 
-// Ids per bin: 32 times the Gaussians per tile (lists average 2 to 8 times them; a tile beyond
-// that is rebuilt from the records by bin_sort_kernel).  0, no bins, without Gaussians or tiles and
+// Ids per bin: 32 times the Gaussians per tile.  Lists of 32-px tiles average 2 to 8 times them, those
+// of smaller tiles or wider Gaussians more (ss_tile_index_entries_workspace_bytes then names the plain
+// form); a tile beyond its bin is listed by bin_sort_kernel.  0, no bins, without Gaussians or tiles and
 // where very many tiles would make them larger than 256 MB + 256 B per Gaussian.
 int bin_ids_for(int64_t n, int64_t T) {
   if (n <= 0 || T <= 0) return 0;
@@ -154,15 +155,14 @@ __device__ __forceinline__ TileRect tile_rect_of(const Splat* rec, int64_t i, in
   return tile_rect(reinterpret_cast<const int4*>(rec + i)[3], ts);
 }
 
-// Calls visit(gaussian, tile) for every (tile, Gaussian) pair of the index, in any order.
+// Calls visit(slot, gaussian, tile) for every tile of Gaussian i of each lane of a warp, in any order.
 // Each lane enumerates a rectangle of up to kSmallRect tiles itself (unrolled, so independent
 // atomics are in flight together); a larger rectangle is enumerated by the whole warp so one
 // huge Gaussian cannot serialise a lane.  Tile coordinates advance incrementally (no division).
 template <bool CULL, typename Visit>
-__device__ __forceinline__ void enumerate_pairs(const Splat* rec, int64_t n, int ts,
+__device__ __forceinline__ void enumerate_pairs(const Splat* rec, int64_t i, int64_t n, int ts,
                                                 const Frames& frames, float cutoff2,
                                                 Visit visit) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int lane = threadIdx.x & 31;
   TileRect r{0, 0, 0, 0};
   int tiles_x = 0, first_tile = 0;
@@ -215,6 +215,31 @@ __device__ __forceinline__ void enumerate_pairs(const Splat* rec, int64_t n, int
       }
     }
   }
+}
+
+// Whether a tile whose bin does not hold its list of len ids is listed by testing every record of its
+// image, or else from the pairs (place_overflow).  A CTA tests ~0.25 records per ns, so lists of more
+// than 1/8 of the image's Gaussians are sooner found that way (`tests` 8), and all of them where the
+// whole set's tests are few (see index_tests).  Long lists of large images count for more: from the pairs
+// they would be sorted in place.  Either way the work is bounded by the pairs or by kFewTests.
+constexpr int kSortIds = 4096;                      // most ids sorted in shared memory
+constexpr int kWindowIds = 32 * (kSortIds + 1024);  // most ids a bitmap there holds: 163,840
+constexpr int64_t kFewTests = 1 << 24;              // ~45 us
+inline int index_tests(int64_t n, int64_t T) { return n * T <= kFewTests ? INT_MAX : 8; }
+__host__ __device__ inline bool listed_from_records(int64_t len, int64_t count, int tests) {
+  return len * (len > kSortIds && count > kWindowIds && tests < 64 ? 64 : tests) >= count;
+}
+
+// Words in the padding after the counters, zeroed with them.  Of counter 0: the bins' size, whether
+// some tile needs place_overflow, and its tickets; of each counter: the slots claimed in its list.
+constexpr int kBinsWord = 2, kOverflowWord = 3, kTicketWord = 5, kPlacedWord = 6, kExitWord = 7;
+constexpr int kClaimWord = 4;
+// Notes that a tile of cnt pairs needs place_overflow.
+__device__ __forceinline__ void note_overflow(int64_t cnt, int64_t t, const Frames& frames,
+                                              int64_t n, int K, int tests, int* tile_count) {
+  if (K > 0 && cnt > K &&
+      !listed_from_records(cnt, frame_of_tile(frames, (int)t, n).gauss_count, tests))
+    tile_count[kOverflowWord] = 1;
 }
 
 // Counts one CTA's pairs: thread l holds Gaussian `first + l` with record s (`in`: there is one).
@@ -337,8 +362,8 @@ __device__ __forceinline__ void count_pairs(const Splat& s, bool in, int first, 
   }
 }
 
-// Per-tile counts by atomics, and with BINS the bins.  The second padding word after counter 0
-// (zeroed with the counters) tells bin_sort_kernel that the bins belong to these counts.
+// Per-tile counts by atomics, and with BINS the bins.  A padding word of counter 0 tells
+// bin_sort_kernel that the bins belong to these counts.
 template <bool CULL, bool BINS>
 __global__ void tile_count_kernel(const Splat* __restrict__ rec, int64_t n, int ts, Frames frames,
                                   float cutoff2, int* __restrict__ tile_count,
@@ -346,7 +371,7 @@ __global__ void tile_count_kernel(const Splat* __restrict__ rec, int64_t n, int 
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (BINS && i == 0) tile_count[2] = K;
+  if (BINS && i == 0) tile_count[kBinsWord] = K;
   Splat s{};
   int tiles_x = 0, first_tile = 0;
   if (i < n) {
@@ -380,7 +405,7 @@ __global__ void project_count_kernel(RSField field, int64_t n, int ts, Frames fr
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (BINS && i == 0) tile_count[2] = K;
+  if (BINS && i == 0) tile_count[kBinsWord] = K;
   for (int64_t v = i; v < clear_vec; v += (int64_t)gridDim.x * blockDim.x)
     clear[v] = make_uint4(0u, 0u, 0u, 0u);
   Splat s{};
@@ -414,7 +439,7 @@ __global__ void pack_count_kernel(PackField f, int64_t n, int ts, Frames frames,
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (BINS && i == 0) tile_count[2] = K;
+  if (BINS && i == 0) tile_count[kBinsWord] = K;
   for (int64_t v = i; v < clear_vec; v += (int64_t)gridDim.x * blockDim.x)
     clear[v] = make_uint4(0u, 0u, 0u, 0u);
   Splat s{};
@@ -434,13 +459,16 @@ __global__ void tile_fill_kernel(const Splat* __restrict__ rec, int64_t n, int t
                                  float cutoff2, int64_t T, const long long* __restrict__ off64,
                                  int* __restrict__ tile_count, int32_t* __restrict__ offsets32,
                                  int32_t* __restrict__ gids, int64_t cap, int* big_count,
-                                 uint32_t* status) {
+                                 uint32_t* status, int K, int tests, int64_t gaussians) {
   pdl_wait();
   pdl_trigger();
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   long long total = off64[T];
-  for (int64_t t = tid; t <= T; t += stride) offsets32[t] = (int32_t)min(off64[t], 2147483647LL);
+  for (int64_t t = tid; t <= T; t += stride) {
+    offsets32[t] = (int32_t)min(off64[t], 2147483647LL);
+    if (t < T) note_overflow(off64[t + 1] - off64[t], t, frames, gaussians, K, tests, tile_count);
+  }
   if (tid == 0) {
     *big_count = 0;
     if (total > 2147483647LL) raise_status(status, SS_STATUS_INDEX_INT32);
@@ -450,7 +478,7 @@ __global__ void tile_fill_kernel(const Splat* __restrict__ rec, int64_t n, int t
 #pragma unroll
   for (int k = 0; k < kSmallRect; ++k) pos[k] = -1;
   int owner = -1;
-  enumerate_pairs<CULL>(rec, n, ts, frames, cutoff2, [&](int k, int g, int t) {
+  enumerate_pairs<CULL>(rec, tid, n, ts, frames, cutoff2, [&](int k, int g, int t) {
     long long p = off64[t] + (atomicSub(tile_count + (int64_t)t * kCounterStride, 1) - 1);
     if (k < 0) {
       if (p < cap) gids[p] = g;
@@ -486,8 +514,8 @@ __device__ __forceinline__ long long warp_inclusive(long long v, int lane) {
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    scan_counts_kernel(const int* __restrict__ tile_count, int64_t items,
-                       long long* __restrict__ off64, int32_t* __restrict__ off32) {
+    scan_counts_kernel(int* __restrict__ tile_count, int64_t items, long long* __restrict__ off64,
+                       int32_t* __restrict__ off32, Frames frames, int64_t n, int K, int tests) {
   pdl_wait();
   pdl_trigger();
   __shared__ long long before[kScanThreads / 32], warp_total[kScanThreads / 32];
@@ -517,6 +545,7 @@ __global__ void __launch_bounds__(kScanThreads)
     const long long o = warp_total[warp] + (incl - own);
     off64[idx] = o;
     off32[idx] = (int32_t)(o < 2147483647LL ? o : 2147483647LL);
+    if (idx + 1 < items) note_overflow(own, idx, frames, n, K, tests, tile_count);
   }
 }
 
@@ -708,19 +737,19 @@ __global__ void __launch_bounds__(1024) tile_sort_big_kernel(const int32_t* __re
 //             tile's ids side by side): a bit per Gaussian of the image in shared memory, set from
 //             the bin and read back in order, one window of ids after the other, windows without
 //             ids skipped.  Costs the list plus 1/32 of the window, however the ids lie.
-//   rebuilt   a tile whose bin overflowed: the windows again, set by testing every record of the
-//             image instead.
+//   records   a tile whose bin overflowed with a good part of the image's Gaussians: the windows again,
+//             set by testing every record of the image instead.
+//   pairs     other tiles whose bin overflowed: place_overflow.
 //
 // Bound by latency (a few dependent L2 reads and block-wide steps per tile), hence small CTAs, 10 to
 // an SM.  Lists of ~1,100 of 2 M ids on 2,040 tiles took 39 + 161 us in the warp and block sorts of
 // the plain form, lists of ~2,000 of 250 k on 1,024 tiles 35 + 81 us; here 29 and 22 us.
 constexpr int kSortThreads = 128;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortIds = 4096;
 constexpr int kBuckets = 1024;
 constexpr int kBucketIds = 24;
 constexpr int kWindowWords = kSortIds + kBuckets;
-constexpr int kWindowIds = 32 * kWindowWords;  // 163,840
+static_assert(kWindowIds == 32 * kWindowWords, "one bitmap");
 constexpr int kBitmapIds = 32 * kSortIds;      // a window below the bucket prefixes: 131,072
 
 // Exclusive prefix of v over the CTA's threads (tmp: kSortWarps + 1 words, ends holding the total
@@ -769,13 +798,18 @@ __device__ __forceinline__ int emit_bits(const uint32_t* words, int nw, int firs
   return tmp[kSortWarps];
 }
 
+// A list that other CTAs have just placed: not to be read from the L1.
+struct PlacedIds {
+  const int32_t* p;
+  __device__ __forceinline__ int operator[](int e) const { return __ldcg(p + e); }
+};
+
 // Orders a bin of len <= kSortIds ids by NB buckets of 2^shift ids and writes it to g; false,
-// with nothing written and the buckets' prefixes in hist, when some bucket is too full.  Called by
-// every thread.
-template <int NB>
-__device__ __forceinline__ bool bucket_sort(const int32_t* __restrict__ bin, int len, int first,
-                                            int count, int* buf, int* hist, int* tmp,
-                                            int32_t* __restrict__ g, int& shift) {
+// with nothing written and the buckets' prefixes in hist, when some bucket is too full (the bin may be
+// g itself).  Called by every thread.
+template <int NB, typename Bin>
+__device__ __forceinline__ bool bucket_sort(Bin bin, int len, int first, int count, int* buf,
+                                            int* hist, int* tmp, int32_t* g, int& shift) {
   constexpr int kOwn = NB / kSortThreads;
   shift = 0;
   while (((count - 1) >> shift) >= NB) ++shift;
@@ -822,9 +856,9 @@ __device__ __forceinline__ bool bucket_sort(const int32_t* __restrict__ bin, int
 
 // One tile by the whole CTA (see above).  Every thread calls it.
 template <bool CULL>
-__device__ __noinline__ void cta_sort_bin(const Splat* __restrict__ rec, int64_t n, int ts,
+__device__ __forceinline__ void cta_sort_bin(const Splat* __restrict__ rec, int64_t n, int ts,
                                           const Frames& frames, float cutoff2, int t,
-                                          long long lo, int len, bool rebuild,
+                                          long long lo, int len, bool records,
                                           const int32_t* __restrict__ bin,
                                           int32_t* __restrict__ gids, uint32_t* smem, int* tmp) {
   const Frame fr = frame_of_tile(frames, t, n);
@@ -835,27 +869,36 @@ __device__ __noinline__ void cta_sort_bin(const Splat* __restrict__ rec, int64_t
     for (int w = threadIdx.x; w < nw; w += kSortThreads) smem[w] = 0u;
     __syncthreads();
   };
-  if (rebuild) {
+  if (records) {
     const int local = t - fr.first_tile;
     const int gx = local % fr.tiles_x, gy = local / fr.tiles_x;
     const int px0 = gx * ts, py0 = gy * ts;
     int done = 0;
     for (int w0 = 0; w0 < count; w0 += kWindowIds) {
       const int ids = min(count - w0, kWindowIds), nw = (ids + 31) >> 5;
-      // a warp tests 32 consecutive records: their ballot is the bitmap's word
-#pragma unroll 4
-      for (int w = threadIdx.x >> 5; w < nw; w += kSortWarps) {
-        const int rel = 32 * w + (threadIdx.x & 31);
-        bool hit = false;
-        if (rel < ids) {
-          const int64_t i = (int64_t)first + w0 + rel;
-          const int4 b = reinterpret_cast<const int4*>(rec + i)[3];
-          hit = b.z > b.x && b.w > b.y && b.x < px0 + ts && b.z > px0 && b.y < py0 + ts &&
-                b.w > py0;
-          if (CULL && hit) hit = !culled(load_splat(rec, i), gx, gy, ts, cutoff2);
+      // a warp tests 32 consecutive records, whose ballot is the bitmap's word; eight words' loads in
+      // flight
+      constexpr int kWords = 8;
+      for (int wa = threadIdx.x >> 5; wa < nw; wa += kWords * kSortWarps) {
+        int4 b[kWords];
+#pragma unroll
+        for (int u = 0; u < kWords; ++u) {
+          const int rel = 32 * (wa + u * kSortWarps) + (threadIdx.x & 31);
+          b[u] = rel < ids ? reinterpret_cast<const int4*>(rec + first + w0 + rel)[3]
+                           : make_int4(0, 0, 0, 0);
         }
-        const unsigned word = __ballot_sync(0xffffffffu, hit);
-        if ((threadIdx.x & 31) == 0) smem[w] = word;
+#pragma unroll
+        for (int u = 0; u < kWords; ++u) {
+          const int w = wa + u * kSortWarps;
+          if (w >= nw) break;
+          bool hit = b[u].z > b[u].x && b[u].w > b[u].y && b[u].x < px0 + ts && b[u].z > px0 &&
+                     b[u].y < py0 + ts && b[u].w > py0;
+          if (CULL && hit)
+            hit = !culled(load_splat(rec, (int64_t)first + w0 + 32 * w + (threadIdx.x & 31)), gx, gy,
+                          ts, cutoff2);
+          const unsigned word = __ballot_sync(0xffffffffu, hit);
+          if ((threadIdx.x & 31) == 0) smem[w] = word;
+        }
       }
       __syncthreads();
       done += emit_bits(smem, nw, first + w0, g + done, len - done, tmp);
@@ -907,6 +950,156 @@ __device__ __noinline__ void cta_sort_bin(const Splat* __restrict__ rec, int64_t
   }
 }
 
+// Puts g[0, len), a list in arrival order, into ascending order.  Every thread of the CTA calls it.
+__device__ __noinline__ void sort_placed(int32_t* g, int len, int first, int count, uint32_t* smem,
+                                         int* tmp) {
+  const PlacedIds list{g};
+  int* buf = reinterpret_cast<int*>(smem);
+  int shift = 0;
+  if (len <= 512) {
+    if (bucket_sort<256>(list, len, first, count, buf, buf + kSortIds, tmp, g, shift)) return;
+  } else if (len <= kSortIds) {
+    if (bucket_sort<kBuckets>(list, len, first, count, buf, buf + kSortIds, tmp, g, shift)) return;
+  }
+  __syncthreads();  // every thread has left the buckets
+  auto sync = [] { __syncthreads(); };
+  if (count <= kWindowIds) {
+    const int nw = (count + 31) >> 5;
+    for (int w = threadIdx.x; w < nw; w += kSortThreads) smem[w] = 0u;
+    __syncthreads();
+    for (int e = threadIdx.x; e < len; e += kSortThreads) {
+      const int rel = list[e] - first;
+      atomicOr(&smem[rel >> 5], 1u << (rel & 31));
+    }
+    __syncthreads();
+    emit_bits(smem, nw, first, g, len, tmp);
+  } else if (len <= kSortIds) {
+    for (int e = threadIdx.x; e < len; e += kSortThreads) buf[e] = list[e];
+    __syncthreads();
+    bitonic_sort(buf, len, threadIdx.x, kSortThreads, sync);
+    for (int e = threadIdx.x; e < len; e += kSortThreads) g[e] = buf[e];
+  } else {
+    bitonic_sort(g, len, threadIdx.x, kSortThreads, sync);
+  }
+}
+
+// The tiles whose bins do not hold their lists.
+struct Overflow {
+  int K, tests;
+  bool trusted;  // the bins belong to the counts
+  __device__ __forceinline__ bool beyond(int64_t len) const { return len > K || !trusted; }
+  __device__ __forceinline__ bool records(int64_t len, int64_t count) const {
+    return listed_from_records(len, count, tests);
+  }
+};
+
+// Places the ids of the tiles beyond their bins that listed_from_records leaves in their lists, by a
+// cursor per tile: share `part` of `parts` of the pairs.  A warp takes `lanes` Gaussians at a time and
+// shares their pairs evenly, four per lane in flight (it waits on the offsets and cursors in the L2).
+template <bool CULL>
+__device__ __noinline__ void place_overflow(const Splat* __restrict__ rec, int64_t n, int ts,
+                                            const Frames& frames, float cutoff2,
+                                            const long long* __restrict__ off64, int* tile_count,
+                                            const Overflow over, int32_t* gids, int64_t cap,
+                                            int part, int parts, int lanes) {
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t warp = (int64_t)part * kSortWarps + (threadIdx.x >> 5);
+  for (int64_t b = lanes * warp; b < n; b += (int64_t)lanes * parts * kSortWarps) {
+    const int64_t i = b + lane;
+    TileRect r{0, 0, 0, 0};
+    int tiles_x = 0, first_tile = 0, images = 0;
+    if (lane < lanes && i < n) {
+      r = tile_rect_of(rec, i, ts);
+      const Frame fr = frame_of_gaussian(frames, i, n);
+      tiles_x = fr.tiles_x;
+      first_tile = fr.first_tile;
+      images = fr.gauss_count;
+    }
+    const int cnt = r.gw * r.gh;
+    const int own = cnt > kHugeRect ? 0 : cnt;
+    int incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(all, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const int excl = incl - own, total = __shfl_sync(all, incl, 31);
+    const int corner = first_tile + r.gy0 * tiles_x + r.gx0;
+    // tile k of lane l's rectangle, its list's first slot and length; -1 when not placed here
+    auto tile_of = [&](int l, unsigned k, bool some, long long& lo, int& len) {
+      const unsigned gw = (unsigned)__shfl_sync(all, r.gw, l);
+      const int tx = __shfl_sync(all, tiles_x, l), c = __shfl_sync(all, corner, l);
+      const int count = __shfl_sync(all, images, l);
+      const int gx0 = __shfl_sync(all, r.gx0, l), gy0 = __shfl_sync(all, r.gy0, l);
+      if (!some) return -1;
+      const int row = (int)(k / gw), col = (int)(k - (unsigned)row * gw);
+      if (CULL && culled(load_splat(rec, b + l), gx0 + col, gy0 + row, ts, cutoff2)) return -1;
+      const int t = c + row * tx + col;
+      lo = off64[t];
+      const long long hi = off64[t + 1];
+      len = (int)(hi - lo);
+      return hi > cap || !over.beyond(hi - lo) || over.records(hi - lo, count) ? -1 : t;
+    };
+    // a slot of tile t's list for every lane with t >= 0, one atomic for the lanes of a tile (these are
+    // the tiles that many pairs share).  Every lane calls it.
+    auto claim = [&](int t) {
+      const unsigned peers = __match_any_sync(all, t);
+      const int leader = __ffs(peers) - 1;
+      int at = 0;
+      if (t >= 0 && lane == leader)
+        at = atomicAdd(tile_count + (int64_t)t * kCounterStride + kClaimWord, __popc(peers));
+      return __shfl_sync(all, at, leader) + __popc(peers & ((1u << lane) - 1u));
+    };
+    constexpr int kPairs = 2;
+    for (int e0 = 0; e0 < total; e0 += 32 * kPairs) {
+      int t[kPairs], l[kPairs], len[kPairs], at[kPairs];
+      long long lo[kPairs];
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u) {
+        const int e = e0 + 32 * u + lane;
+        l[u] = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if (__shfl_sync(all, excl, l[u] + step) <= e) l[u] += step;
+        t[u] = tile_of(l[u], (unsigned)(e - __shfl_sync(all, excl, l[u])), e < total, lo[u], len[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u) at[u] = claim(t[u]);
+#pragma unroll
+      for (int u = 0; u < kPairs; ++u)
+        if (t[u] >= 0 && at[u] < len[u]) gids[lo[u] + at[u]] = (int32_t)(b + l[u]);
+    }
+    for (unsigned huge = __ballot_sync(all, cnt > kHugeRect); huge; huge &= huge - 1) {
+      const int l = __ffs(huge) - 1, tiles = __shfl_sync(all, cnt, l);
+      for (int k0 = 0; k0 < tiles; k0 += 32) {
+        long long lo;
+        int len;
+        const int t = tile_of(l, (unsigned)(k0 + lane), k0 + lane < tiles, lo, len);
+        const int at = claim(t);
+        if (t >= 0 && at < len) gids[lo + at] = (int32_t)(b + l);
+      }
+    }
+  }
+}
+
+// Waits until `parts` shares are placed; false when they are not after about a second.  Every thread
+// calls it.
+constexpr int kPlacedPolls = 1 << 20;
+__device__ __forceinline__ bool wait_placed(const int* placed, int parts) {
+  bool ok = true;
+  if (threadIdx.x == 0) {
+    ok = false;
+    for (int k = 0; k < kPlacedPolls && !ok; ++k) {
+      int v;
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(placed) : "memory");
+      ok = v >= parts;
+      if (!ok) __nanosleep(200);
+    }
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
 // Tiles per CTA: with up to kWarpTilesMax Gaussians per tile on average most lists are short, and a
 // CTA takes four tiles, each warp sorting its own in registers (lists up to kWarpIds; bitonic, no
 // block-wide step), longer ones then by the whole CTA in turn; beyond that one tile, by the CTA.
@@ -914,37 +1107,86 @@ __device__ __noinline__ void cta_sort_bin(const Splat* __restrict__ rec, int64_t
 constexpr int kWarpIds = 256;
 constexpr int64_t kWarpTilesMax = 128;
 
+// Where some bin overflowed, the CTAs number themselves as they start.  The first `parts` place the
+// overflowing tiles' ids (place_overflow) and wait for nobody; the others take the tiles, and wait for
+// the first before they sort the placed lists, which they share out singly.  So every wait is for CTAs
+// that already run.  Count and fill of 100k Gaussians on 1024x1024: 41 px wide in 4-px tiles (lists of 180
+// beside bins of 96) 0.58 ms, 0.27 in the plain form; 97 px in 16-px tiles (1,130 beside 832) 0.32 and
+// 0.36; within 40 px of one point in 32-px tiles (10k beside 3,168) 0.14 and 0.17.  When all such tiles
+// were tested against every record they took 19.0, 1.09 and 0.45 ms.
+// Half the CTAs that the tiles need place pairs, between these numbers; only below twice the first does
+// the grid have CTAs for it that leave at once otherwise (222 of them beside 256 cost 0.7 us).
+constexpr int64_t kLeastParts = 74, kMostParts = 1184;
+
+struct BinSort {
+  const Splat* rec;
+  int64_t n;
+  int ts;
+  float cutoff2;
+  int64_t T;
+  int tiles_per_cta, parts, lanes, tests;
+  const long long* off64;
+  int* tile_count;
+  const int32_t* bins;
+  int K;
+  int32_t* gids;
+  int64_t cap;
+  uint32_t* status;
+};
+
+// Sorts the placed lists among tiles first, first + step, …; or lists those tiles from the records when
+// their ids did not come.  Every thread calls it.
 template <bool CULL>
-__global__ void __launch_bounds__(kSortThreads)
-    bin_sort_kernel(const Splat* __restrict__ rec, int64_t n, int ts, Frames frames,
-                    float cutoff2, int64_t T, int tiles_per_cta,
-                    const long long* __restrict__ off64, const int* __restrict__ tile_count,
-                    const int32_t* __restrict__ bins, int K, int32_t* __restrict__ gids,
-                    int64_t cap, uint32_t* status) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ __align__(16) uint32_t smem[kWindowWords];  // a bitmap, or ids and buckets
-  __shared__ int tmp[kSortWarps + 1];
-  const int64_t t0 = (int64_t)blockIdx.x * tiles_per_cta;
-  const bool trusted = tile_count[2] == K;  // the bins belong to these counts
-  if (t0 == 0 && threadIdx.x == 0) {
-    const long long total = off64[T];
-    if (total > 2147483647LL) raise_status(status, SS_STATUS_INDEX_INT32);
-    if (total > cap) raise_status(status, SS_STATUS_INDEX_OVERFLOW);
+__device__ __noinline__ void sort_placed_tiles(const BinSort& a, const Frames& frames,
+                                               const Overflow over, bool placed, int64_t first,
+                                               int64_t step, uint32_t* smem, int* tmp) {
+  __shared__ int todo[kSortThreads], num_todo;
+  for (int64_t base = first; base < a.T; base += step * kSortThreads) {
+    if (threadIdx.x == 0) num_todo = 0;
+    __syncthreads();
+    const int64_t mine = base + step * threadIdx.x;
+    if (mine < a.T) {
+      const long long hi = a.off64[mine + 1], len = hi - a.off64[mine];
+      if (hi <= a.cap && len > 0 && over.beyond(len) &&
+          !over.records(len, frame_of_tile(frames, (int)mine, a.n).gauss_count))
+        todo[atomicAdd(&num_todo, 1)] = (int)mine;
+    }
+    __syncthreads();
+    const int count = num_todo;
+    for (int k = 0; k < count; ++k) {
+      const int t = todo[k];
+      const long long lo = a.off64[t];
+      const int len = (int)(a.off64[t + 1] - lo);
+      const Frame fr = frame_of_tile(frames, t, a.n);
+      if (placed)
+        sort_placed(a.gids + lo, len, fr.gauss_first, fr.gauss_count, smem, tmp);
+      else
+        cta_sort_bin<CULL>(a.rec, a.n, a.ts, frames, a.cutoff2, t, lo, len, true, a.bins, a.gids,
+                           smem, tmp);
+      if (threadIdx.x == 0)
+        a.tile_count[(int64_t)t * kCounterStride + kClaimWord] = 0;  // for another fill
+      __syncthreads();
+    }
   }
-  bool mine = true;  // the CTA path takes the tile
-  if (tiles_per_cta > 1) {
+}
+
+// Sorts the tiles_per_cta tiles from t0 on, but for those that place_overflow lists (`some` of them).
+template <bool CULL>
+__device__ __forceinline__ void sort_tiles(const BinSort& a, const Frames& frames, int64_t t0,
+                                           const Overflow& over, bool some, uint32_t* smem,
+                                           int* tmp) {
+  if (a.tiles_per_cta > 1) {
     const int lane = threadIdx.x & 31;
     const int64_t t = t0 + (threadIdx.x >> 5);
-    mine = false;
-    if (t < T) {
-      const long long lo = off64[t], hi = off64[t + 1];
+    bool mine = false;  // the CTA takes the tile
+    if (t < a.T) {
+      const long long lo = __ldg(a.off64 + t), hi = __ldg(a.off64 + t + 1);
       const int len = (int)(hi - lo);
-      if (hi <= cap && len > 0) {  // else truncated: the renderers scan all Gaussians
-        mine = len > kWarpIds || len > K || !trusted;
+      if (hi <= a.cap && len > 0) {  // else truncated: the renderers scan all Gaussians
+        mine = len > kWarpIds || over.beyond(len);
         if (!mine) {
-          const int32_t* bin = bins + t * K;
-          int32_t* g = gids + lo;
+          const int32_t* bin = a.bins + t * a.K;
+          int32_t* g = a.gids + lo;
           if (len <= 32)
             warp_sort_list<1>(bin, g, len, lane);
           else if (len <= 64)
@@ -958,18 +1200,71 @@ __global__ void __launch_bounds__(kSortThreads)
     }
     if (!__syncthreads_or(mine)) return;
   }
-  for (int u = 0; u < tiles_per_cta; ++u) {
+  for (int u = 0; u < a.tiles_per_cta; ++u) {
     const int64_t t = t0 + u;
-    if (t >= T) break;
-    const long long lo = off64[t], hi = off64[t + 1];
+    if (t >= a.T) break;
+    const long long lo = __ldg(a.off64 + t), hi = __ldg(a.off64 + t + 1);
     const int len = (int)(hi - lo);  // at most the image's Gaussians
-    if (hi > cap || len == 0) continue;
-    const bool rebuild = len > K || !trusted;
-    if (tiles_per_cta > 1 && len <= kWarpIds && !rebuild) continue;  // a warp has sorted it
-    cta_sort_bin<CULL>(rec, n, ts, frames, cutoff2, (int)t, lo, len, rebuild, bins + t * K, gids,
-                       smem, tmp);
+    if (hi > a.cap || len == 0) continue;
+    const bool beyond = over.beyond(len);
+    if (a.tiles_per_cta > 1 && len <= kWarpIds && !beyond) continue;  // a warp has sorted it
+    if (some && beyond && !over.records(len, frame_of_tile(frames, (int)t, a.n).gauss_count)) continue;
+    cta_sort_bin<CULL>(a.rec, a.n, a.ts, frames, a.cutoff2, (int)t, lo, len, beyond,
+                       a.bins + t * a.K, a.gids, smem, tmp);
     __syncthreads();
   }
+}
+
+// The kernel where some tile's ids are to be placed.
+template <bool CULL>
+__device__ __noinline__ void sort_and_place(const BinSort& a, const Frames& frames, bool trusted,
+                                            uint32_t* smem, int* tmp) {
+  const Overflow over{a.K, a.tests, trusted};
+  if (threadIdx.x == 0) tmp[0] = atomicAdd(a.tile_count + kTicketWord, 1);
+  __syncthreads();
+  const int number = tmp[0] - a.parts, tile_ctas = (int)gridDim.x - a.parts;
+  __syncthreads();
+  if (number < 0) {
+    place_overflow<CULL>(a.rec, a.n, a.ts, frames, a.cutoff2, a.off64, a.tile_count, over, a.gids,
+                         a.cap, number + a.parts, a.parts, a.lanes);
+    __threadfence();  // the ids before the word that tells of them
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(a.tile_count + kPlacedWord, 1);
+  } else {
+    for (int64_t t0 = (int64_t)number * a.tiles_per_cta; t0 < a.T;
+         t0 += (int64_t)tile_ctas * a.tiles_per_cta)
+      sort_tiles<CULL>(a, frames, t0, over, true, smem, tmp);
+    const bool placed = wait_placed(a.tile_count + kPlacedWord, a.parts);
+    if (!placed && threadIdx.x == 0)
+      raise_status(a.status, SS_STATUS_INDEX_OVERFLOW);  // late ids may spoil a list
+    sort_placed_tiles<CULL>(a, frames, over, placed, number, tile_ctas, smem, tmp);
+  }
+  __syncthreads();
+  // the last CTA leaves the tickets as they were, for another fill of these counts
+  if (threadIdx.x == 0 && atomicAdd(a.tile_count + kExitWord, 1) == (int)gridDim.x - 1)
+    a.tile_count[kTicketWord] = a.tile_count[kPlacedWord] = a.tile_count[kExitWord] = 0;
+}
+
+template <bool CULL>
+__global__ void __launch_bounds__(kSortThreads, 7)
+    bin_sort_kernel(__grid_constant__ const BinSort a, __grid_constant__ const Frames frames) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ __align__(16) uint32_t smem[kWindowWords];  // a bitmap, or ids and buckets
+  __shared__ int tmp[kSortWarps + 1];
+  const bool trusted = a.tile_count[kBinsWord] == a.K;  // the bins belong to these counts
+  const bool place = a.parts > 0 && (!trusted || a.tile_count[kOverflowWord] != 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const long long total = a.off64[a.T];
+    if (total > 2147483647LL) raise_status(a.status, SS_STATUS_INDEX_INT32);
+    if (total > a.cap) raise_status(a.status, SS_STATUS_INDEX_OVERFLOW);
+  }
+  if (place) {
+    sort_and_place<CULL>(a, frames, trusted, smem, tmp);
+    return;
+  }
+  const int64_t t0 = (int64_t)blockIdx.x * a.tiles_per_cta;
+  if (t0 < a.T) sort_tiles<CULL>(a, frames, t0, Overflow{a.K, 0, trusted}, false, smem, tmp);
 }
 
 // Bits that hold every id below n and the pad 2^bits - 1 above them.
@@ -1083,7 +1378,7 @@ int index_count(const Frames& frames, int ts, int64_t T, const void* records, in
   if (one_scan) {
     launch("scan_counts_kernel", scan_counts_kernel,
            (unsigned)((T + kScanThreads) / kScanThreads), kScanThreads, 0, s, w.tile_count, T + 1,
-           w.offsets64, tile_offsets);
+           w.offsets64, tile_offsets, frames, n, w.bin_ids, index_tests(n, T));
     return check_launch("tile_offsets scan");
   }
   size_t sb = w.scan_bytes;
@@ -1095,7 +1390,7 @@ int index_count(const Frames& frames, int ts, int64_t T, const void* records, in
   // int32 offsets for callers that only run stage 1 (the fill rewrites them identically).
   launch("tile_fill_kernel", tile_fill_kernel<false>, (int)((T + 1 + kThreads - 1) / kThreads), kThreads, 0, s, 
       rec, 0, ts, frames, cutoff2, T, w.offsets64, w.tile_count, tile_offsets, nullptr,
-      INT64_MAX, w.big_count, nullptr);
+      INT64_MAX, w.big_count, nullptr, w.bin_ids, index_tests(n, T), n);
   return check_launch("tile_offsets");
 }
 
@@ -1117,10 +1412,20 @@ int index_fill(const Frames& frames, int ts, int64_t T, const void* records, int
   float cutoff2 = sigma_cutoff * sigma_cutoff;
   if (w.bins) {  // the count left every tile's ids in its bin
     const int per = n <= kWarpTilesMax * T ? kSortWarps : 1;
+    const int64_t ctas = (T + per - 1) / per;
+    const int tests = index_tests(n, T);
+    int64_t parts = ctas / 2 < kMostParts ? ctas / 2 : kMostParts;
+    if (parts < kLeastParts) parts = kLeastParts;
+    const int lanes = n >= parts * kSortThreads ? 32 : 8;  // a warp's Gaussians at a time
+    const int64_t share = (n + lanes * kSortWarps - 1) / (lanes * kSortWarps);
+    if (share < parts) parts = share;
+    if (tests == INT_MAX) parts = 0;  // all from the records: nothing is placed
+    const int64_t least = parts ? parts + (ctas < kLeastParts ? ctas : kLeastParts) : 0;
+    const BinSort a{rec, n, ts, cutoff2, T, per, (int)parts, lanes, tests, w.offsets64,
+                    w.tile_count, w.bins, w.bin_ids, tile_gids, gid_capacity, status};
 #define SS_BIN(C)                                                                             \
-  launch("bin_sort_kernel", bin_sort_kernel<C>, (unsigned)((T + per - 1) / per), kSortThreads,  \
-         0, s, rec, n, ts, frames, cutoff2, T, per, w.offsets64, w.tile_count, w.bins,          \
-         w.bin_ids, tile_gids, gid_capacity, status)
+  launch("bin_sort_kernel", bin_sort_kernel<C>, (unsigned)(ctas > least ? ctas : least),        \
+         kSortThreads, 0, s, a, frames)
     if (ellipse_cull) SS_BIN(true); else SS_BIN(false);
 #undef SS_BIN
     return check_launch("bin_sort");
@@ -1132,12 +1437,12 @@ int index_fill(const Frames& frames, int ts, int64_t T, const void* records, int
     launch("tile_fill_kernel", tile_fill_kernel<true>, blocks, kThreads, 0, s, rec, n, ts, frames, cutoff2, T,
                                                        w.offsets64, w.tile_count, offsets32,
                                                        tile_gids, gid_capacity, w.big_count,
-                                                       status);
+                                                       status, 0, 0, n);
   else
     launch("tile_fill_kernel", tile_fill_kernel<false>, blocks, kThreads, 0, s, rec, n, ts, frames, cutoff2, T,
                                                         w.offsets64, w.tile_count, offsets32,
                                                         tile_gids, gid_capacity, w.big_count,
-                                                        status);
+                                                        status, 0, 0, n);
   if ((rc = check_launch("tile_fill"))) return rc;
   int sort_blocks = (int)((T + (kThreads / 32) - 1) / (kThreads / 32));
   launch("tile_sort_kernel", tile_sort_kernel, sort_blocks, kThreads, 0, s, tile_offsets, tile_gids, gid_capacity, T,
@@ -1172,6 +1477,18 @@ int ss_tile_index_binned_workspace_bytes(int64_t n, int height, int width, int t
   if (rc) return rc;
   if (!bytes) return fail(SS_ERR_INVALID_ARGUMENT, "null bytes pointer");
   *bytes = binned_workspace_bytes(n, make_grid(height, width, tile_size).T);
+  return SS_OK;
+}
+
+int ss_tile_index_entries_workspace_bytes(int64_t n, int64_t tiles, int images, int64_t entries,
+                                          size_t* bytes) {
+  if (n < 0 || tiles < 0 || images < 0 || entries < 0)
+    return fail(SS_ERR_INVALID_ARGUMENT, "negative size");
+  if (!bytes) return fail(SS_ERR_INVALID_ARGUMENT, "null bytes pointer");
+  const int64_t slots = tiles * bin_ids_for(n, tiles);
+  const bool full = tiles > 0 && entries > slots / 2 && index_tests(n, tiles) != INT_MAX &&
+                    !listed_from_records(entries / tiles, n / (images > 0 ? images : 1), 8);
+  *bytes = full ? index_workspace_bytes(tiles) : binned_workspace_bytes(n, tiles);
   return SS_OK;
 }
 

@@ -60,9 +60,7 @@ class RenderPlan:
         f32 = dict(device=d, dtype=torch.float32)
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, **f32)
         self.offsets = torch.zeros(self.T + 1, device=d, dtype=torch.int32)
-        self.idx_ws_bytes = _native.size_query("ss_tile_index_binned_workspace_bytes", n, self.H, self.W,
-                                               self.tile_size)
-        self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=d, dtype=torch.uint8)
+        self._size_index(0)
         if self.capacity <= 0:
             self.capacity = 1
         self.gids = torch.empty(self.capacity, device=d, dtype=torch.int32)
@@ -95,8 +93,16 @@ class RenderPlan:
         plan.project(params)
         plan.count()
         total = int(plan.offsets[-1].item())
-        return cls(n=n, H=H, W=W, capacity=int(total * headroom) + 4096,
-                   has_opacity=plan.has_opacity, device=plan.device, **kw)
+        sized = cls(n=n, H=H, W=W, capacity=int(total * headroom) + 4096,
+                    has_opacity=plan.has_opacity, device=plan.device, **kw)
+        sized._size_index(total)
+        return sized
+
+    def _size_index(self, entries: int):
+        """The index workspace for about ``entries`` tile-list entries (0: not known)."""
+        self.idx_ws_bytes = _native.size_query("ss_tile_index_entries_workspace_bytes", self.n,
+                                               self.T, 1, entries)
+        self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=self.device, dtype=torch.uint8)
 
     # -- stages --------------------------------------------------------------------------
     def project(self, params):

@@ -150,6 +150,11 @@ class _CapacityCache:
     def __init__(self):
         self.entries = {}
 
+    def entries_of(self, key) -> int:
+        """About the entries of the key's calls so far, 0 before the first."""
+        ent = self.entries.get(key)
+        return 0 if ent is None else (ent["cap"] - 1024) * 4 // 5
+
     def capacity(self, key, offsets) -> int:
         ent = self.entries.get(key)
         if ent is None:
@@ -169,6 +174,11 @@ class _CapacityCache:
 
 
 CAPACITY = _CapacityCache()
+
+
+def index_workspace_bytes(n: int, T: int, entries: int) -> int:
+    """Bytes of one image's index workspace for about ``entries`` entries (0: not known)."""
+    return _native.size_query("ss_tile_index_entries_workspace_bytes", n, T, 1, entries)
 
 
 class EagerPlan:
@@ -197,9 +207,7 @@ class EagerPlan:
         d = device
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, device=d, dtype=torch.float32)
         self.offsets = torch.zeros(self.T + 1, device=d, dtype=torch.int32)
-        self.idx_ws_bytes = _native.size_query("ss_tile_index_binned_workspace_bytes", n, H, W,
-                                               tile_size)
-        self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=d, dtype=torch.uint8)
+        self._size_index(0)
         self.capacity = 0
         self.gids = None
         self.generation = 0
@@ -208,6 +216,12 @@ class EagerPlan:
         self.status_event = torch.cuda.Event()  # re-recorded by every call
         self.event = None
         self._size_list(1)
+
+    def _size_index(self, entries: int):
+        self.idx_ws_bytes = index_workspace_bytes(self.n, self.T, entries)
+        self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=self.records.device,
+                                  dtype=torch.uint8)
+        self.entries = 0  # of a call whose index outgrew the workspace's form, for the next one
 
     def _size_list(self, capacity: int):
         self.capacity = int(capacity)
@@ -229,11 +243,15 @@ class EagerPlan:
             self.event = None
         if grow:
             total = int(self.offsets[-1].item())
+            self.entries = total
             if total > self.capacity or self.capacity <= 1:
                 self._size_list(int(total * self.HEADROOM) + 4096)
                 self.step_block.zero_()
 
     def note_status(self):
+        if self.entries and index_workspace_bytes(self.n, self.T, self.entries) != self.idx_ws_bytes:
+            self._size_index(self.entries)  # this call's index is made: the next one's workspace
+        self.entries = 0
         self.host_status.copy_(self.status, non_blocking=True)
         self.status_event.record()
         self.event = self.status_event
@@ -263,13 +281,18 @@ def _index(n: int, H: int, W: int, tile_size: int, ellipse_cull: bool, sigma_cut
            capacity, exact: bool, dev, records, pack=None) -> TileIndex:
     tiles_x, tiles_y = tile_grid(H, W, tile_size)
     T = tiles_x * tiles_y
+    key = (dev.index, n, H, W, tile_size, bool(ellipse_cull))
+    known = 0 if exact else CAPACITY.entries_of(key)
     offsets = torch.empty(T + 1, device=dev, dtype=torch.int32)
-    ws_bytes = _native.size_query("ss_tile_index_binned_workspace_bytes", n, H, W, tile_size)
+    ws_bytes = index_workspace_bytes(n, T, known)
     ws = torch.empty(max(ws_bytes, 1), device=dev, dtype=torch.uint8)
-    if pack is None:
-        status = torch.zeros(1, device=dev, dtype=torch.int32)
+
+    def count():
         _native.call("ss_tile_index_count", _p(records), n, H, W, tile_size, int(ellipse_cull),
                      float(sigma_cutoff), _p(offsets), _p(ws), ws_bytes, _p(status), _stream())
+    if pack is None:
+        status = torch.zeros(1, device=dev, dtype=torch.int32)
+        count()
     else:
         word = torch.empty(4, device=dev, dtype=torch.int32)  # cleared by the call, 16 bytes
         status = word[:1]
@@ -278,11 +301,15 @@ def _index(n: int, H: int, W: int, tile_size: int, ellipse_cull: bool, sigma_cut
                      ws_bytes, _p(word), 16, _p(status), _stream())
     if T == 0:
         capacity = 0
-    elif exact:
-        capacity = int(offsets[-1].item())
-    elif capacity is None:
-        key = (dev.index, n, H, W, tile_size, bool(ellipse_cull))
-        capacity = CAPACITY.capacity(key, offsets)
+    elif exact or capacity is None:
+        if exact:
+            known = capacity = int(offsets[-1].item())
+        else:
+            capacity = CAPACITY.capacity(key, offsets)
+            known = 0 if known else CAPACITY.entries_of(key)  # a first call has read the total
+        if known and index_workspace_bytes(n, T, known) < ws_bytes:
+            ws_bytes = index_workspace_bytes(n, T, known)  # the plain form: count again without bins
+            count()
     gids = torch.empty(max(capacity, 1), device=dev, dtype=torch.int32)
     _native.call("ss_tile_index_fill", _p(records), n, H, W, tile_size, int(ellipse_cull),
                  float(sigma_cutoff), _p(offsets), _p(gids), int(capacity), _p(ws), ws_bytes,
