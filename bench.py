@@ -588,6 +588,7 @@ def run_batched(args, dev, workload):
     tuned = None
     if not args.no_tune:
         from structsplat_b200 import autotune
+        shapes = autotune.asked_shapes()  # the other legs take the library's own
         fp = fresh()
         tuned = autotune.tune_fit(sizes, counts, Batch.concat_fields(fp),
                                   Batch(sizes, counts, device=dev).concat_images(targets),
@@ -649,6 +650,8 @@ def run_batched(args, dev, workload):
         t_loop_first = timed(loop_step, Kg)
         t_loop_graph *= t_loop / t_loop_first
     del graphs, plans, start
+    if tuned is not None:
+        autotune.ask_shapes(shapes)
 
     # ranks fit disjoint shares of the images: the job is as slow as its slowest rank
     from structsplat_b200.replicas import max_over_ranks, sum_over_ranks

@@ -218,17 +218,22 @@ int ss_render_forward(const void* records, int64_t n, const int32_t* tile_gids,
                       float* den, uint32_t* status, ss_stream_t stream);
 
 /* Launch tuning (process-wide, used by the autotuner): warps per backward CTA for a render
- * tile size — 4 or 8 for tile 16, 8 or 16 for tile 32, 0 restores the default (8 for both).
- * Results do not depend on it.  ss_get_backward_warps returns the value in effect (-1 for an
- * unsupported tile size). */
+ * tile size — 4 or 8 for tile 16, 8 or 16 for tile 32; 0 leaves it to each launch (8 at 16 px; at
+ * 32 px 16 for few tiles or many Gaussians per tile, else 8).  Results do not depend on it.
+ * ss_asked_backward_warps returns the value set, 0 where none is; ss_get_backward_warps the same
+ * with 8 where none is.  Both give -1 for an unsupported tile size. */
 int ss_set_backward_warps(int tile_size, int warps);
+int ss_asked_backward_warps(int tile_size);
 int ss_get_backward_warps(int tile_size);
 
 /* Launch tuning (process-wide): records per streamed chunk of the forward for a render tile
- * size — 64, 128 or 256, 0 restores the default (256).  Only tile lists longer than the
- * forward's stage (512 records, 768 for sets of long lists, 256 at 16 px) stream; images do not depend on it.  ss_get_forward_chunk returns
- * the value in effect (-1 for an unsupported tile size). */
+ * size — 64, 128 or 256, 0 restores the default (256); at most half the stage, so 256 means 128
+ * at 16 px.  Only tile lists longer than the forward's stage (512 records, 768 for sets of long
+ * lists, 256 at 16 px) stream; images do not depend on it.  ss_asked_forward_chunk returns the value
+ * set, 0 where none is; ss_get_forward_chunk the same with 256 where none is.  Both give -1 for an
+ * unsupported tile size. */
 int ss_set_forward_chunk(int tile_size, int records);
+int ss_asked_forward_chunk(int tile_size);
 int ss_get_forward_chunk(int tile_size);
 
 /* `deterministic` of every backward, fit and finalize call: 0 adds with atomics; 1 to 3 are bitwise

@@ -73,8 +73,10 @@ SIGNATURES = {
     "ss_set_backward_warps": [_int, _int],
     "ss_set_dependent_launch": [_int],
     "ss_get_dependent_launch": [],
+    "ss_asked_backward_warps": [_int],
     "ss_get_backward_warps": [_int],
     "ss_set_forward_chunk": [_int, _int],
+    "ss_asked_forward_chunk": [_int],
     "ss_get_forward_chunk": [_int],
     "ss_render_backward_workspace_bytes": [_i64, _i64, _int, _int, _int, _szp],
     "ss_render_backward": [_vp, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _int, _int, _int, _int,

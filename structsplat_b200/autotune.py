@@ -52,6 +52,20 @@ class TuneResult:
         return self
 
 
+def asked_shapes() -> dict:
+    """The shapes asked of the library so far, 0 where it chooses by itself: {tile size: (backward
+    warps, forward chunk)}."""
+    lib = _native.lib()
+    return {ts: (lib.ss_asked_backward_warps(ts), lib.ss_asked_forward_chunk(ts)) for ts in (16, 32)}
+
+
+def ask_shapes(shapes: dict):
+    """Ask for the shapes of an earlier ``asked_shapes``."""
+    for ts, (warps, chunk) in shapes.items():
+        _native.call("ss_set_backward_warps", ts, warps)
+        _native.call("ss_set_forward_chunk", ts, chunk)
+
+
 def cache_path() -> Path:
     env = os.environ.get("STRUCTSPLAT_B200_TUNE_CACHE")
     return Path(env) if env else Path.home() / ".cache" / "structsplat_b200" / "tune.json"
@@ -119,8 +133,7 @@ def _pick(key, candidates, build, repeats, use_cache, longest=None) -> TuneResul
         if hit and (hit["tile_size"], hit["backward_warps"]) in set(candidates):
             return TuneResult(hit["tile_size"], hit["backward_warps"], key, hit["times_ms"],
                               cached=True, forward_chunk=hit.get("forward_chunk", 0)).apply()
-    before = {ts: (_native.lib().ss_get_backward_warps(ts),
-                   _native.lib().ss_get_forward_chunk(ts)) for ts in (16, 32)}
+    before = asked_shapes()
     times = {}
     chunk = 0
     try:
@@ -138,9 +151,7 @@ def _pick(key, candidates, build, repeats, use_cache, longest=None) -> TuneResul
                 times[f"{ts}x{warps}/chunk{c}"] = chunk_times[c]
             chunk = min(chunk_times, key=chunk_times.get)
     finally:
-        for t, (w, c) in before.items():
-            _native.call("ss_set_backward_warps", t, w)
-            _native.call("ss_set_forward_chunk", t, c)
+        ask_shapes(before)
     result = TuneResult(ts, warps, key, times, forward_chunk=chunk).apply()
     if use_cache:
         _store(key, result)

@@ -418,8 +418,21 @@ def fit_batch(fields, targets, iters: int = 100, settings: FitSettings | None = 
     outgrew its capacity the plan is rebuilt with more room (in deterministic mode the steps
     since the last check are replayed from a snapshot, so the result never depends on it).
     ``tune=True`` lets the autotuner pick the tile size and backward warps for this workload
-    (``autotune.tune_fit``) instead of ``tile_size``.
+    (``autotune.tune_fit``) instead of ``tile_size``; the library's shapes are as before afterwards.
     """
+    if tune:
+        from .autotune import ask_shapes, asked_shapes
+        before = asked_shapes()
+        try:
+            return _fit_batch(fields, targets, iters, settings, graph, log_every, check_every,
+                              tile_size, True)
+        finally:
+            ask_shapes(before)
+    return _fit_batch(fields, targets, iters, settings, graph, log_every, check_every, tile_size,
+                      False)
+
+
+def _fit_batch(fields, targets, iters, settings, graph, log_every, check_every, tile_size, tune):
     settings = settings or FitSettings()
     sizes = [(int(t.shape[0]), int(t.shape[1])) for t in targets]
     counts = [int(f["means"].shape[0]) for f in fields]

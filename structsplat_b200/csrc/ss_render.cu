@@ -1992,9 +1992,13 @@ int ss_set_backward_warps(int tile_size, int warps) {
   return SS_OK;
 }
 
-int ss_get_backward_warps(int tile_size) {
+int ss_asked_backward_warps(int tile_size) {
   if (tile_size != 16 && tile_size != 32) return -1;
-  const int w = g_backward_warps[tile_size == 16 ? 0 : 1].load(std::memory_order_relaxed);
+  return g_backward_warps[tile_size == 16 ? 0 : 1].load(std::memory_order_relaxed);
+}
+
+int ss_get_backward_warps(int tile_size) {
+  const int w = ss_asked_backward_warps(tile_size);
   return w ? w : 8;
 }
 
@@ -2008,9 +2012,13 @@ int ss_set_forward_chunk(int tile_size, int records) {
   return SS_OK;
 }
 
-int ss_get_forward_chunk(int tile_size) {
+int ss_asked_forward_chunk(int tile_size) {
   if (tile_size != 16 && tile_size != 32) return -1;
-  const int c = g_forward_chunk[tile_size == 16 ? 0 : 1].load(std::memory_order_relaxed);
+  return g_forward_chunk[tile_size == 16 ? 0 : 1].load(std::memory_order_relaxed);
+}
+
+int ss_get_forward_chunk(int tile_size) {
+  const int c = ss_asked_forward_chunk(tile_size);
   return c ? c : kForwardChunk;
 }
 
