@@ -7,9 +7,9 @@ workload picks, by timing on the GPU it runs on, among
   list up to 512 or 768 Gaussians for the forward and 448 or 1,152 for the backward, by its warps
   and the Gaussians per tile, a 16x16 tile up to 256 and 512; longer lists stream), and
 * warps per backward CTA (4 or 8 for tile 16, 8 or 16 for tile 32), and
-* when the workload's longest tile list is longer than 512 records (the forward then streams it
-  through two chunks, but for sets of long lists, which it stages up to 768), the forward's chunk
-  depth: 64, 128 or 256 records, timed at the chosen shape.
+* when the workload's longest tile list is longer than the forward's stage at the chosen tile (512
+  records, 256 at 16 px; it then streams through two chunks, but for 32-px sets of long lists, which
+  are staged up to 768), the forward's chunk depth: 64, 128 or 256 records, timed at the chosen shape.
 
 The forward's threads follow the tile (one warp per 8x8 block).  Timing runs the render forward
 and backward of the actual workload (the field and images in hand), median of a few CUDA-event
@@ -32,8 +32,10 @@ import torch
 from . import _native
 
 CANDIDATES = ((16, 4), (16, 8), (32, 8), (32, 16))
-CHUNKS = (64, 128, 256)  # forward records per streamed chunk
+CHUNKS = (64, 128, 256)  # forward records per streamed chunk (at most half the stage)
 STAGE_RECORDS = 512      # the forward's whole-list stage at 32 px
+STAGES = {16: 256, 32: STAGE_RECORDS}
+KERNELS = 2              # of the cache's keys: raised when the tile kernels' shapes change
 
 
 @dataclass
@@ -105,7 +107,7 @@ def workload_key(pixels: int, gaussians: int, entries: int, images: int, normali
     parts = [dev, f"px={_bucket(pixels)}", f"g/px={_bucket(gaussians / max(pixels, 1))}",
              f"e/g={_bucket(entries / max(gaussians, 1))}", f"img={_bucket(images)}",
              f"norm={int(normalize)}", f"fade={int(fade)}", f"det={int(deterministic)}",
-             f"fit={int(fit)}"]
+             f"fit={int(fit)}", f"k={KERNELS}"]
     if fused:
         parts.append("fused=1")
     return "|".join(parts)
@@ -142,10 +144,10 @@ def _pick(key, candidates, build, repeats, use_cache, longest=None) -> TuneResul
             times[f"{ts}x{warps}"] = round(_time(build(ts), repeats), 4)
         best = min(times, key=times.get)
         ts, warps = (int(v) for v in best.split("x"))
-        if longest is not None and longest(ts) > STAGE_RECORDS:
+        if longest is not None and longest(ts) > STAGES[ts]:
             _native.call("ss_set_backward_warps", ts, warps)
             chunk_times = {}
-            for c in CHUNKS:
+            for c in (c for c in CHUNKS if 2 * c <= STAGES[ts]):
                 _native.call("ss_set_forward_chunk", ts, c)
                 chunk_times[c] = round(_time(build(ts), repeats), 4)
                 times[f"{ts}x{warps}/chunk{c}"] = chunk_times[c]
@@ -203,11 +205,11 @@ def tune_fit(sizes, counts, params: dict, target: torch.Tensor, settings=None,
         plan = plans[ts]
 
         def run():
-            if plan.s.use_fused():
-                plan.forward_backward()
+            if plan.s.use_fused():  # as FitPlan.step runs them
+                plan.forward_backward(plan.det)
             else:
                 plan.forward_loss()
-                plan.backward()
+                plan.backward(plan.det)
         return run
 
     try:

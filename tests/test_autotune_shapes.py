@@ -64,3 +64,19 @@ def test_a_tuned_fit_leaves_the_shapes(monkeypatch):
     monkeypatch.setattr(batch, "_fit_batch", fit)
     assert batch.fit_batch([], [], tune=True)["tuned"]
     assert autotune.asked_shapes() == UNSET
+
+
+@pytest.mark.parametrize("tile,longest,chunks", [(16, 256, []), (16, 257, [64, 128]), (32, 512, []),
+                                                 (32, 513, [64, 128, 256])])
+def test_chunks_are_timed_from_the_tiles_own_stage_on(monkeypatch, tile, longest, chunks):
+    times = (1.0, 2.0, 3.0, 4.0) if tile == 16 else (4.0, 3.0, 1.0, 2.0)
+    r = _pick(monkeypatch, times + tuple(range(1, 1 + len(chunks))), longest=lambda ts: longest)
+    assert r.tile_size == tile
+    assert [k for k in r.times_ms if "/chunk" in k] == [
+        f"{tile}x{r.backward_warps}/chunk{c}" for c in chunks]
+    assert r.forward_chunk == (chunks[0] if chunks else 0)
+
+
+def test_cached_shapes_of_other_kernels_are_not_taken():
+    key = autotune.workload_key(1, 1, 1, 1, True, False, False, fit=True)
+    assert f"k={autotune.KERNELS}" in key.split("|")
