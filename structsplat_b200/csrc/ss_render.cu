@@ -1311,8 +1311,20 @@ __global__ void finalize_rs_kernel(const Splat* __restrict__ rec, int64_t n,
   if (logits && g_logits) g_logits[g] = logit_chain(logits[g], m[3]);
 }
 
+// Tiles of [0, T) before the first whose list does not fit the capacity: those that a deterministic
+// backward evaluates (it leaves out the rest, whose entries have neither ids nor partials).
+__device__ __forceinline__ int64_t tiles_that_fit(const int32_t* offsets, int64_t T, int64_t cap) {
+  if (offsets[T] <= cap) return T;
+  int64_t lo = 0;
+  for (int64_t hi = T; lo < hi;) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (offsets[mid + 1] <= cap) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
 // Deterministic mode, after the backward: the entries of the tile lists ordered by Gaussian.
-// Keys are the entry ids (n for slots past the filled part of the index); a stable radix sort
+// Keys are the entry ids (n for slots past the evaluated part of the index); a stable radix sort
 // keeps each Gaussian's entries in ascending tile order; the segment kernel records where each
 // Gaussian's run begins and ends (Gaussians without entries keep the empty run 0..0).
 __global__ void entry_keys_kernel(const int32_t* __restrict__ gids,
@@ -1323,8 +1335,7 @@ __global__ void entry_keys_kernel(const int32_t* __restrict__ gids,
   pdl_trigger();
   // the entries of tiles [0, T): positions [offsets[0], offsets[T]) of the list (offsets[0] > 0
   // for a window of an image's tile rows)
-  const int64_t first = offsets[0], last = offsets[T];
-  const int64_t total = last < cap ? last : cap;
+  const int64_t first = offsets[0], total = offsets[tiles_that_fit(offsets, T, cap)];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cap; e += stride) {
     const int32_t id = e >= first && e < total ? gids[e] : -1;
