@@ -239,10 +239,13 @@ int ss_get_forward_chunk(int tile_size);
 /* `deterministic` of every backward, fit and finalize call: 0 adds with atomics; 1 to 3 are bitwise
  * reproducible and give the same gradients.  1 takes any tile index and orders its entries by
  * Gaussian with a sort.  SS_DETERMINISTIC_SLOTS needs an index of whole images built without the
- * ellipse cull (each Gaussian listed in every tile of its rectangle) and no sort; with an index that
- * overflowed its capacity its gradients are zero.  SS_DETERMINISTIC_RUNS
- * needs an index that this library built from these records, culled or not, and no sort.  One value
- * for all calls on one workspace. */
+ * ellipse cull (each Gaussian listed in every tile of its rectangle) and no sort.
+ * SS_DETERMINISTIC_RUNS needs an index that this library built from these records, culled or not, and
+ * no sort.  One value for all calls on one workspace.
+ * An index that overflowed its capacity raises SS_STATUS_DETERMINISTIC_TRUNCATED.  Modes 1 and 3 then
+ * sum the tiles whose lists fit, and so do slots in the fit calls (ss_fit_*, and a backward that is
+ * given pixel_grad), which go on stepping until the status is looked at; in the render calls slots
+ * give zero gradients. */
 #define SS_DETERMINISTIC_SLOTS 2
 #define SS_DETERMINISTIC_RUNS 3
 /* Workspace of ss_render_backward: per-Gaussian moment accumulators (36 B per Gaussian) or,

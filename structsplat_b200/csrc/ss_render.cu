@@ -1360,13 +1360,15 @@ __global__ void entry_segments_kernel(const uint32_t* __restrict__ keys, int64_t
 // Slot mode, before the backward: each Gaussian's partials get consecutive slots, one per tile of
 // its rectangle (its entries, in an index built without the ellipse cull).  A CTA reserves its
 // Gaussians' slots with one atomic; where they land varies from run to run, the order of a
-// Gaussian's partials does not.  An index that overflowed its capacity leaves no slots (the
-// gradients are zero and the backward raises SS_STATUS_DETERMINISTIC_TRUNCATED).  One pass over the
+// Gaussian's partials does not.  In an index that overflowed its capacity the backward leaves out the
+// tiles from the first truncated one on (and raises SS_STATUS_DETERMINISTIC_TRUNCATED): with `rest` a
+// Gaussian gets slots for its tiles before that one, which come first in its rectangle, and without
+// it none (its gradients are zero).  One pass over the
 // rectangles in place of keys, a radix sort of the whole capacity and segments, nine launches: 9
 // us against 150 us for 250k Gaussians with 2 M entries.
 __global__ void __launch_bounds__(kEpilogueThreads)
-    entry_slots_kernel(const Splat* __restrict__ rec, int64_t n, int ts,
-                       const int32_t* __restrict__ offsets, int64_t T, int64_t cap,
+    entry_slots_kernel(const Splat* __restrict__ rec, int64_t n, int ts, Frames frames,
+                       const int32_t* __restrict__ offsets, int64_t T, int64_t cap, bool rest,
                        unsigned* __restrict__ cursor, int32_t* __restrict__ seg) {
   pdl_wait();
   pdl_trigger();
@@ -1376,10 +1378,23 @@ __global__ void __launch_bounds__(kEpilogueThreads)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool room = offsets[T] <= cap;
   int cnt = 0;
-  if (g < n && room) {
+  if (g < n && (room || rest)) {
     const int4 r = reinterpret_cast<const int4*>(rec + g)[3];
-    if (r.z > r.x && r.w > r.y)
-      cnt = ((r.z - 1) / ts - r.x / ts + 1) * ((r.w - 1) / ts - r.y / ts + 1);
+    if (r.z > r.x && r.w > r.y) {
+      const int gx0 = r.x / ts, gy0 = r.y / ts;
+      const int gw = (r.z - 1) / ts - gx0 + 1, gh = (r.w - 1) / ts - gy0 + 1;
+      if (room) {
+        cnt = gw * gh;
+      } else {
+        const Frame fr = frame_of_gaussian(frames, g, n);
+        const int64_t left = max(tiles_that_fit(offsets, T, cap) - fr.first_tile, (int64_t)0);
+        const int64_t row = left / fr.tiles_x - gy0;  // the first truncated tile's in the rectangle
+        if (row >= gh)
+          cnt = gw * gh;
+        else if (row >= 0)
+          cnt = (int)row * gw + min(max((int)(left % fr.tiles_x) - gx0, 0), gw);
+      }
+    }
   }
   int incl = cnt;  // the total is at most the capacity, below 2^31
 #pragma unroll
@@ -1398,13 +1413,14 @@ __global__ void __launch_bounds__(kEpilogueThreads)
   if (threadIdx.x == 0) cta_first = atomicAdd(cursor, (unsigned)total);
   __syncthreads();
   if (g >= n) return;
-  const int beg = room ? (int)cta_first + before + incl - cnt : 0;
+  const int beg = room || rest ? (int)cta_first + before + incl - cnt : 0;
   seg[g] = beg;
   seg[n + g] = beg + cnt;
 }
 
-int assign_entry_slots(const void* records, int64_t n, int ts, const int32_t* offsets, int64_t T,
-                       int64_t cap, void* ws, cudaStream_t s) {
+int assign_entry_slots(const Frames& f, const void* records, int64_t n, int ts,
+                       const int32_t* offsets, int64_t T, int64_t cap, bool rest, void* ws,
+                       cudaStream_t s) {
   const EntryOrder eo = entry_order_layout(ws, n, cap);
   if (cap == 0) {
     cudaMemsetAsync(eo.seg, 0, sizeof(int32_t) * 2 * n, s);
@@ -1413,7 +1429,7 @@ int assign_entry_slots(const void* records, int64_t n, int ts, const int32_t* of
   cudaMemsetAsync(eo.keys_in, 0, sizeof(unsigned), s);  // the cursor: no keys in this mode
   launch("entry_slots_kernel", entry_slots_kernel,
          (unsigned)((n + kEpilogueThreads - 1) / kEpilogueThreads), kEpilogueThreads, 0, s,
-         static_cast<const Splat*>(records), n, ts, offsets, T, cap, eo.keys_in, eo.seg);
+         static_cast<const Splat*>(records), n, ts, f, offsets, T, cap, rest, eo.keys_in, eo.seg);
   return check_launch("entry slots");
 }
 
@@ -1865,7 +1881,7 @@ int render_backward_tiles(const Frames& f, int ts, int64_t T, const float* grad_
   const float4* pg = reinterpret_cast<const float4*>(pixel_grad);
   int rc;
   if (deterministic == kEntrySlots &&
-      (rc = assign_entry_slots(records, n, ts, offsets, T, cap, ws, s)))
+      (rc = assign_entry_slots(f, records, n, ts, offsets, T, cap, pixel_grad != nullptr, ws, s)))
     return rc;
   if (pixel_grad) {
     if (ts == 16)
@@ -2266,7 +2282,8 @@ int ss_fit_forward_backward(const ss_batch* batch, const void* records, int64_t 
   const Splat* rec = static_cast<const Splat*>(records);
   float* ws = static_cast<float*>(workspace);
   if (deterministic == kEntrySlots && n > 0 &&
-      (rc = assign_entry_slots(records, n, batch->tile_size, tile_offsets, T, gid_capacity, ws, s)))
+      (rc = assign_entry_slots(f, records, n, batch->tile_size, tile_offsets, T, gid_capacity, true,
+                               ws, s)))
     return rc;
   if (batch->tile_size == 16)
     launch_fused<16>((unsigned)T, s, deterministic, rec, n, tile_gids, gid_capacity,
@@ -2311,7 +2328,8 @@ int ss_render_forward_backward(const void* records, int64_t n, const int32_t* ti
   const Splat* rec = static_cast<const Splat*>(records);
   float* ws = static_cast<float*>(workspace);
   if (deterministic == kEntrySlots && n > 0 &&
-      (rc = assign_entry_slots(records, n, tile_size, tile_offsets, T, gid_capacity, ws, s)))
+      (rc = assign_entry_slots(f, records, n, tile_size, tile_offsets, T, gid_capacity, false, ws,
+                               s)))
     return rc;
   if (tile_size == 16)
     launch_fused<16>((unsigned)T, s, deterministic, rec, n, tile_gids, gid_capacity,
