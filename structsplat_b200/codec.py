@@ -54,18 +54,27 @@ def _inflate(payload: bytes, codec: str, raw_len):
     raise ValueError(f"unknown stream_codec {codec!r}; expected 'zlib' or 'png'")
 
 
-_POOL: tuple | None = None  # (process id, executor)
+_POOL: ThreadPoolExecutor | None = None
 _POOL_LOCK = threading.Lock()
 
 
 def _pool() -> ThreadPoolExecutor:
-    """At most four threads, started on first use and kept by this process (a forked child, which
-    inherits none of them, starts its own); joined at exit."""
+    """At most four threads, started on first use and kept by this process; joined at exit."""
     global _POOL
     with _POOL_LOCK:
-        if _POOL is None or _POOL[0] != os.getpid():
-            _POOL = (os.getpid(), ThreadPoolExecutor(4, thread_name_prefix="sspl1-inflate"))
-        return _POOL[1]
+        if _POOL is None:
+            _POOL = ThreadPoolExecutor(4, thread_name_prefix="sspl1-inflate")
+        return _POOL
+
+
+def _forked():
+    """A child inherits neither the threads nor whoever held the lock: it starts its own."""
+    global _POOL, _POOL_LOCK
+    _POOL, _POOL_LOCK = None, threading.Lock()
+
+
+if hasattr(os, "register_at_fork"):
+    os.register_at_fork(after_in_child=_forked)
 
 
 def _inflate_all(streams, codec: str):
