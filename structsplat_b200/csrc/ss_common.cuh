@@ -137,6 +137,12 @@ __device__ __forceinline__ void support_rect(float mx, float my, long long rx, l
   y1 = (int)yh + 1;
 }
 
+// A projection's radius (a whole float >= 1, infinite for a support without bound) as the int64 that
+// the callers' radii tensors hold.
+__device__ __forceinline__ long long radius_i64(float r) {
+  return r <= 1e15f ? (long long)r : (1LL << 40);
+}
+
 // The same for radii that are whole floats >= 1 (a projection's), in 32-bit arithmetic where the
 // centre and radii are small enough for it to be exact: conversions to int64 run at a fraction
 // of the rate, and every Gaussian near an image takes the short way.
@@ -155,9 +161,7 @@ __device__ __forceinline__ void support_rect_f(float mx, float my, float rx, flo
     y1 = any ? yh + 1 : 0;
     return;
   }
-  const long long lim = 1LL << 40;
-  support_rect(mx, my, rx < 1e12f ? (long long)rx : lim, ry < 1e12f ? (long long)ry : lim, H, W,
-               x0, y0, x1, y1);
+  support_rect(mx, my, radius_i64(rx), radius_i64(ry), H, W, x0, y0, x1, y1);
 }
 
 __device__ __forceinline__ Splat make_splat(float mx, float my, float a, float b, float c,
@@ -399,11 +403,6 @@ __device__ __forceinline__ Splat rs_project_one(const RSField& f, const RSParams
   int x0, y0, x1, y1;
   support_rect_f(p.mx, p.my, rx, ry, H, W, x0, y0, x1, y1);
   return make_splat(p.mx, p.my, a, b, c, op, p.cr, p.cg, p.cb, x0, y0, x1, y1);
-}
-
-// Radius as the int64 the callers' radii tensors hold.
-__device__ __forceinline__ long long radius_i64(float r) {
-  return r <= 1e15f ? (long long)r : (1LL << 40);
 }
 
 // The backward's per-(tile, Gaussian) record in deterministic mode: nine moments, padded.
