@@ -218,16 +218,16 @@ __device__ __forceinline__ void enumerate_pairs(const Splat* rec, int64_t i, int
 }
 
 // Whether a tile whose bin does not hold its list of len ids is listed by testing every record of its
-// image, or else from the pairs (place_overflow).  A CTA tests ~0.25 records per ns, so lists of more
-// than 1/8 of the image's Gaussians are sooner found that way (`tests` 8), and all of them where the
-// whole set's tests are few (see index_tests).  Long lists of large images count for more: from the pairs
-// they would be sorted in place.  Either way the work is bounded by the pairs or by kFewTests.
+// image, or else from the pairs (place_overflow).  The machine tests ~370 records per ns and places ~40
+// pairs, so lists of more than 1/8 of the image's Gaussians are sooner found that way (`tests` 8), and all
+// of them where the whole set's tests are few (see index_tests).  Either way the work is bounded by the
+// pairs or by kFewTests.
 constexpr int kSortIds = 4096;                      // most ids sorted in shared memory
 constexpr int kWindowIds = 32 * (kSortIds + 1024);  // most ids a bitmap there holds: 163,840
 constexpr int64_t kFewTests = 1 << 24;              // ~45 us
 inline int index_tests(int64_t n, int64_t T) { return n * T <= kFewTests ? INT_MAX : 8; }
 __host__ __device__ inline bool listed_from_records(int64_t len, int64_t count, int tests) {
-  return len * (len > kSortIds && count > kWindowIds && tests < 64 ? 64 : tests) >= count;
+  return len * tests >= count;
 }
 
 // Words in the padding after the counters, zeroed with them.  Of counter 0: the bins' size, whether
@@ -950,7 +950,10 @@ __device__ __forceinline__ void cta_sort_bin(const Splat* __restrict__ rec, int6
   }
 }
 
-// Puts g[0, len), a list in arrival order, into ascending order.  Every thread of the CTA calls it.
+// Puts g[0, len), a list in arrival order, into ascending order: by buckets, or by windows of the ids as
+// in cta_sort_bin, but in place: while a window's bits are set, the ids of later windows move to the end
+// of the list, from its end on, and leave the room that the window's ids then take.  Every thread of the
+// CTA calls it.
 __device__ __noinline__ void sort_placed(int32_t* g, int len, int first, int count, uint32_t* smem,
                                          int* tmp) {
   const PlacedIds list{g};
@@ -961,25 +964,43 @@ __device__ __noinline__ void sort_placed(int32_t* g, int len, int first, int cou
   } else if (len <= kSortIds) {
     if (bucket_sort<kBuckets>(list, len, first, count, buf, buf + kSortIds, tmp, g, shift)) return;
   }
-  __syncthreads();  // every thread has left the buckets
-  auto sync = [] { __syncthreads(); };
-  if (count <= kWindowIds) {
-    const int nw = (count + 31) >> 5;
+  constexpr int kOwn = 8, kChunk = kOwn * kSortThreads;
+  int done = 0;
+  for (int w0 = 0; done < len && w0 < count; w0 += kWindowIds) {
+    const int ids = min(count - w0, kWindowIds), nw = (ids + 31) >> 5;
+    __syncthreads();  // every thread has left the buckets, or the window before
     for (int w = threadIdx.x; w < nw; w += kSortThreads) smem[w] = 0u;
     __syncthreads();
-    for (int e = threadIdx.x; e < len; e += kSortThreads) {
-      const int rel = list[e] - first;
-      atomicOr(&smem[rel >> 5], 1u << (rel & 31));
+    int end = len;  // the ids of later windows start here
+    for (int hi = len; hi > done; hi -= kChunk) {
+      const int lo = max(done, hi - kChunk);
+      int later[kOwn], num = 0;
+#pragma unroll
+      for (int u = 0; u < kOwn; ++u) {
+        const int e = lo + u * kSortThreads + threadIdx.x;
+        later[u] = e < hi ? list[e] : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kOwn; ++u) {
+        const int rel = later[u] - first - w0;
+        if (later[u] >= 0 && rel < ids) {
+          atomicOr(&smem[rel >> 5], 1u << (rel & 31));
+          later[u] = -1;
+        }
+        num += later[u] >= 0;
+      }
+      if (w0 + ids == count) continue;  // the last window: nothing is later
+      int at = block_exclusive(num, tmp);  // the chunk has been read
+      __syncthreads();
+      end -= tmp[kSortWarps];
+#pragma unroll
+      for (int u = 0; u < kOwn; ++u)
+        if (later[u] >= 0) g[end + at++] = later[u];
     }
     __syncthreads();
-    emit_bits(smem, nw, first, g, len, tmp);
-  } else if (len <= kSortIds) {
-    for (int e = threadIdx.x; e < len; e += kSortThreads) buf[e] = list[e];
-    __syncthreads();
-    bitonic_sort(buf, len, threadIdx.x, kSortThreads, sync);
-    for (int e = threadIdx.x; e < len; e += kSortThreads) g[e] = buf[e];
-  } else {
-    bitonic_sort(g, len, threadIdx.x, kSortThreads, sync);
+    const int room = w0 + ids == count ? len - done : end - done;
+    emit_bits(smem, nw, first + w0, g + done, room, tmp);
+    done += room;
   }
 }
 
@@ -1416,7 +1437,8 @@ int index_fill(const Frames& frames, int ts, int64_t T, const void* records, int
     const int tests = index_tests(n, T);
     int64_t parts = ctas / 2 < kMostParts ? ctas / 2 : kMostParts;
     if (parts < kLeastParts) parts = kLeastParts;
-    const int lanes = n >= parts * kSortThreads ? 32 : 8;  // a warp's Gaussians at a time
+    int lanes = 32;  // a warp's Gaussians at a time
+    while (lanes > 1 && n < parts * kSortWarps * lanes) lanes >>= 1;
     const int64_t share = (n + lanes * kSortWarps - 1) / (lanes * kSortWarps);
     if (share < parts) parts = share;
     if (tests == INT_MAX) parts = 0;  // all from the records: nothing is placed

@@ -27,16 +27,18 @@ def test_wide_gaussians(n, H, W, ts, r, cull):
     _same(_records(_uniform(n, H, W), H, W, r, conic), n, H, W, ts, cull)
 
 
-# bins of 3,168, 832 and 31,296 ids, lists of up to 10k and 45k in one part of the image
-@pytest.mark.parametrize("n,ts,sigma", [(100_000, 32, 40), (100_000, 16, 40), (1_000_000, 32, 60)])
+# bins of 3,168, 832, 2,400 and 31,296 ids, lists of up to 10k, 5k and 45k in one part of the image; ids of
+# one, two and seven windows
+@pytest.mark.parametrize("n,ts,sigma", [(100_000, 32, 40), (100_000, 16, 40), (300_000, 16, 55),
+                                        (1_000_000, 32, 60)])
 def test_clumps(n, ts, sigma):
     require_cuda()
     m = np.random.default_rng(0).normal(512, sigma, (n, 2))
     _same(_records(m, 1024, 1024, 6), n, 1024, 1024, ts)
 
 
-# More than 163,840 Gaussians; one tile gets `run` ids in a row, too many for a bucket, in a list that
-# shared memory holds (3,000, 4,096) and one that it does not, below 1/64 of the ids
+# More than 163,840 Gaussians; one tile gets `run` ids in a row, too many for a bucket, in a list that the
+# buckets hold (3,000, 4,096) and one that they do not
 @pytest.mark.parametrize("n,side,run", [(200_000, 1024, 3_000), (200_000, 1024, 4_096),
                                         (400_000, 2048, 5_000)])
 def test_consecutive_ids_in_one_tile(n, side, run):
