@@ -558,7 +558,11 @@ struct FwdSmem {
   static constexpr int kWarps = kThreads / 32;
   // Two CTAs of a 32-px tile's 16 warps share an SM, eight of a 16-px tile's four (64 registers a
   // thread either way), the stage as large as that leaves.  16-px tiles used to stage 512 records
-  // too, four CTAs to an SM: 18.0 -> 15.7 us for 20k Gaussians on 517x389.  Eight warps with two
+  // too, four CTAs to an SM: 18.0 -> 15.7 us for 20k Gaussians on 517x389, 359 -> 265 for 800k on
+  // 3840x2160, 136 -> 133 for lists of 200 (300k on 1024x1024).  A few very long lists among short ones
+  // are the other side: they end on SMs of their own, where 64 registers a thread cost more than
+  // occupancy gains (70 % of those 300k in one clump, lists up to 7,704: 288 -> 340); nothing known at
+  // the launch tells the two apart.  Eight warps with two
   // blocks each, four CTAs to an SM, were no gain for 32-px tiles: alone 312 us against 318 at
   // 3840x2160, but the 1024x1024 step 125 us against 117, the kernel overlapping its neighbours
   // less.
@@ -615,8 +619,11 @@ __device__ __forceinline__ int block_hits(const float4 (*st)[4], const int4* rec
 // be refilled).  MASKS: by block masks; long lists are often of wide Gaussians that hit most blocks
 // (1024x1024, 250k heavy-tailed: 673 us for the forward without them, 710 us with), so only the
 // fused pass, whose streamed lists are mostly dense fields of small ones, uses them (1920x1080,
-// 2 M around 1 px: 945 -> 884 us).  Every thread of the CTA calls it: it holds the CTA's barriers.
-template <int TS, int NT, bool FADE, bool MASKS, typename List>
+// 2 M around 1 px: 945 -> 884 us).  AHEAD > 0: the ids of the chunk after the next are loaded during the
+// evaluation, at most AHEAD per thread, so that its copies need not wait for them (16-px lists of
+// thousands: 253 -> 232 us for 100k Gaussians on 640x480, 70 % in one clump; 32 px 394 -> 378).  Every
+// thread of the CTA calls it: it holds the CTA's barriers.
+template <int TS, int NT, bool FADE, bool MASKS, int AHEAD, typename List>
 __device__ __forceinline__ void stream_block(float4 (*stage)[4], int stage_slots,
                                              const Splat* __restrict__ rec, const TileList& L,
                                              const List& q, int qcap, int carry0, int null_slot,
@@ -630,18 +637,42 @@ __device__ __forceinline__ void stream_block(float4 (*stage)[4], int stage_slots
   auto len = [&](int64_t k0) { return (int)(count - k0 < half ? count - k0 : half); };
   bool exact = false;
   int qn = 0;
+  int ids[AHEAD > 0 ? AHEAD : 1];
+  auto load_ids = [&](int64_t k0) {
+    const int m = len(k0);
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int slot = (threadIdx.x + u * NT) >> 2;
+      ids[u] = slot < m ? L.gid(k0 + slot) : 0;
+    }
+  };
   if (!chunk0_issued) {
     stage_range<NT>(stage, rec, L, 0, len(0), nullptr, rects);
     cp_async_commit();
   }
+  if (AHEAD > 0) load_ids(half);
   for (int c = 0; c < nchunks; ++c) {
     const int64_t k0 = (int64_t)c * half;
-    if (c + 1 < nchunks)
-      stage_range<NT>(stage + ((c + 1) & 1) * half, rec, L, k0 + half, len(k0 + half), nullptr,
-                      rects ? rects + ((c + 1) & 1) * half : nullptr);
-    cp_async_commit();
-    cp_async_wait_one();
-    __syncthreads();
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // chunk c is there, and every warp has left the half that chunk c + 1 takes
+    if (c + 1 < nchunks) {
+      float4(*to)[4] = stage + ((c + 1) & 1) * half;
+      int4* rto = rects ? rects + ((c + 1) & 1) * half : nullptr;
+      if constexpr (AHEAD > 0) {
+        const int m = len(k0 + half), piece = threadIdx.x & 3;
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+          const int slot = (threadIdx.x + u * NT) >> 2;
+          if (slot < m)
+            cp_async16(rto && piece == 3 ? static_cast<void*>(&rto[slot]) : &to[slot][piece],
+                       reinterpret_cast<const float4*>(rec + ids[u]) + piece);
+        }
+        load_ids(k0 + 2 * half);
+      } else {
+        stage_range<NT>(to, rec, L, k0 + half, len(k0 + half), nullptr, rto);
+      }
+      cp_async_commit();
+    }
     const int m = len(k0), s0 = (c & 1) * half;
     exact = !check_records<TS, NT>(stage + s0, rects ? rects + s0 : nullptr,
                                    MASKS ? masks + s0 : nullptr, m, tx0, ty0) || exact;
@@ -651,8 +682,8 @@ __device__ __forceinline__ void stream_block(float4 (*stage)[4], int stage_slots
                             null_slot, sx0, sy0, lane, tail, acc);
       if (!last) carry_pending(stage, q, qn, carry0, lane);
     }
-    __syncthreads();
   }
+  __syncthreads();
 }
 
 // Forward of one tile, one warp per 8x8 block.  LOSS == kNoLoss: writes out and den.
@@ -714,10 +745,11 @@ __global__ void __launch_bounds__(FwdSmem<TS, LONG>::kThreads, (FwdSmem<TS, LONG
                        exact, S::kNullSlot, sx0, sy0, lane, tail, acc);
   } else {
     // a streamed list moves through two chunks of `chunk` records (at most half the stage)
-    stream_block<TS, NT, FADE, false>(stage, 2 * min(chunk, S::kStage / 2), rec, L, list,
-                                      S::kListLen, S::kStage + warp * kCarrySlots, S::kNullSlot,
-                                      true, block_bit, tx0, ty0, sx0, sy0, lane, tail, acc, masks,
-                                      false, rects);
+    constexpr int kAhead = 4 * (S::kStage / 2 < kForwardChunk ? S::kStage / 2 : kForwardChunk) / NT;
+    stream_block<TS, NT, FADE, false, kAhead>(stage, 2 * min(chunk, S::kStage / 2), rec, L, list,
+                                              S::kListLen, S::kStage + warp * kCarrySlots,
+                                              S::kNullSlot, true, block_bit, tx0, ty0, sx0, sy0, lane,
+                                              tail, acc, masks, false, rects);
   }
   float v[2][4];
   combine_groups(acc, lane, v);
@@ -1155,7 +1187,7 @@ __global__ void __launch_bounds__(NT, (BackwardOccupancy<TS, NT>::kBlocks))
         for (int ch = 0; ch < 4; ++ch) acc[k][ch] = make_float2(0.f, 0.f);
       const PixelList list{reinterpret_cast<uint32_t*>(pix + by * TS + bx), TS * 4};
       if (!whole)
-        stream_block<TS, NT, FADE, true>(stage, kStageMax, rec, L, list, kPixelListLen,
+        stream_block<TS, NT, FADE, true, 0>(stage, kStageMax, rec, L, list, kPixelListLen,
                                    kStageMax + warp * kCarrySlots, kNullSlot, active, 1u << b,
                                    tx0, ty0, tx0 + bx, ty0 + by, lane, tail, acc, masks, i == 0,
                                    nullptr);
