@@ -179,6 +179,7 @@ class FitPlan:
         self.offsets = torch.zeros(batch.tiles + 1, device=d, dtype=torch.int32)
         self.status = torch.zeros(1, device=d, dtype=torch.int32)
         self.entries = 0  # as measured last
+        self.idx_ws_bytes = -1
         self._size_index(0)
         if capacity <= 0:
             capacity = self.measure_entries() * 3 // 2 + 4096
@@ -232,8 +233,11 @@ class FitPlan:
 
     def _size_index(self, entries: int):
         """The index workspace for about ``entries`` tile-list entries (0: not known)."""
-        self.idx_ws_bytes = _native.size_query("ss_tile_index_entries_workspace_bytes", self.n,
-                                               self.batch.tiles, self.batch.images, entries)
+        nbytes = _native.size_query("ss_tile_index_entries_workspace_bytes", self.n,
+                                    self.batch.tiles, self.batch.images, entries)
+        if nbytes == self.idx_ws_bytes:
+            return
+        self.idx_ws_bytes, self.idx_ws = nbytes, None  # given back before the next is taken
         self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=self.batch.device,
                                   dtype=torch.uint8)
 

@@ -60,6 +60,7 @@ class RenderPlan:
         f32 = dict(device=d, dtype=torch.float32)
         self.records = torch.empty(max(n, 1) * RECORD_FLOATS, **f32)
         self.offsets = torch.zeros(self.T + 1, device=d, dtype=torch.int32)
+        self.idx_ws_bytes = -1
         self._size_index(0)
         if self.capacity <= 0:
             self.capacity = 1
@@ -100,8 +101,11 @@ class RenderPlan:
 
     def _size_index(self, entries: int):
         """The index workspace for about ``entries`` tile-list entries (0: not known)."""
-        self.idx_ws_bytes = _native.size_query("ss_tile_index_entries_workspace_bytes", self.n,
-                                               self.T, 1, entries)
+        nbytes = _native.size_query("ss_tile_index_entries_workspace_bytes", self.n, self.T, 1,
+                                    entries)
+        if nbytes == self.idx_ws_bytes:
+            return
+        self.idx_ws_bytes, self.idx_ws = nbytes, None  # given back before the next is taken
         self.idx_ws = torch.empty(max(self.idx_ws_bytes, 1), device=self.device, dtype=torch.uint8)
 
     # -- stages --------------------------------------------------------------------------

@@ -170,3 +170,27 @@ def test_plans_take_the_plain_form_for_wide_fields():
         out, _ = R.render_cuda_exact_with_coverage(p["means"], conics, p["colors"], radii, H, W,
                                                    tile_size=ts)
         assert torch.equal(out, image)
+
+
+def test_a_plan_keeps_the_workspace_that_fits():
+    """Planning takes one index workspace when the measured entries ask for the form it began with."""
+    require_cuda()
+    from structsplat_b200.batch import FitPlan
+    from structsplat_b200.synthetic import make_field
+    n, H, W = 5_000, 256, 256
+    f = make_field(H, W, n, 3)
+    p = {k: torch.tensor(getattr(f, k), device="cuda")
+         for k in ("means", "log_scales", "rotations", "colors", "opacity_logits")}
+    seen = []
+    empty = torch.empty
+
+    def counted(*args, **kw):
+        t = empty(*args, **kw)
+        seen.append(t.numel() if t.dtype == torch.uint8 else 0)
+        return t
+    try:
+        torch.empty = counted
+        plan = FitPlan(Batch([(H, W)], [n]), p, torch.zeros(H * W, 3, device="cuda"))
+    finally:
+        torch.empty = empty
+    assert seen.count(plan.idx_ws_bytes) == 1
