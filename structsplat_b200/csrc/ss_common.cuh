@@ -88,6 +88,11 @@ constexpr unsigned kDependentTiles = 592;  // two rounds of two CTAs per SM
 // size a kernel is launched with, set once per kernel and device).
 int allow_dynamic_smem(const void* kern, size_t bytes);
 
+// Runs `kern` with the SM's memory split in favour of shared memory (set once per kernel and device).  An
+// SM changes the split only when it is empty: a kernel that starts early beside a predecessor with
+// another split crowds on the SMs that the predecessor left free.
+int prefer_shared_memory(const void* kern);
+
 // launch_as() and launch() of a kernel whose shared memory is dynamic: `smem` bytes, opted in first.
 template <typename... KArgs, typename... Args>
 int launch_smem_as(bool dependent, const char* what, void (*kern)(KArgs...), dim3 grid, dim3 block,

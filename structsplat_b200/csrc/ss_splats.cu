@@ -40,6 +40,21 @@ int check_launch(const char* what) {
   return SS_OK;
 }
 
+int prefer_shared_memory(const void* kern) {
+  static std::mutex mu;
+  static std::vector<std::pair<const void*, int>> done;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return check_launch("cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mu);
+  for (const auto& d : done)
+    if (d.first == kern && d.second == dev) return SS_OK;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                           cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+    return check_launch("shared memory carve-out attribute");
+  done.emplace_back(kern, dev);
+  return SS_OK;
+}
+
 int allow_dynamic_smem(const void* kern, size_t bytes) {
   // (kernel, device) pairs already opted in; a handful of kernels use more than 48 KB
   static std::mutex mu;
