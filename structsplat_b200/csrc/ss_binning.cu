@@ -555,38 +555,6 @@ __global__ void __launch_bounds__(kScanThreads)
   }
 }
 
-// Ascending sort of buf[0..len) using a bitonic network over the next power of two in which
-// every comparator puts the smaller key first; positions >= len act as +inf and never move.
-template <typename Sync>
-__device__ void bitonic_sort(int* buf, int len, int tid, int nthreads, Sync sync) {
-  int n2 = 1;
-  while (n2 < len) n2 <<= 1;
-  for (int lk = 1; (1 << lk) <= n2; ++lk) {
-    const int k = 1 << lk;
-    for (int lj = lk - 1; lj >= 0; --lj) {
-      const int j = 1 << lj;
-      for (int p = tid; p < (n2 >> 1); p += nthreads) {
-        int blk = p >> lj, r = p & (j - 1), a, b;
-        if (j == (k >> 1)) {
-          a = blk * k + r;
-          b = blk * k + k - 1 - r;
-        } else {
-          a = blk * 2 * j + r;
-          b = a + j;
-        }
-        if (b < len) {
-          int va = buf[a], vb = buf[b];
-          if (va > vb) {
-            buf[a] = vb;
-            buf[b] = va;
-          }
-        }
-      }
-      sync();
-    }
-  }
-}
-
 // Ascending sort of up to 32*K keys held in registers across a warp: key k of lane l is element
 // 32k + l, missing elements are INT_MAX.  Standard bitonic network: at block size `size` and
 // distance j, elements e and e^j are compared and the block (e & size) == 0 sorts upward.
@@ -724,10 +692,10 @@ __global__ void __launch_bounds__(1024) tile_sort_big_kernel(const int32_t* __re
     } else if (len <= kBigSortSmem) {
       for (int e = threadIdx.x; e < len; e += blockDim.x) sbuf[e] = gids[lo + e];
       __syncthreads();
-      bitonic_sort(sbuf, len, threadIdx.x, blockDim.x, sync);
+      sort_ascending(sbuf, len, threadIdx.x, blockDim.x, sync);
       for (int e = threadIdx.x; e < len; e += blockDim.x) gids[lo + e] = sbuf[e];
     } else {
-      bitonic_sort(gids + lo, len, threadIdx.x, blockDim.x, sync);
+      sort_ascending(gids + lo, len, threadIdx.x, blockDim.x, sync);
     }
     __syncthreads();
   }

@@ -564,6 +564,29 @@ __device__ __forceinline__ void sum_entry_partials(const float* __restrict__ par
   }
 }
 
+// Ascending sort of v[0, m) by `threads` threads (t the caller's): a bitonic network whose every
+// exchange leaves the smaller value at the lower place, so the places from m up to the next power of
+// two need not exist.
+template <typename Sync>
+__device__ __forceinline__ void sort_ascending(int* v, int m, int t, int threads, Sync sync) {
+  int half = 1;  // pairs of the network: half the next power of two
+  while (2 * half < m) half <<= 1;
+  for (int size = 2; size <= 2 * half; size <<= 1) {
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+      for (int p = t; p < half; p += threads) {
+        const int i = 2 * p - (p & (stride - 1));  // the lower of the pair's places
+        const int j = stride == (size >> 1) ? (i ^ (size - 1)) : i + stride;
+        if (j < m && v[i] > v[j]) {
+          const int x = v[i];
+          v[i] = v[j];
+          v[j] = x;
+        }
+      }
+      sync();
+    }
+  }
+}
+
 __device__ __forceinline__ void raise_status(uint32_t* status, uint32_t bits) {
   if (status) atomicOr(status, bits);
 }

@@ -167,41 +167,27 @@ __device__ __forceinline__ void stage_with_masks(float4 (*dst)[4], const Splat* 
                                                  const TileList& L, int m, int4* rects,
                                                  uint16_t* masks, int tx0, int ty0) {
   constexpr int kIters = 4 * SLOTS / NT;
-  static_assert(kIters * NT == 4 * SLOTS && NT % 4 == 0, "pieces per thread");
+  static_assert(kIters * NT == 4 * SLOTS && NT % 4 == 0 && kIters <= 8, "pieces per thread");
   const int piece = threadIdx.x & 3;
-  if constexpr (kIters <= 8) {
-    int4 r[kIters];
+  int4 r[kIters];
+#pragma unroll
+  for (int k = 0; k < kIters; ++k) {
+    const int slot = (threadIdx.x + k * NT) >> 2;
+    if (slot < m) {
+      const float4* from = reinterpret_cast<const float4*>(rec + L.gid(slot)) + piece;
+      if (piece == 3)
+        r[k] = *reinterpret_cast<const int4*>(from);
+      else
+        cp_async16(&dst[slot][piece], from);
+    }
+  }
+  if (piece == 3) {
 #pragma unroll
     for (int k = 0; k < kIters; ++k) {
       const int slot = (threadIdx.x + k * NT) >> 2;
       if (slot < m) {
-        const float4* from = reinterpret_cast<const float4*>(rec + L.gid(slot)) + piece;
-        if (piece == 3)
-          r[k] = *reinterpret_cast<const int4*>(from);
-        else
-          cp_async16(&dst[slot][piece], from);
-      }
-    }
-    if (piece == 3) {
-#pragma unroll
-      for (int k = 0; k < kIters; ++k) {
-        const int slot = (threadIdx.x + k * NT) >> 2;
-        if (slot < m) {
-          rects[slot] = r[k];
-          masks[slot] = block_mask<TS>(r[k], tx0, ty0);
-        }
-      }
-    }
-  } else {
-    for (int q = threadIdx.x; q < 4 * m; q += NT) {
-      const int slot = q >> 2;
-      const float4* from = reinterpret_cast<const float4*>(rec + L.gid(slot)) + piece;
-      if (piece == 3) {
-        const int4 r = *reinterpret_cast<const int4*>(from);
-        rects[slot] = r;
-        masks[slot] = block_mask<TS>(r, tx0, ty0);
-      } else {
-        cp_async16(&dst[slot][piece], from);
+        rects[slot] = r[k];
+        masks[slot] = block_mask<TS>(r[k], tx0, ty0);
       }
     }
   }
@@ -1389,6 +1375,32 @@ __global__ void entry_segments_kernel(const uint32_t* __restrict__ keys, int64_t
   }
 }
 
+// First of cnt consecutive places for each thread's Gaussian: a CTA's lie side by side, reserved with one
+// atomic (the total is at most the capacity, below 2^31).  Every thread of the CTA calls it.
+__device__ __forceinline__ int reserve_run(int cnt, unsigned* cursor) {
+  constexpr int kWarps = kEpilogueThreads / 32;
+  __shared__ int warp_total[kWarps];
+  __shared__ unsigned cta_first;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) warp_total[warp] = incl;
+  __syncthreads();
+  int before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    before += w < warp ? warp_total[w] : 0;
+    total += warp_total[w];
+  }
+  if (threadIdx.x == 0) cta_first = atomicAdd(cursor, (unsigned)total);
+  __syncthreads();
+  return (int)cta_first + before + incl - cnt;
+}
+
 // Slot mode, before the backward: each Gaussian's partials get consecutive slots, one per tile of
 // its rectangle (its entries, in an index built without the ellipse cull).  A CTA reserves its
 // Gaussians' slots with one atomic; where they land varies from run to run, the order of a
@@ -1404,10 +1416,7 @@ __global__ void __launch_bounds__(kEpilogueThreads)
                        unsigned* __restrict__ cursor, int32_t* __restrict__ seg) {
   pdl_wait();
   pdl_trigger();
-  __shared__ int warp_total[kEpilogueThreads / 32];
-  __shared__ unsigned cta_first;
   const int64_t g = (int64_t)blockIdx.x * kEpilogueThreads + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool room = offsets[T] <= cap;
   int cnt = 0;
   if (g < n && (room || rest)) {
@@ -1428,24 +1437,9 @@ __global__ void __launch_bounds__(kEpilogueThreads)
       }
     }
   }
-  int incl = cnt;  // the total is at most the capacity, below 2^31
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) warp_total[warp] = incl;
-  __syncthreads();
-  int before = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < kEpilogueThreads / 32; ++w) {
-    before += w < warp ? warp_total[w] : 0;
-    total += warp_total[w];
-  }
-  if (threadIdx.x == 0) cta_first = atomicAdd(cursor, (unsigned)total);
-  __syncthreads();
+  const int first = reserve_run(cnt, cursor);
   if (g >= n) return;
-  const int beg = room || rest ? (int)cta_first + before + incl - cnt : 0;
+  const int beg = room || rest ? first : 0;
   seg[g] = beg;
   seg[n + g] = beg + cnt;
 }
@@ -1563,10 +1557,7 @@ __global__ void __launch_bounds__(kEpilogueThreads)
                        int32_t* __restrict__ seg) {
   pdl_wait();
   pdl_trigger();
-  __shared__ int warp_total[kWarpsPerCta];
-  __shared__ unsigned cta_first;
   const int64_t g = (int64_t)blockIdx.x * kEpilogueThreads + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int cnt = 0;
   unsigned mask = 0;
   if (g < n) {
@@ -1576,24 +1567,9 @@ __global__ void __launch_bounds__(kEpilogueThreads)
       cnt = __popc(mask);
     }
   }
-  int incl = cnt;  // the total is at most the capacity, below 2^31
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) warp_total[warp] = incl;
-  __syncthreads();
-  int before = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < kWarpsPerCta; ++w) {
-    before += w < warp ? warp_total[w] : 0;
-    total += warp_total[w];
-  }
-  if (threadIdx.x == 0) cta_first = atomicAdd(cursor, (unsigned)total);
-  __syncthreads();
+  const int first = reserve_run(cnt, cursor);
   if (g >= n) return;
-  const int beg = (int)cta_first + before + incl - cnt;
+  const int beg = first;
   seg[g] = beg;
   seg[n + g] = beg + cnt;
   if (mask) masks[beg] = mask;
@@ -1615,29 +1591,6 @@ __global__ void __launch_bounds__(kMarkThreads)
                                   : (int)rank[e];
                 order[beg + k] = e;
               });
-}
-
-// Ascending sort of v[0, m) by `threads` threads (t the caller's): a bitonic network whose every
-// exchange leaves the smaller value at the lower place, so the places from m up to the next power of
-// two need not exist.
-template <typename Sync>
-__device__ __forceinline__ void sort_ascending(int* v, int m, int t, int threads, Sync sync) {
-  int half = 1;  // pairs of the network: half the next power of two
-  while (2 * half < m) half <<= 1;
-  for (int size = 2; size <= 2 * half; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int p = t; p < half; p += threads) {
-        const int i = 2 * p - (p & (stride - 1));  // the lower of the pair's places
-        const int j = stride == (size >> 1) ? (i ^ (size - 1)) : i + stride;
-        if (j < m && v[i] > v[j]) {
-          const int x = v[i];
-          v[i] = v[j];
-          v[j] = x;
-        }
-      }
-      sync();
-    }
-  }
 }
 
 // The runs of rectangles of more than kMaskTiles tiles into ascending order: up to kWarpRun entries
