@@ -1165,17 +1165,26 @@ __device__ __noinline__ void sort_placed_tiles(const BinSort& a, const Frames& f
   }
 }
 
+// Where the list of a warp's tile (with four to a CTA; else of the CTA's) begins and ends.
+struct ListEnds {
+  long long lo, hi;
+};
+__device__ __forceinline__ ListEnds ends_of(const BinSort& a, int64_t t0) {
+  const int64_t t = t0 + (a.tiles_per_cta > 1 ? threadIdx.x >> 5 : 0);
+  return t < a.T ? ListEnds{__ldg(a.off64 + t), __ldg(a.off64 + t + 1)} : ListEnds{0, 0};
+}
+
 // Sorts the tiles_per_cta tiles from t0 on, but for those that place_overflow lists (`some` of them).
 template <bool CULL>
 __device__ __forceinline__ void sort_tiles(const BinSort& a, const Frames& frames, int64_t t0,
-                                           const Overflow& over, bool some, uint32_t* smem,
-                                           int* tmp) {
+                                           const ListEnds& ends, const Overflow& over, bool some,
+                                           uint32_t* smem, int* tmp) {
   if (a.tiles_per_cta > 1) {
     const int lane = threadIdx.x & 31;
     const int64_t t = t0 + (threadIdx.x >> 5);
     bool mine = false;  // the CTA takes the tile
     if (t < a.T) {
-      const long long lo = __ldg(a.off64 + t), hi = __ldg(a.off64 + t + 1);
+      const long long lo = ends.lo, hi = ends.hi;
       const int len = (int)(hi - lo);
       if (hi <= a.cap && len > 0) {  // else truncated: the renderers scan all Gaussians
         mine = len > kWarpIds || over.beyond(len);
@@ -1198,7 +1207,9 @@ __device__ __forceinline__ void sort_tiles(const BinSort& a, const Frames& frame
   for (int u = 0; u < a.tiles_per_cta; ++u) {
     const int64_t t = t0 + u;
     if (t >= a.T) break;
-    const long long lo = __ldg(a.off64 + t), hi = __ldg(a.off64 + t + 1);
+    const bool one = a.tiles_per_cta == 1;
+    const long long lo = one ? ends.lo : __ldg(a.off64 + t);
+    const long long hi = one ? ends.hi : __ldg(a.off64 + t + 1);
     const int len = (int)(hi - lo);  // at most the image's Gaussians
     if (hi > a.cap || len == 0) continue;
     const bool beyond = over.beyond(len);
@@ -1228,7 +1239,7 @@ __device__ __noinline__ void sort_and_place(const BinSort& a, const Frames& fram
   } else {
     for (int64_t t0 = (int64_t)number * a.tiles_per_cta; t0 < a.T;
          t0 += (int64_t)tile_ctas * a.tiles_per_cta)
-      sort_tiles<CULL>(a, frames, t0, over, true, smem, tmp);
+      sort_tiles<CULL>(a, frames, t0, ends_of(a, t0), over, true, smem, tmp);
     const bool placed = wait_placed(a.tile_count + kPlacedWord, a.parts);
     if (!placed && threadIdx.x == 0)
       raise_status(a.status, SS_STATUS_INDEX_OVERFLOW);  // late ids may spoil a list
@@ -1247,6 +1258,8 @@ __global__ void __launch_bounds__(kSortThreads, 7)
   pdl_trigger();
   __shared__ __align__(16) uint32_t smem[kWindowWords];  // a bitmap, or ids and buckets
   __shared__ int tmp[kSortWarps + 1];
+  const int64_t t0 = (int64_t)blockIdx.x * a.tiles_per_cta;
+  const ListEnds ends = ends_of(a, t0);  // on their way while the words below are
   const bool trusted = a.tile_count[kBinsWord] == a.K;  // the bins belong to these counts
   const bool place = a.parts > 0 && (!trusted || a.tile_count[kOverflowWord] != 0);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1258,8 +1271,7 @@ __global__ void __launch_bounds__(kSortThreads, 7)
     sort_and_place<CULL>(a, frames, trusted, smem, tmp);
     return;
   }
-  const int64_t t0 = (int64_t)blockIdx.x * a.tiles_per_cta;
-  if (t0 < a.T) sort_tiles<CULL>(a, frames, t0, Overflow{a.K, 0, trusted}, false, smem, tmp);
+  if (t0 < a.T) sort_tiles<CULL>(a, frames, t0, ends, Overflow{a.K, 0, trusted}, false, smem, tmp);
 }
 
 // Bits that hold every id below n and the pad 2^bits - 1 above them.
