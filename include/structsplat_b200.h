@@ -154,9 +154,9 @@ int ss_tile_index_workspace_bytes(int64_t n, int height, int width, int tile_siz
 int ss_tile_index_binned_workspace_bytes(int64_t n, int height, int width, int tile_size,
                                          size_t* bytes);
 /* The better of the two sizes for an index of about `entries` pairs on `tiles` tiles of `images`
- * images.  Lists longer than their bins cost more than the plain form's: 100k Gaussians of 41 px on
- * 1024x1024 in 4-px tiles (12 M pairs) 580 us against 266, where a field whose lists fill less than
- * half the bins takes half the plain form's time. */
+ * images.  Short lists that outgrow their bins cost more than the plain form's: 100k Gaussians of
+ * 41 px on 1024x1024 in 4-px tiles (12 M pairs) 597 us against 266, where a field whose lists fit
+ * takes half the plain form's time. */
 int ss_tile_index_entries_workspace_bytes(int64_t n, int64_t tiles, int images, int64_t entries,
                                           size_t* bytes);
 /* Stage 1: per-tile counts and offsets.  tile_offsets (T+1) int32 receives the offsets;

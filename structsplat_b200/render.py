@@ -150,10 +150,10 @@ class _CapacityCache:
     def __init__(self):
         self.entries = {}
 
-    def entries_of(self, key) -> int:
-        """About the entries of the key's calls so far, 0 before the first."""
+    def workspace(self, key):
+        """Index workspace bytes for the entries of the key's calls so far, None before the first."""
         ent = self.entries.get(key)
-        return 0 if ent is None else (ent["cap"] - 1024) * 4 // 5
+        return None if ent is None else ent["workspace"]
 
     def capacity(self, key, offsets) -> int:
         ent = self.entries.get(key)
@@ -163,14 +163,20 @@ class _CapacityCache:
             host = torch.zeros(1, dtype=torch.int32, pin_memory=True)
             ent = self.entries[key] = {"cap": cap, "host": host, "event": None,
                                        "recorder": torch.cuda.Event()}
+            self._size(ent, key, offsets, total)
         elif ent["event"] is not None and ent["event"].query():
             seen = int(ent["host"][0])
             if seen > ent["cap"]:
                 ent["cap"] = int(seen * 1.25) + 1024
+                self._size(ent, key, offsets, seen)
         ent["host"].copy_(offsets[-1:], non_blocking=True)
         ent["recorder"].record()
         ent["event"] = ent["recorder"]
         return ent["cap"]
+
+    @staticmethod
+    def _size(ent, key, offsets, total: int):
+        ent["workspace"] = index_workspace_bytes(key[1], offsets.numel() - 1, total)
 
 
 CAPACITY = _CapacityCache()
@@ -282,9 +288,9 @@ def _index(n: int, H: int, W: int, tile_size: int, ellipse_cull: bool, sigma_cut
     tiles_x, tiles_y = tile_grid(H, W, tile_size)
     T = tiles_x * tiles_y
     key = (dev.index, n, H, W, tile_size, bool(ellipse_cull))
-    known = 0 if exact else CAPACITY.entries_of(key)
+    known = None if exact else CAPACITY.workspace(key)
     offsets = torch.empty(T + 1, device=dev, dtype=torch.int32)
-    ws_bytes = index_workspace_bytes(n, T, known)
+    ws_bytes = known or index_workspace_bytes(n, T, 0)
     ws = torch.empty(max(ws_bytes, 1), device=dev, dtype=torch.uint8)
 
     def count():
@@ -303,12 +309,15 @@ def _index(n: int, H: int, W: int, tile_size: int, ellipse_cull: bool, sigma_cut
         capacity = 0
     elif exact or capacity is None:
         if exact:
-            known = capacity = int(offsets[-1].item())
+            capacity = int(offsets[-1].item())
+            # only lists that nearly fill their bins (64 B a tile besides) ask for the plain form
+            better = index_workspace_bytes(n, T, capacity) if 8 * capacity > ws_bytes - 64 * T \
+                else ws_bytes
         else:
             capacity = CAPACITY.capacity(key, offsets)
-            known = 0 if known else CAPACITY.entries_of(key)  # a first call has read the total
-        if known and index_workspace_bytes(n, T, known) < ws_bytes:
-            ws_bytes = index_workspace_bytes(n, T, known)  # the plain form: count again without bins
+            better = known or CAPACITY.workspace(key)  # a first call has read the total
+        if better < ws_bytes:
+            ws_bytes = better  # count again without bins
             count()
     gids = torch.empty(max(capacity, 1), device=dev, dtype=torch.int32)
     _native.call("ss_tile_index_fill", _p(records), n, H, W, tile_size, int(ellipse_cull),

@@ -147,10 +147,10 @@ def test_overflow_costs_no_multiple_of_the_plain_form():
 
 def test_plans_take_the_plain_form_for_wide_fields():
     require_cuda()
-    n, H, W, ts = 20_000, 512, 512, 16
+    n, H, W, ts = 5_000, 1024, 1024, 16  # bins of 96 ids, lists of ~120
     g = torch.Generator("cuda").manual_seed(0)
-    p = {"means": torch.rand(n, 2, device="cuda", generator=g) * 512,
-         "log_scales": torch.full((n, 2), 2.9, device="cuda"),
+    p = {"means": torch.rand(n, 2, device="cuda", generator=g) * 1024,
+         "log_scales": torch.full((n, 2), 3.18, device="cuda"),
          "rotations": torch.rand(n, device="cuda", generator=g),
          "colors": torch.rand(n, 3, device="cuda", generator=g), "opacity_logits": None}
     plan = RenderPlan.for_field(p, H, W, tile_size=ts)
